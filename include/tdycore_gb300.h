@@ -241,9 +241,10 @@ typedef struct {
 } TDyNewtonOptions;
 /* Inner-solve schedules.  TILE: every kernel of a BiCGStab iteration runs over
  * all cells of the batch, instances masked as they converge (one iteration is
- * a CUDA graph).  BLOCK: one CTA per instance runs the instance's whole
- * BiCGStab loop (CTAs take instances from a counter, largest first).  AUTO:
- * an autotuner times the tile, block and split schedules (instances up to
+ * a CUDA graph).  BLOCK: one to eight CTAs per instance (a cluster) run the
+ * instance's whole BiCGStab loop (clusters take instances from a counter,
+ * largest first); an instance of more than 65536 cells stays on the tile
+ * schedule.  AUTO: an autotuner times the tile, block and split schedules (instances up to
  * 4096, 16384 or 65536 cells on the block schedule, the rest on the tile
  * schedule) on the first solve of a size class and keeps the fastest for the
  * process.  The cluster preconditioner runs on the tile schedule. */

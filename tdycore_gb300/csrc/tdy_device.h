@@ -1,6 +1,8 @@
 // tdy_device.h -- host-side interface of the CUDA translation unit.
 #pragma once
 
+#include <cuda_runtime_api.h>
+
 #include "tdy_internal.h"
 
 namespace tdy {
@@ -17,6 +19,12 @@ enum { FORM_SNES = 0, FORM_TS = 1, FORM_TV = 2 };
 // been synchronised.
 int dmem_alloc(void **p, size_t bytes, void *stream);
 void dmem_free(void *p, void *stream);
+
+// Streams and events from the per-device pools (of the current device), and
+// back to them (null ones ignored) once their work has completed.
+int device_pool_stream(cudaStream_t *st);
+int device_pool_event(cudaEvent_t *ev);
+void device_pool_release(int dev, cudaStream_t st, cudaEvent_t ev);
 
 int device_setup(_p_TDy *t);
 void device_destroy(_p_TDy *t);

@@ -1569,6 +1569,10 @@ static void pool_release(int dev, cudaStream_t st, cudaEvent_t ev) {
   if (ev) g_event_pool[dev].push_back(ev);
 }
 
+int device_pool_stream(cudaStream_t *st) { return pool_stream(st); }
+int device_pool_event(cudaEvent_t *ev) { return pool_event(ev); }
+void device_pool_release(int dev, cudaStream_t st, cudaEvent_t ev) { pool_release(dev, st, ev); }
+
 int device_setup(_p_TDy *t) {
   const Mesh &m = t->mesh;
   const MPFAOSetup &s = t->setup;

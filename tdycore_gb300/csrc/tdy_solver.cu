@@ -16,15 +16,17 @@
 //   * one BiCGStab iteration is built once as a CUDA graph with the explicit
 //     graph API (kernel nodes in a chain, no stream capture, so device calls
 //     that other threads make meanwhile cannot invalidate it) and replayed;
-//   * the sparse matrix-vector product's threads per row (1, 4 or 8) are
-//     picked by timing the candidates on the first solve.
+//   * the sparse matrix-vector product's threads per row (1, 2, 4 or 8) are
+//     picked by timing the candidates on the first solve that uses them.
 // No reference counterpart: the reference hands F and J to PETSc's SNES/KSP.
+#include <cooperative_groups.h>
 #include <cuda_runtime.h>
 
 #include <algorithm>
 #include <chrono>
 #include <climits>
 #include <cmath>
+#include <cstdint>
 #include <cstring>
 #include <mutex>
 #include <tuple>
@@ -58,6 +60,7 @@ struct Krylov {
        *ph = nullptr, *sh = nullptr, *y = nullptr;     // vectors (T)
   void *la = nullptr, *lcp = nullptr, *linv = nullptr; // line factors (T)
   void *cinv = nullptr;                                // clusters: 1/diagonal of the other cells (T)
+  void *sell = nullptr;                                // matrix values of the block schedule's instances (T)
   void *clu = nullptr;                                 // clusters: LU factors (T), grown on demand
   size_t clu_cap = 0;                                  // elements of clu
   cudaGraphExec_t graph = nullptr;
@@ -98,6 +101,21 @@ struct SolverState {
   // block_max_cells cells take the block schedule (-2: not chosen yet)
   int *inst_line_off = nullptr, *block_inst = nullptr, *block_mask = nullptr, *ticket = nullptr;
   std::vector<int> h_inst_line_off, h_order;  // h_order: instances by size, largest first
+  // the block schedule's matrix layout (built on its first use): slices of 32
+  // rows, entry k of the 32 rows side by side, column indices local to the
+  // instance; only instances up to kBlockCap cells have slices
+  int nslices = 0;
+  std::vector<int> h_slice_off, h_slice_row;  // first slice per instance; first row per slice
+  std::vector<long long> h_sell_off;          // first element per slice
+  int *slice_off = nullptr, *slice_row = nullptr, *slice_end = nullptr;
+  long long *sell_off = nullptr;
+  uint16_t *sell_col = nullptr;
+  // this solve's instances on the block schedule, class by class (CTAs per
+  // instance 8, 4, 2, 1), each class largest first
+  std::vector<int> h_block_list;
+  cudaStream_t side[3] = {nullptr, nullptr, nullptr};  // the classes run side by side
+  cudaEvent_t fork = nullptr, joined[3] = {nullptr, nullptr, nullptr};
+  int device = 0;
   long long block_max_cells = -2, mask_for = -3;
   int n_block = 0, n_tile = 0;
   std::vector<double> tune_ms;  // measured candidates of the last tuning (ms per linear solve)
@@ -117,6 +135,9 @@ struct SolverState {
   ~SolverState() {
     for (cudaEvent_t e : tev)
       if (e) cudaEventDestroy(e);
+    // (joined into the solve's stream, which every solve synchronises)
+    device_pool_release(device, nullptr, fork);
+    for (int i = 0; i < 3; i++) device_pool_release(device, side[i], joined[i]);
     for (Krylov *k : {&k32, &k64}) {
       if (k->graph) cudaGraphExecDestroy(k->graph);
       if (k->clu) dmem_free(k->clu, st);
@@ -283,8 +304,8 @@ __global__ void __launch_bounds__(256) spmv_kernel(int n, const int *rowptr, con
 
 // Thomas factorisation of every vertical line from the FP64 Jacobian
 template <class T>
-__global__ void line_factor_kernel(int nlines, const int *line_off, const int *pd, const int *plo, const int *phi,
-                                   const double *J, T *la, T *lcp, T *linv) {
+__global__ void line_factor_kernel(int nlines, const int *line_off, const int *line_cells, const int *pd,
+                                   const int *plo, const int *phi, const double *J, T *la, T *lcp, T *linv) {
   const int l = blockIdx.x * blockDim.x + threadIdx.x;
   if (l >= nlines) return;
   double cp = 0.0;
@@ -294,9 +315,10 @@ __global__ void line_factor_kernel(int nlines, const int *line_off, const int *p
     if (den == 0.0) den = (b != 0.0) ? b : 1.0;  // singular line: fall back to its diagonal
     const double inv = 1.0 / den;
     cp = c * inv;
-    la[k] = (T)a;
-    lcp[k] = (T)cp;
-    linv[k] = (T)inv;
+    const int i = line_cells[k];  // factors by cell: the lines of a warp are neighbours in every layer
+    la[i] = (T)a;
+    lcp[i] = (T)cp;
+    linv[i] = (T)inv;
   }
 }
 
@@ -308,13 +330,13 @@ __device__ __forceinline__ void line_solve_one(int l, const int *line_off, const
   T prev = 0;
   for (int k = k0; k < k1; k++) {
     const int i = line_cells[k];
-    prev = e_mul(e_fma(-la[k], prev, in[i]), linv[k]);
+    prev = e_mul(e_fma(-la[i], prev, in[i]), linv[i]);
     out[i] = prev;
   }
   T next = 0;
   for (int k = k1 - 1; k >= k0; k--) {
     const int i = line_cells[k];
-    next = e_fma(-lcp[k], next, out[i]);
+    next = e_fma(-lcp[i], next, out[i]);
     out[i] = next;
   }
 }
@@ -435,158 +457,597 @@ __global__ void xr_update_kernel(int n, const int *cs, const int *act, const dou
 }
 
 // ---------------------------------------------------------------------------
-// Block schedule: one CTA of kBlockThreads threads per instance runs the
-// instance's whole BiCGStab loop with the line preconditioner, performing the
-// tile schedule's operations in the tile schedule's order (reductions in
-// kChunk-cell chunks with the same per-chunk tree and in-order chunk sum, the
-// product's rows split over TPR lanes the same way), so the two schedules
-// give the same bits.  CTAs take instances from a ticket counter, largest
-// first; an instance's result does not depend on which CTA takes it.
+// Block schedule: C CTAs of kBlockThreads threads (a cluster; C = 1, 2, 4, 8)
+// run an instance's whole BiCGStab loop with the line preconditioner,
+// performing the tile schedule's operations in the tile schedule's order
+// (reductions in kChunk-cell chunks with the same per-chunk tree and in-order
+// chunk sum, each row's 8 phases and their tree), so the schedules and every C
+// give the same bits.  Clusters take instances from a ticket counter, largest
+// first; an instance's result does not depend on which cluster takes it.
+//
+// What bounds it is latency, then one SM's FP64 pipe (the dot products
+// accumulate in FP64) and its L2 bandwidth (the matrix is read twice an
+// iteration), hence
+//   * the vector that the sparse product gathers from, z, sits in shared
+//     memory, and the line solves work on it in place; so do, where they fit,
+//     the other vectors and the line factors (read back from L2 they cost a
+//     round trip in each of the ten passes of an iteration);
+//   * the matrix is stored in slices of 32 rows (entry k of the rows side by
+//     side, 16-bit column indices local to the instance), so the owner of a
+//     row reads it with coalesced, independent loads;
+//   * CTA q owns the cells with index [q, q + 1) * 256 / C modulo 256 in the
+//     instance: the vector updates and products of its cells take all its
+//     threads, and each of the 256 accumulators of a chunk reduction runs over
+//     cells of one CTA;
+//   * the tree of a reduction runs in one warp (7 additions from shared
+//     memory, 5 shuffles) instead of 8 levels of block barriers, and thread 0
+//     alone forms the scalars (a division by every thread would occupy the
+//     FP64 pipe for thousands of cycles).
 constexpr int kBlockThreads = 256;
-static_assert(kBlockThreads == 256, "the block schedule's reductions mirror the 256-thread chunk reductions");
+static_assert(kBlockThreads == 256 && kChunk % kBlockThreads == 0,
+              "the block schedule's reductions mirror the 256-thread chunk reductions");
+// largest instance of the block schedule (16-bit column indices)
+constexpr long long kBlockCap = 65536;
 
 template <class T>
 struct BlockSolve {
-  int ninst;                 // instances on the block schedule
+  int ninst;                 // instances of this launch
   const int *inst;           // their indices, largest first
   int *ticket;               // zeroed before the launch
   const int *seg_off;        // cells of instance g: [seg_off[g], seg_off[g + 1])
   const int *inst_line_off;  // lines of instance g: [inst_line_off[g], inst_line_off[g + 1])
-  const int *line_off, *line_cells;
-  const T *la, *lcp, *linv;
-  const int *rowptr, *colidx;
+  const int *slice_off;      // first slice of instance g
+  const long long *sell_off;
+  const int *rowptr;
   const T *A;
-  T *b, *r, *r0, *p, *v, *s, *t, *ph, *sh, *y;
-  const int *newt_active;
+  const uint16_t *col;
+  const T *la, *lcp, *linv;  // by cell
+  const double *F;
+  T *vec[8], *z, *x;  // V_*, z and the lines' cells where they exceed shared memory (y: the result)
+  int slots;          // KEEP_MATRIX: matrix slots of a CTA
   int *lin_its;
   double tol2;
   int max_it;
 };
 
-// (a, b) and, with c, (c, d) over cells [i0, i1): chunk_dot_kernel's
-// accumulation and tree per chunk, chunk_sum_kernel's in-order sum; every
-// thread returns the result
-template <class TA, class TB>
-__device__ __forceinline__ void block_dot(int i0, int i1, const TA *a, const TB *b, const TA *c, const TB *d,
-                                          double *red, double *out1, double *out2) {
-  const int tid = threadIdx.x;
-  double tot = 0.0, tot2 = 0.0;
-  for (int k0 = i0; k0 < i1; k0 += kChunk) {
-    const int k1 = min(k0 + kChunk, i1);
-    double acc = 0.0, acc2 = 0.0;
-    for (int i = k0 + tid; i < k1; i += kBlockThreads) {
-      acc = op_dot(acc, a[i], b[i]);
-      if (c) acc2 = op_dot(acc2, c[i], d[i]);
-    }
-    red[tid] = acc;
-    red[kBlockThreads + tid] = acc2;
+// What of an instance lives in shared memory: everything (each CTA the cells,
+// line factors and matrix rows it owns, and all of z), everything but the
+// matrix, z only, or nothing.
+enum { V_R0 = 0, V_R, V_P, V_V, V_S, V_T, V_PH, V_Y };
+enum { KEEP_MATRIX = 0, KEEP_ALL = 1, KEEP_Z = 2, KEEP_NONE = 3 };
+// chunks of an nc-cell instance that are reduced together, and the two sets of
+// their accumulators
+constexpr int kRedChunksMax = 2;
+__host__ __device__ constexpr int red_chunks(int nc) { return nc > kChunk ? kRedChunksMax : 1; }
+__host__ __device__ constexpr int red_doubles(int nc) { return 2 * red_chunks(nc) * 2 * kBlockThreads; }
+// cells a CTA owns at most, and cells of the lines it solves
+__host__ __device__ inline int owned_cells(int nc, int C) {
+  return (nc + kBlockThreads - 1) / kBlockThreads * (kBlockThreads / C);
+}
+// The lines' cells and factors lie line by line in shared memory, nlp layers
+// apart: 16-byte loads fetch kLineVec layers, and nlp is an odd multiple of
+// kLineVec, which spreads the lines of a warp over the banks.
+template <class T>
+struct LineVec;
+template <>
+struct LineVec<float> {
+  using type = float4;
+};
+template <>
+struct LineVec<double> {
+  using type = double2;
+};
+template <class T>
+constexpr int kLineVec = 16 / (int)sizeof(T);
+template <class T>
+__host__ __device__ constexpr int line_pitch(int nl) {
+  return ((nl + kLineVec<T> - 1) / kLineVec<T> | 1) * kLineVec<T>;
+}
+
+inline size_t up16(size_t b) { return (b + 15) & ~size_t(15); }
+// (lines: lines a CTA solves at most; slots: matrix slots of one CTA's rows)
+template <class T>
+size_t block_smem(int keep, int nc, int lines, int nl, size_t slots, int C) {
+  size_t b = sizeof(double) * red_doubles(nc);
+  if (keep != KEEP_NONE) b += up16(sizeof(T) * nc);
+  if (keep != KEEP_NONE) b += sizeof(T) * lines * line_pitch<T>(nl);
+  if (keep <= KEEP_ALL)
+    b += 3 * sizeof(T) * lines * line_pitch<T>(nl) + up16((8 * sizeof(T) + sizeof(unsigned)) * owned_cells(nc, C));
+  if (keep == KEEP_MATRIX) b += (sizeof(T) + sizeof(uint16_t)) * slots;
+  return b;
+}
+
+// exact conversion without the FP64 pipe (a conversion instruction costs as
+// much there as an FMA); zeros, subnormals, infinities and NaN the plain way
+__device__ __forceinline__ double to_f64(double x) { return x; }
+__device__ __forceinline__ double to_f64(float x) {
+  const unsigned u = __float_as_uint(x), e = u & 0x7f800000u;
+  if (e == 0u || e == 0x7f800000u) return (double)x;
+  return __hiloint2double((int)((u & 0x80000000u) | (((u & 0x7fffffffu) >> 3) + (896u << 20))), (int)(u << 29));
+}
+
+template <int C>
+__device__ __forceinline__ void csync() {
+  if constexpr (C == 1)
     __syncthreads();
-    for (int w = kBlockThreads / 2; w > 0; w >>= 1) {
-      if (tid < w) {
-        red[tid] += red[tid + w];
-        red[kBlockThreads + tid] += red[kBlockThreads + tid + w];
+  else
+    cooperative_groups::this_cluster().sync();
+}
+// the same shared variable of CTA `rank` of the cluster
+template <int C, class U>
+__device__ __forceinline__ U *peer(U *p, int rank) {
+  if constexpr (C == 1)
+    return p;
+  else
+    return cooperative_groups::this_cluster().map_shared_rank(p, rank);
+}
+
+// G rows of the sliced matrix times z by TPR lanes each: the sums of row_dot,
+// valid in lane 0.  Row u has rn[u] entries from element base[u] on.  The
+// loads of all rows and of two steps of each phase are in flight together
+// (one row at a time, every row waited for L2: 2.7 k cycles a row at 1 k
+// cells, 1.1 k so).
+template <class T, int TPR, int G, bool GLOBAL>
+__device__ __forceinline__ void sell_dot(const unsigned *base, const int *rn, int lane, const T *A, const uint16_t *col,
+                                         const T *z, T *out) {
+  constexpr int NP = 8 / TPR;
+  T P[G][NP];
+  int most = 0;
+#pragma unroll
+  for (int u = 0; u < G; u++) {
+    most = max(most, rn[u]);
+#pragma unroll
+    for (int q = 0; q < NP; q++) P[u][q] = 0;
+  }
+#pragma unroll 2
+  for (int k0 = lane; k0 < most; k0 += 8) {
+    T a[G][NP];
+    int c[G][NP];
+#pragma unroll
+    for (int u = 0; u < G; u++)
+#pragma unroll
+      for (int q = 0; q < NP; q++) {
+        const int k = k0 + TPR * q;
+        if (k < rn[u]) {
+          // (the read-only path lets loads pass the stores of earlier rows)
+          a[u][q] = GLOBAL ? __ldg(A + base[u] + 32 * k) : A[base[u] + 32 * k];
+          c[u][q] = GLOBAL ? __ldg(col + base[u] + 32 * k) : col[base[u] + 32 * k];
+        }
+      }
+#pragma unroll
+    for (int u = 0; u < G; u++)
+#pragma unroll
+      for (int q = 0; q < NP; q++)
+        if (k0 + TPR * q < rn[u]) P[u][q] = e_fma(a[u][q], z[c[u][q]], P[u][q]);
+  }
+#pragma unroll
+  for (int u = 0; u < G; u++) {
+#pragma unroll
+    for (int o = 4; o >= TPR; o >>= 1) {
+#pragma unroll
+      for (int q = 0; q < o / TPR; q++) P[u][q] = e_add(P[u][q], P[u][q + o / TPR]);
+    }
+    out[u] = P[u][0];
+  }
+#pragma unroll
+  for (int o = TPR / 2; o > 0; o >>= 1)
+#pragma unroll
+    for (int u = 0; u < G; u++) out[u] = e_add(out[u], __shfl_down_sync(0xffffffffu, out[u], o, TPR));
+}
+
+// x <- (line-tridiagonal)^-1 x for n lines of nl layers, one thread per line;
+// layer k of line l sits at [l * xp + k] of x and at [l * fl + k * fs] of the
+// factors (VEC: fl = xp, fs = 1).  The recurrence is the critical path: a layer
+// takes 9 cycles in FP32 and 126 in FP64 forward, half of that backward; with
+// 4-byte loads, the load instructions took 27 in FP32.
+template <class T, bool VEC>
+__device__ __forceinline__ void block_lines(int n, int nl, int xp, int fl, int fs, const T *la, const T *lcp,
+                                            const T *linv, T *x) {
+  constexpr int V = kLineVec<T>, U = 8;
+  using VT = typename LineVec<T>::type;
+#pragma unroll 1
+  for (int l = threadIdx.x; l < n; l += kBlockThreads) {
+    T *const xl = x + l * xp;
+    const T *const al = la + l * fl, *const cl = lcp + l * fl, *const dl = linv + l * fl;
+    auto load = [&](T *dst, const T *src, int k, int step) {
+      if constexpr (VEC) {
+#pragma unroll
+        for (int u = 0; u < U; u += V) *reinterpret_cast<VT *>(dst + u) = *reinterpret_cast<const VT *>(src + k + u);
+      } else {
+#pragma unroll
+        for (int u = 0; u < U; u++) dst[u] = src[(k + u) * step];
+      }
+    };
+    const int full = nl / U * U;
+    T prev = 0;
+#pragma unroll 1
+    for (int k = 0; k < full; k += U) {
+      alignas(16) T v[U], a[U], d[U];
+      load(v, xl, k, 1);
+      load(a, al, k, fs);
+      load(d, dl, k, fs);
+#pragma unroll
+      for (int u = 0; u < U; u++) v[u] = prev = e_mul(e_fma(-a[u], prev, v[u]), d[u]);
+      if constexpr (VEC) {
+#pragma unroll
+        for (int u = 0; u < U; u += V) *reinterpret_cast<VT *>(xl + k + u) = *reinterpret_cast<VT *>(v + u);
+      } else {
+#pragma unroll
+        for (int u = 0; u < U; u++) xl[k + u] = v[u];
+      }
+    }
+#pragma unroll 1
+    for (int k = full; k < nl; k++) xl[k] = prev = e_mul(e_fma(-al[k * fs], prev, xl[k]), dl[k * fs]);
+    T next = 0;
+#pragma unroll 1
+    for (int k = nl - 1; k >= full; k--) xl[k] = next = e_fma(-cl[k * fs], next, xl[k]);
+#pragma unroll 1
+    for (int k = full - U; k >= 0; k -= U) {
+      alignas(16) T v[U], c[U];
+      load(v, xl, k, 1);
+      load(c, cl, k, fs);
+#pragma unroll
+      for (int u = U - 1; u >= 0; u--) v[u] = next = e_fma(-c[u], next, v[u]);
+      if constexpr (VEC) {
+#pragma unroll
+        for (int u = 0; u < U; u += V) *reinterpret_cast<VT *>(xl + k + u) = *reinterpret_cast<VT *>(v + u);
+      } else {
+#pragma unroll
+        for (int u = 0; u < U; u++) xl[k + u] = v[u];
+      }
+    }
+  }
+}
+
+// (two CTAs per SM: the loops' loads hide behind the other CTA's barriers)
+template <class T, int C, int KEEP>
+__global__ void __launch_bounds__(kBlockThreads, sizeof(T) == 4 ? 2 : 1) bicgstab_block_kernel(const BlockSolve<T> B) {
+  static_assert(KEEP != KEEP_NONE || C == 1, "clusters exchange z through shared memory");
+  constexpr int NO = kBlockThreads / C;  // cells (of 256 consecutive ones) that a CTA owns
+  // reductions (two sets in turn), z, the own lines, own vectors, line
+  // factors, own rows (first element << 8 | entries)
+  extern __shared__ double bsm[];
+  __shared__ int cur, stop;
+  __shared__ T c_alpha, c_beta, c_omega;
+  __shared__ double c_sum[2][2 * kRedChunksMax], c_ratio, c_alpha64, c_omega64;
+  const int tid = threadIdx.x;
+  const int q = C == 1 ? 0 : (int)(blockIdx.x % C);
+  int buf = 0;
+  for (;;) {
+    if (q == 0 && tid == 0) {
+      const int k = atomicAdd(B.ticket, 1);
+#pragma unroll
+      for (int r = 0; r < C; r++) *peer<C>(&cur, r) = k;
+    }
+    csync<C>();
+    const int k = cur;
+    csync<C>();  // every thread has read the ticket before the next one is drawn
+    if (k >= B.ninst) return;
+    const int g = B.inst[k];
+    const int c0 = B.seg_off[g], nc = B.seg_off[g + 1] - c0;
+    const int nc2 = B.inst_line_off[g + 1] - B.inst_line_off[g], nl = nc / nc2;
+    const int nj = (nc + kBlockThreads - 1) / kBlockThreads;
+    const int *rowptr = B.rowptr + c0;
+    const long long *so = B.sell_off + B.slice_off[g];
+    const int nred = red_chunks(nc);
+    constexpr bool SHARED = KEEP <= KEEP_ALL;
+    const int nown = owned_cells(nc, C);
+    // lines q, q + C, ... of the instance
+    const int n1 = (nc2 - q + C - 1) / C, lines = (nc2 + C - 1) / C;
+    const int nlp = KEEP == KEEP_NONE ? nl : line_pitch<T>(nl), nf = lines * nlp;
+    char *at_byte = reinterpret_cast<char *>(bsm + red_doubles(nc));
+    T *const z = KEEP == KEEP_NONE ? B.z + c0 : reinterpret_cast<T *>(at_byte);
+    at_byte += (nc * sizeof(T) + 15) & ~size_t(15);
+    T *const x = KEEP == KEEP_NONE ? B.x + c0 : reinterpret_cast<T *>(at_byte);
+    T *const lf = x + nf;
+    T *const w = lf + 3 * nf;
+    unsigned *const rinfo = reinterpret_cast<unsigned *>(w + 8 * nown);
+    // own cell e is cell i(e) of the instance
+    auto cell = [&](int e) { return e / NO * kBlockThreads + q * NO + e % NO; };
+    // vector k at own cell e (the base of each vector is formed where it is
+    // used: held in registers they spill)
+    auto at = [&](int k, int e) -> T & { return SHARED ? w[k * nown + e] : B.vec[k][c0 + cell(e)]; };
+    // f(e, i) for the own cells
+    auto each = [&](auto f) {
+#pragma unroll 1
+      for (int e = tid; e < nown; e += kBlockThreads) {
+        const int i = cell(e);
+        if (i < nc) f(e, i);
+      }
+    };
+    const T *A = B.A + so[0];
+    const uint16_t *col = B.col + so[0];
+    if constexpr (SHARED) {
+      for (int e = tid; e < n1 * nl; e += kBlockThreads) {
+        const int kk = e / n1, l = e - kk * n1, i = c0 + kk * nc2 + q + C * l;
+        lf[l * nlp + kk] = B.la[i];
+        lf[nf + l * nlp + kk] = B.lcp[i];
+        lf[2 * nf + l * nlp + kk] = B.linv[i];
+      }
+      if constexpr (KEEP == KEEP_ALL) {
+        // (an instance whose vectors fit shared memory has far fewer than 2^24 entries)
+        each([&](int e, int i) {
+          rinfo[e] = (unsigned)(so[i >> 5] - so[0] + (i & 31)) << 8 | (unsigned)(rowptr[i + 1] - rowptr[i]);
+        });
+      } else {
+        // the own rows in slices of 32 of their own: those of slice e / 32 as
+        // wide as in HBM, where they are (parts of) neighbouring slices
+        T *const As = reinterpret_cast<T *>(reinterpret_cast<char *>(w) +
+                                            (((8 * sizeof(T) + sizeof(unsigned)) * nown + 15) & ~size_t(15)));
+        uint16_t *const cs = reinterpret_cast<uint16_t *>(As + B.slots);
+        // widths of the own slices, then their offsets
+        const int ns = (nown + 31) / 32;
+        unsigned off = 0;
+        for (int sl = 0; sl < ns; sl++) {
+          int width = 0;
+          for (int e = sl * 32; e < min(nown, sl * 32 + 32); e += min(NO, 32)) {
+            const int i = cell(e);
+            if (i < nc) width = max(width, (int)(so[(i >> 5) + 1] - so[i >> 5]) / 32);
+          }
+          if (tid / 32 == sl % (kBlockThreads / 32)) {
+            const int e = sl * 32 + (tid & 31), i = cell(e);
+            if (e < nown && i < nc) {
+              const int rn = rowptr[i + 1] - rowptr[i];
+              rinfo[e] = (off + (tid & 31)) << 8 | (unsigned)rn;
+              const T *src = A + (so[i >> 5] - so[0]) + (i & 31);
+              const uint16_t *csrc = col + (so[i >> 5] - so[0]) + (i & 31);
+#pragma unroll 4
+              for (int k = 0; k < rn; k++) {
+                As[off + (tid & 31) + 32 * k] = __ldg(src + 32 * k);
+                cs[off + (tid & 31) + 32 * k] = __ldg(csrc + 32 * k);
+              }
+            }
+          }
+          off += 32 * width;
+        }
+        A = As;
+        col = cs;
+      }
+    }
+    auto row_info = [&](int e, int i, unsigned *base, int *rn) {
+      if constexpr (SHARED) {
+        *base = rinfo[e] >> 8;
+        *rn = (int)(rinfo[e] & 255u);
+      } else {
+        *base = (unsigned)(so[i >> 5] - so[0]) + (i & 31);
+        *rn = rowptr[i + 1] - rowptr[i];
+      }
+    };
+
+    // (vector k0, vector k1) and, with k2 >= 0, (vector k2, vector k3): per
+    // chunk the accumulators and the 256-way tree of chunk_dot_kernel, then the
+    // chunks in order.  With C > 1 each sum and chunk has threads (and a part of
+    // the FP64 pipe) of its own, and one warp does each tree (the additions of a
+    // warp take 60 cycles each); another one does `side` meanwhile.  Thread 0 of
+    // each CTA gets the sums; the cluster is synchronised in between.
+    auto nothing = []() {};
+    auto dots = [&](int k0, int k1, int k2, int k3, double *s0, double *s1, auto side) {
+      constexpr int JC = kChunk / kBlockThreads;
+      const int nsum = k2 >= 0 ? 2 : 1;
+      double t0 = 0.0, t1 = 0.0;
+      __syncthreads();  // the vectors are complete
+      for (int jr = 0; jr < nj; jr += nred * JC) {
+        double *red = bsm + buf * (nred * 2 * kBlockThreads);
+        const int nch = min(nred, (nj - jr + JC - 1) / JC), np = nsum * nch;
+        // pair p: sum p / nch of chunk p % nch; its accumulator of index
+        // q * NO + o modulo 256
+#pragma unroll 1
+        for (int pr = tid / NO; pr < np; pr += C) {
+          const int hs = pr >= nch, o = tid % NO, j0 = jr + (pr - hs * nch) * JC, j1 = min(j0 + JC, nj);
+          const int ka = hs ? k2 : k0, kb = hs ? k3 : k1;
+          double acc = 0.0;
+#pragma unroll 4
+          for (int j = j0; j < j1; j++)
+            if (j * kBlockThreads + q * NO + o < nc)
+              acc = __fma_rn(to_f64(at(ka, j * NO + o)), to_f64(at(kb, j * NO + o)), acc);
+#pragma unroll
+          for (int rk = 0; rk < C; rk++) peer<C>(red, rk)[pr * kBlockThreads + q * NO + o] = acc;
+        }
+        csync<C>();
+        if (jr == 0 && tid == 128) side();
+        if (tid / 32 < np) {
+          const double *d = red + (tid / 32) * kBlockThreads + (tid & 31);
+          double t = __dadd_rn(__dadd_rn(__dadd_rn(d[0], d[128]), __dadd_rn(d[64], d[192])),
+                               __dadd_rn(__dadd_rn(d[32], d[160]), __dadd_rn(d[96], d[224])));
+#pragma unroll
+          for (int o = 16; o > 0; o >>= 1) t = __dadd_rn(t, __shfl_down_sync(0xffffffffu, t, o));
+          if ((tid & 31) == 0) c_sum[buf][tid / 32] = t;
+        }
+        __syncthreads();
+        if (tid == 0)
+          for (int ch = 0; ch < nch; ch++) {
+            t0 = __dadd_rn(t0, c_sum[buf][ch]);
+            if (nsum > 1) t1 = __dadd_rn(t1, c_sum[buf][nch + ch]);
+          }
+        buf ^= 1;
+      }
+      *s0 = t0;
+      if (nsum > 1) *s1 = t1;
+    };
+    // vector `out` = A z at the own cells, two lanes per row (more lanes spend
+    // FP64 additions on their tree: 3 for 4 rows with 8 lanes, 4 for 16 with 2)
+    auto product = [&](int out, bool keep_z) {
+      constexpr int TPR = 2, G = sizeof(T) == 4 ? 2 : 1, RP = kBlockThreads / TPR;
+      const int lane = tid % TPR;
+#pragma unroll 1
+      for (int e0 = tid / TPR; e0 - tid / TPR < nown; e0 += G * RP) {
+        unsigned base[G];
+        int rn[G];
+        T sum[G];
+#pragma unroll
+        for (int u = 0; u < G; u++) {
+          const int e = e0 + u * RP, i = cell(e);
+          base[u] = 0;
+          rn[u] = 0;
+          if (e < nown && i < nc) row_info(e, i, &base[u], &rn[u]);
+        }
+        sell_dot<T, TPR, G, KEEP != KEEP_MATRIX>(base, rn, lane, A, col, z, sum);
+#pragma unroll
+        for (int u = 0; u < G; u++) {
+          const int e = e0 + u * RP, i = cell(e);
+          if (lane == 0 && e < nown && i < nc) {
+            at(out, e) = sum[u];
+            if (keep_z) at(V_PH, e) = z[i];
+          }
+        }
+      }
+    };
+    // the line solves' input goes to the CTA that solves the cell's line
+    auto to_line = [&](int i, T v) {
+      const int kk = i / nc2, l = i - kk * nc2;
+      peer<C>(x, l & (C - 1))[l / C * nlp + kk] = v;
+    };
+    // M^-1 of the lines' input, to every CTA's z
+    auto precondition = [&]() {
+      csync<C>();
+      if constexpr (SHARED)
+        block_lines<T, true>(n1, nl, nlp, nlp, 1, lf, lf + nf, lf + 2 * nf, x);
+      else
+        block_lines<T, false>(n1, nl, nlp, C, nc2, B.la + c0 + q, B.lcp + c0 + q, B.linv + c0 + q, x);
+      __syncthreads();
+      for (int e = tid; e < n1 * nl; e += kBlockThreads) {
+        const int kk = e / n1, l = e - kk * n1, i = kk * nc2 + q + C * l;
+        const T v = x[l * nlp + kk];
+#pragma unroll
+        for (int rk = 0; rk < C; rk++) peer<C>(z, rk)[i] = v;
+      }
+      csync<C>();
+    };
+
+    // thread 0's scalars
+    double bnorm2 = 0.0, tol = 0.0, rho = 1.0, alpha = 1.0, omega = 1.0, d0, d1;
+    int its = 0;
+    each([&](int e, int i) {
+      const T f = (T)B.F[c0 + i];
+      at(V_R0, e) = f;
+      at(V_R, e) = f;
+      at(V_P, e) = 0;
+      at(V_V, e) = 0;
+      at(V_Y, e) = 0;
+    });
+    dots(V_R0, V_R0, -1, -1, &bnorm2, nullptr, nothing);
+    // the scalars of an iteration's first half, from rn = (r0, r)
+    auto begin = [&](double rn, int it) {
+      stop = it >= B.max_it || rn == 0.0;
+      if (stop) return;
+      const double beta = (rn / rho) * c_ratio;  // alpha / omega
+      rho = rn;
+      c_beta = (T)beta;
+      c_omega = (T)omega;
+    };
+    if (tid == 0) {
+      c_ratio = 1.0;
+      tol = B.tol2 * bnorm2;
+      if (bnorm2 > 0.0)
+        begin(bnorm2, 0);  // r = r0
+      else
+        stop = 1;
+    }
+    __syncthreads();
+    for (int it = 0; !stop; it++) {
+      {
+        const T tb = c_beta, to = c_omega;
+        each([&](int e, int i) {
+          const T pi = op_p(at(V_R, e), at(V_P, e), at(V_V, e), tb, to);
+          at(V_P, e) = pi;
+          to_line(i, pi);
+        });
+      }
+      precondition();
+      product(V_V, true);
+      dots(V_R0, V_V, -1, -1, &d0, nullptr, nothing);
+      if (tid == 0) {
+        stop = d0 == 0.0;
+        if (!stop) {
+          alpha = rho / d0;
+          c_alpha = (T)alpha;
+        }
+      }
+      __syncthreads();
+      if (stop) break;
+      const T ta = c_alpha;
+      each([&](int e, int i) {
+        const T si = e_fma(-ta, at(V_V, e), at(V_R, e));
+        at(V_S, e) = si;
+        to_line(i, si);
+      });
+      dots(V_S, V_S, -1, -1, &d0, nullptr, nothing);
+      if (tid == 0) {
+        stop = d0 <= tol;  // converged at the half step
+        if (stop) its++;
+      }
+      __syncthreads();
+      if (stop) {
+        each([&](int e, int) { at(V_Y, e) = op_y(at(V_Y, e), at(V_PH, e), ta); });
+        break;
+      }
+      precondition();
+      product(V_T, false);
+      dots(V_T, V_T, V_T, V_S, &d0, &d1, nothing);
+      if (tid == 0) {
+        omega = d0 > 0.0 ? d1 / d0 : 0.0;
+        c_omega = (T)omega;
+        c_alpha64 = alpha;
+        c_omega64 = omega;
+      }
+      __syncthreads();
+      const T to = c_omega;
+      each([&](int e, int i) {
+        at(V_Y, e) = op_y2(at(V_Y, e), at(V_PH, e), z[i], ta, to);
+        at(V_R, e) = e_fma(-to, at(V_T, e), at(V_S, e));
+      });
+      dots(V_R, V_R, V_R0, V_R, &d0, &d1, [&]() { c_ratio = c_alpha64 / c_omega64; });
+      if (tid == 0) {
+        its++;
+        if (d0 <= tol || omega == 0.0)
+          stop = 1;
+        else
+          begin(d1, it + 1);
       }
       __syncthreads();
     }
-    tot += red[0];
-    tot2 += red[kBlockThreads];
-    __syncthreads();  // every thread has read the chunk's sums
-  }
-  *out1 = tot;
-  if (out2) *out2 = tot2;
-}
-
-// y = A x over rows [c0, c1): the row sums of spmv_kernel (row_dot)
-template <class T, int TPR>
-__device__ __forceinline__ void block_spmv(int c0, int c1, const int *rowptr, const int *colidx, const T *A,
-                                           const T *x, T *y) {
-  const int nrow = c1 - c0;
-  for (int base = 0; base < nrow * TPR; base += kBlockThreads) {
-    const int gt = base + (int)threadIdx.x, rl = gt / TPR, lane = gt % TPR, row = c0 + rl;
-    const T acc = row_dot<T, TPR>(rl < nrow, rl < nrow ? rowptr[row] : 0, rl < nrow ? rowptr[row + 1] : 0, lane,
-                                  colidx, A, x);
-    if (rl < nrow && lane == 0) y[row] = acc;
+    if constexpr (SHARED) each([&](int e, int i) { B.vec[V_Y][c0 + i] = at(V_Y, e); });
+    if (q == 0 && tid == 0) B.lin_its[g] = its;
   }
 }
 
-template <class T, int TPR>
-__global__ void __launch_bounds__(kBlockThreads) bicgstab_block_kernel(BlockSolve<T> B) {
-  __shared__ double red[2 * kBlockThreads];
-  __shared__ int cur;
-  const int tid = threadIdx.x;
-  for (;;) {
-    if (tid == 0) cur = atomicAdd(B.ticket, 1);
-    __syncthreads();
-    const int k = cur;
-    __syncthreads();  // every thread has read the ticket before the next one is drawn
-    if (k >= B.ninst) return;
-    const int g = B.inst[k];
-    const int c0 = B.seg_off[g], c1 = B.seg_off[g + 1];
-    const int l0 = B.inst_line_off[g], l1 = B.inst_line_off[g + 1];
-    int its = 0;
-    double bnorm2 = 0.0;
-    if (B.newt_active[g]) block_dot<T, T>(c0, c1, B.b, B.b, nullptr, nullptr, red, &bnorm2, nullptr);
-    if (bnorm2 > 0.0) {
-      double rho = 1.0, alpha = 1.0, omega = 1.0;
-      for (int it = 0; it < B.max_it; it++) {
-        double rn;
-        block_dot<T, T>(c0, c1, B.r0, B.r, nullptr, nullptr, red, &rn, nullptr);
-        if (rn == 0.0) break;
-        const double beta = (rn / rho) * (alpha / omega);
-        rho = rn;
-        {
-          const T tb = (T)beta, to = (T)omega;
-          for (int i = c0 + tid; i < c1; i += kBlockThreads) B.p[i] = op_p(B.r[i], B.p[i], B.v[i], tb, to);
-        }
-        __syncthreads();
-        for (int l = l0 + tid; l < l1; l += kBlockThreads)
-          line_solve_one(l, B.line_off, B.line_cells, B.la, B.lcp, B.linv, B.p, B.ph);
-        __syncthreads();
-        block_spmv<T, TPR>(c0, c1, B.rowptr, B.colidx, B.A, B.ph, B.v);
-        __syncthreads();
-        double dv;
-        block_dot<T, T>(c0, c1, B.r0, B.v, nullptr, nullptr, red, &dv, nullptr);
-        if (dv == 0.0) break;
-        alpha = rho / dv;
-        {
-          const T ta = (T)alpha;
-          for (int i = c0 + tid; i < c1; i += kBlockThreads) B.s[i] = e_fma(-ta, B.v[i], B.r[i]);
-        }
-        __syncthreads();
-        double ss;
-        block_dot<T, T>(c0, c1, B.s, B.s, nullptr, nullptr, red, &ss, nullptr);
-        const bool half = ss <= B.tol2 * bnorm2;
-        if (half) {
-          const T ta = (T)alpha;
-          for (int i = c0 + tid; i < c1; i += kBlockThreads) B.y[i] = op_y(B.y[i], B.ph[i], ta);
-          __syncthreads();
-          its++;
-          break;
-        }
-        for (int l = l0 + tid; l < l1; l += kBlockThreads)
-          line_solve_one(l, B.line_off, B.line_cells, B.la, B.lcp, B.linv, B.s, B.sh);
-        __syncthreads();
-        block_spmv<T, TPR>(c0, c1, B.rowptr, B.colidx, B.A, B.sh, B.t);
-        __syncthreads();
-        double tt, ts;
-        block_dot<T, T>(c0, c1, B.t, B.t, B.t, B.s, red, &tt, &ts);
-        omega = tt > 0.0 ? ts / tt : 0.0;
-        {
-          const T ta = (T)alpha, to = (T)omega;
-          for (int i = c0 + tid; i < c1; i += kBlockThreads) {
-            B.y[i] = op_y2(B.y[i], B.ph[i], B.sh[i], ta, to);
-            B.r[i] = e_fma(-to, B.t[i], B.s[i]);
-          }
-        }
-        __syncthreads();
-        double rr;
-        block_dot<T, T>(c0, c1, B.r, B.r, nullptr, nullptr, red, &rr, nullptr);
-        its++;
-        if (rr <= B.tol2 * bnorm2 || omega == 0.0) break;
+// Column indices of the sliced layout, local to the instance, and (each
+// solve) the values of the active instances: one warp per slice, the rows read
+// with coalesced loads and turned through shared memory.
+constexpr int kSliceWarps = 4;
+constexpr int kSliceCols = 32;  // entries of the rows turned at a time
+template <class TO, class TI>
+__global__ void __launch_bounds__(32 * kSliceWarps) sell_fill_kernel(int nslices, const int *slice_row,
+                                                                      const int *slice_end, const long long *sell_off,
+                                                                      const int *cell_seg, const int *active,
+                                                                      const int *seg_off, const int *rowptr,
+                                                                      const TI *in, TO *out) {
+  __shared__ TO buf[kSliceWarps][32][kSliceCols + 1];
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int sl = blockIdx.x * kSliceWarps + warp;
+  if (sl >= nslices) return;  // whole warp
+  const int row0 = slice_row[sl], nrow = slice_end[sl] - row0, g = cell_seg[row0];
+  if (active && !active[g]) return;
+  const long long o0 = sell_off[sl];
+  const int width = (int)((sell_off[sl + 1] - o0) / 32);
+  const int c0 = seg_off[g];
+  for (int k0 = 0; k0 < width; k0 += kSliceCols) {
+    for (int rr = 0; rr < nrow; rr++) {
+      const int p0 = rowptr[row0 + rr], k = k0 + lane;
+      TO x = 0;
+      if (k < rowptr[row0 + rr + 1] - p0) {
+        if constexpr (sizeof(TO) == 2)
+          x = (TO)(in[p0 + k] - c0);
+        else
+          x = (TO)in[p0 + k];
       }
+      buf[warp][rr][lane] = x;
     }
-    if (tid == 0) B.lin_its[g] = its;
-    __syncthreads();
+    __syncwarp();
+    const int n = min(kSliceCols, width - k0);
+    if (lane < nrow)
+      for (int k = 0; k < n; k++) out[o0 + (long long)(k0 + k) * 32 + lane] = buf[warp][lane][k];
+    __syncwarp();
   }
 }
 
@@ -860,15 +1321,15 @@ void bicgstab_iteration(SolverState *s, Krylov &k, double tol2, Emit &e) {
   e(scal_check_kernel, sb, 128, 0, ns, act, s->lin_its, sc, tol2);
 }
 
-// (one allocation for the Jacobian copy and every vector; ordered on the
-// solve's stream, which uses them next)
+// (one allocation for every vector; ordered on the solve's stream, which uses
+// them next)
 template <class T>
 int krylov_alloc(SolverState *s, Krylov &k, cudaStream_t st) {
+  // (the CSR copy Jv and the sliced copy are allocated by the schedules that use them)
   if (k.ready) return 0;
   Arena ar;
   T **vecs[] = {(T **)&k.b, (T **)&k.r,  (T **)&k.r0, (T **)&k.p,  (T **)&k.v,   (T **)&k.s,   (T **)&k.t,
                 (T **)&k.ph, (T **)&k.sh, (T **)&k.y, (T **)&k.la, (T **)&k.lcp, (T **)&k.linv};
-  ar.work((T **)&k.Jv, (size_t)s->nnz);
   for (T **vp : vecs) ar.work(vp, (size_t)s->n);
   int ierr = ar.commit(st);
   if (ierr) return ierr;
@@ -1016,66 +1477,227 @@ int cluster_setup(SolverState *s, Krylov &k, double tau, cudaStream_t st) {
   return 0;
 }
 
+// The sliced matrix layout of the block schedule, on its first use: offsets
+// from the rows' lengths, column indices by sell_fill_kernel.
+int sell_setup(SolverState *s, cudaStream_t st) {
+  if (s->sell_col) return 0;
+  int ierr;
+  std::vector<int> end(s->h_slice_row.size());
+  for (size_t g = 0; g + 1 < s->h_seg_off.size(); g++)
+    for (int k = s->h_slice_off[g]; k < s->h_slice_off[g + 1]; k++)
+      end[k] = std::min(s->h_slice_row[k] + 32, s->h_seg_off[g + 1]);
+  Arena ar;
+  ar.up(&s->slice_off, s->h_slice_off);
+  ar.up(&s->slice_row, s->h_slice_row);
+  ar.up(&s->slice_end, end);
+  ar.up(&s->sell_off, s->h_sell_off);
+  ar.work(&s->sell_col, (size_t)s->h_sell_off.back());
+  if ((ierr = ar.commit(st))) return ierr;
+  s->allocs.push_back(ar.base);
+  if (s->nslices > 0)
+    sell_fill_kernel<uint16_t, int><<<nblk(s->nslices, kSliceWarps), 32 * kSliceWarps, 0, st>>>(
+        s->nslices, s->slice_row, s->slice_end, s->sell_off, s->cell_seg, nullptr, s->seg_off, s->rowptr, s->colidx,
+        s->sell_col);
+  SCUDA(cudaGetLastError());
+  SCUDA(cudaStreamSynchronize(st));  // the host vectors are read
+  return 0;
+}
+
+bool on_block(const SolverState *s, long long thr, int g) {
+  const long long nc = s->h_seg_off[g + 1] - s->h_seg_off[g];
+  return thr >= 0 && nc <= std::min(thr, kBlockCap);
+}
+
 // Instances on the block schedule for a split at `thr` cells (-1: none,
-// LLONG_MAX: all): the list (largest first) and the per-instance mask.
+// LLONG_MAX: all up to kBlockCap): the per-instance mask.
 int set_block_split(SolverState *s, long long thr, cudaStream_t st) {
   if (s->mask_for == thr) return 0;
-  std::vector<int> mask(s->nseg, 0), list;
-  for (int g : s->h_order) {
-    const long long nc = s->h_seg_off[g + 1] - s->h_seg_off[g];
-    if (thr >= 0 && nc <= thr) {
+  std::vector<int> mask(s->nseg, 0);
+  s->n_block = 0;
+  for (int g = 0; g < s->nseg; g++)
+    if (on_block(s, thr, g)) {
       mask[g] = 1;
-      list.push_back(g);
+      s->n_block++;
     }
-  }
-  s->n_block = (int)list.size();
   s->n_tile = s->nseg - s->n_block;
   SCUDA(cudaMemcpyAsync(s->block_mask, mask.data(), sizeof(int) * s->nseg, cudaMemcpyHostToDevice, st));
-  if (!list.empty())
-    SCUDA(cudaMemcpyAsync(s->block_inst, list.data(), sizeof(int) * list.size(), cudaMemcpyHostToDevice, st));
-  SCUDA(cudaStreamSynchronize(st));  // the host vectors are read
+  SCUDA(cudaStreamSynchronize(st));  // the host vector is read
   s->mask_for = thr;
   return 0;
 }
 
-template <class T, int TPR>
-int launch_block(SolverState *s, Krylov &k, const TDyNewtonOptions &o, double tol2, cudaStream_t st) {
+// CTAs per instance: 256 cells each in FP32 and 128 in FP64 (whose arithmetic
+// is the longer part), more in batches that fill the SMs eight times over.
+// The launch lasts as long as its longest instance's iterations, not as the
+// batch's work: 192 instances (217 k cells) take 50 times longer than their
+// arithmetic and matrix traffic.
+int block_ctas(long long cells, long long total, int nsm, size_t tsize) {
+  const long long target = std::max<long long>(tsize == 4 ? 256 : 128, total / (8 * nsm));
+  int c = 1;
+  while (c < 8 && c * target < cells) c *= 2;
+  return c;
+}
+
+// Launch classes of the block schedule: where the vectors live and the CTAs
+// per instance, each split by shared memory (a class asks for what its largest
+// instance needs, so small instances keep their residency beside large ones).
+constexpr size_t kBlockSmemMax = 220 * 1024;  // dynamic shared memory of a CTA
+constexpr size_t kBlockSmemSteps[3] = {36 * 1024, 72 * 1024, kBlockSmemMax};
+constexpr int kBlockClasses = 2 * 4 * 3 + 2;
+
+template <class T, int C, int KEEP>
+int launch_block_class(const BlockSolve<T> &B, size_t smem, int nsm, cudaStream_t st) {
+  auto kern = bicgstab_block_kernel<T, C, KEEP>;
+  if (smem > 48 * 1024) SCUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kBlockSmemMax));
+  int per_sm = 0;
+  SCUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, kBlockThreads, smem));
+  const int grid = C * std::max(1, std::min(B.ninst, nsm * std::max(per_sm, 1) / C));
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3((unsigned)grid);
+  cfg.blockDim = dim3(kBlockThreads);
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = st;
+  cudaLaunchAttribute at[1];
+  at[0].id = cudaLaunchAttributeClusterDimension;
+  at[0].val.clusterDim.x = C;
+  at[0].val.clusterDim.y = 1;
+  at[0].val.clusterDim.z = 1;
+  cfg.attrs = at;
+  cfg.numAttrs = C > 1 ? 1 : 0;
+  SCUDA(cudaLaunchKernelEx(&cfg, kern, B));
+  return 0;
+}
+
+// The active instances of the block schedule, one launch per class, side by
+// side on streams of their own joined into st.
+template <class T>
+int launch_block(SolverState *s, Krylov &k, const TDyNewtonOptions &o, double tol2, long long thr,
+                 const std::vector<int> &act, cudaStream_t st) {
+  int ierr, dev = 0, nsm = 0;
+  SCUDA(cudaGetDevice(&dev));
+  SCUDA(cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev));
+  auto cells = [&](int g) { return s->h_seg_off[g + 1] - s->h_seg_off[g]; };
+  // matrix slots of a CTA's rows at most: its slices are as wide as the widest in HBM
+  auto slots_of = [&](int C, int g) {
+    long long width = 0;
+    for (int k = s->h_slice_off[g]; k < s->h_slice_off[g + 1]; k++)
+      width = std::max(width, s->h_sell_off[k + 1] - s->h_sell_off[k]);
+    return (size_t)width * ((owned_cells(cells(g), C) + 31) / 32);
+  };
+  auto smem_of = [&](int keep, int C, int g) {
+    const int nc = cells(g), nc2 = s->h_inst_line_off[g + 1] - s->h_inst_line_off[g];
+    return block_smem<T>(keep, nc, (nc2 + C - 1) / C, nc / nc2, keep == KEEP_MATRIX ? slots_of(C, g) : 0, C);
+  };
+  long long total = 0, ctas = 0;
+  for (int g = 0; g < s->nseg; g++)
+    if (act[g] && on_block(s, thr, g)) total += cells(g);
+  for (int g = 0; g < s->nseg; g++)
+    if (act[g] && on_block(s, thr, g)) ctas += block_ctas(cells(g), total, nsm, sizeof(T));
+  struct Class {
+    std::vector<int> inst;
+    size_t smem = 0, slots = 0;
+  } cls[kBlockClasses];
+  for (int g : s->h_order) {
+    if (!act[g] || !on_block(s, thr, g)) continue;
+    int c = block_ctas(cells(g), total, nsm, sizeof(T)), lg = c == 8 ? 3 : c == 4 ? 2 : c == 2 ? 1 : 0;
+    while (lg < 3 && smem_of(KEEP_ALL, 1 << lg, g) > kBlockSmemMax) lg++;
+    int i = -1, keep = KEEP_ALL;
+    // the matrix in shared memory, in batches of many CTAs where it leaves two
+    // per SM (28 instances up to 5,264 cells: 2.0 ms against 2.5 ms with the
+    // half limit; 192 instances: 4.6 against 3.8 ms)
+    size_t smem = smem_of(KEEP_MATRIX, 1 << lg, g);
+    if (smem <= (ctas <= 2 * nsm ? kBlockSmemMax : kBlockSmemMax / 2))
+      keep = KEEP_MATRIX;
+    else
+      smem = smem_of(KEEP_ALL, 1 << lg, g);
+    if (smem <= kBlockSmemMax) {
+      int step = 0;
+      while (smem > kBlockSmemSteps[step]) step++;
+      i = ((3 - lg) * 2 + keep) * 3 + 2 - step;  // larger instances first
+    } else if ((smem = smem_of(KEEP_Z, 8, g)) <= kBlockSmemMax) {
+      i = kBlockClasses - 2;
+    } else {
+      smem = smem_of(KEEP_NONE, 1, g);
+      i = kBlockClasses - 1;
+    }
+    cls[i].inst.push_back(g);
+    // (the matrix lies behind everything else: its slots are the class's)
+    const size_t slots = keep == KEEP_MATRIX ? slots_of(1 << lg, g) : 0;
+    cls[i].slots = std::max(cls[i].slots, slots);
+    cls[i].smem = std::max(cls[i].smem, smem - (sizeof(T) + sizeof(uint16_t)) * slots);
+  }
+  for (Class &c : cls) c.smem += (sizeof(T) + sizeof(uint16_t)) * c.slots;
+  s->h_block_list.clear();
+  int first[kBlockClasses], used = 0;
+  for (int i = 0; i < kBlockClasses; i++) {
+    first[i] = (int)s->h_block_list.size();
+    s->h_block_list.insert(s->h_block_list.end(), cls[i].inst.begin(), cls[i].inst.end());
+    used += !cls[i].inst.empty();
+  }
+  if (!used) return 0;
+  SCUDA(cudaMemcpyAsync(s->block_inst, s->h_block_list.data(), sizeof(int) * s->h_block_list.size(),
+                        cudaMemcpyHostToDevice, st));
+  SCUDA(cudaMemsetAsync(s->ticket, 0, kBlockClasses * sizeof(int), st));
   BlockSolve<T> B;
-  B.ninst = s->n_block;
-  B.inst = s->block_inst;
-  B.ticket = s->ticket;
   B.seg_off = s->seg_off;
   B.inst_line_off = s->inst_line_off;
-  B.line_off = s->line_off;
-  B.line_cells = s->line_cells;
+  B.slice_off = s->slice_off;
+  B.sell_off = s->sell_off;
+  B.rowptr = s->rowptr;
+  B.A = (const T *)k.sell;
+  B.col = s->sell_col;
   B.la = (const T *)k.la;
   B.lcp = (const T *)k.lcp;
   B.linv = (const T *)k.linv;
-  B.rowptr = s->rowptr;
-  B.colidx = s->colidx;
-  B.A = (const T *)k.Jv;
-  B.b = (T *)k.b;
-  B.r = (T *)k.r;
-  B.r0 = (T *)k.r0;
-  B.p = (T *)k.p;
-  B.v = (T *)k.v;
-  B.s = (T *)k.s;
-  B.t = (T *)k.t;
-  B.ph = (T *)k.ph;
-  B.sh = (T *)k.sh;
-  B.y = (T *)k.y;
-  B.newt_active = s->newt_active;
+  B.F = s->F;
+  T *const vec[8] = {(T *)k.r0, (T *)k.r, (T *)k.p, (T *)k.v, (T *)k.s, (T *)k.t, (T *)k.ph, (T *)k.y};
+  for (int i = 0; i < 8; i++) B.vec[i] = vec[i];
+  B.z = (T *)k.sh;
+  B.x = (T *)k.b;
   B.lin_its = s->lin_its;
   B.tol2 = tol2;
   B.max_it = o.linear_max_it;
-  int dev = 0, nsm = 0, per_sm = 0;
-  SCUDA(cudaGetDevice(&dev));
-  SCUDA(cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev));
-  SCUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, bicgstab_block_kernel<T, TPR>, kBlockThreads, 0));
-  const int grid = std::max(1, std::min(s->n_block, nsm * std::max(per_sm, 1)));
-  SCUDA(cudaMemsetAsync(s->ticket, 0, sizeof(int), st));
-  bicgstab_block_kernel<T, TPR><<<grid, kBlockThreads, 0, st>>>(B);
-  SCUDA(cudaGetLastError());
+  if (used > 1) {
+    if (!s->fork) {
+      s->device = dev;
+      if ((ierr = device_pool_event(&s->fork))) return ierr;
+      for (int i = 0; i < 3; i++) {
+        if ((ierr = device_pool_stream(&s->side[i]))) return ierr;
+        if ((ierr = device_pool_event(&s->joined[i]))) return ierr;
+      }
+    }
+    SCUDA(cudaEventRecord(s->fork, st));
+    for (int i = 0; i < std::min(used - 1, 3); i++) SCUDA(cudaStreamWaitEvent(s->side[i], s->fork, 0));
+  }
+  int launched = 0;
+  for (int i = 0; i < kBlockClasses; i++) {
+    if (cls[i].inst.empty()) continue;
+    B.ninst = (int)cls[i].inst.size();
+    B.inst = s->block_inst + first[i];
+    B.ticket = s->ticket + i;
+    const size_t smem = cls[i].smem;
+    const cudaStream_t ls = launched % 4 == 0 ? st : s->side[launched % 4 - 1];
+    B.slots = (int)cls[i].slots;
+    switch (i / 3) {
+      case 0: ierr = launch_block_class<T, 8, KEEP_MATRIX>(B, smem, nsm, ls); break;
+      case 1: ierr = launch_block_class<T, 8, KEEP_ALL>(B, smem, nsm, ls); break;
+      case 2: ierr = launch_block_class<T, 4, KEEP_MATRIX>(B, smem, nsm, ls); break;
+      case 3: ierr = launch_block_class<T, 4, KEEP_ALL>(B, smem, nsm, ls); break;
+      case 4: ierr = launch_block_class<T, 2, KEEP_MATRIX>(B, smem, nsm, ls); break;
+      case 5: ierr = launch_block_class<T, 2, KEEP_ALL>(B, smem, nsm, ls); break;
+      case 6: ierr = launch_block_class<T, 1, KEEP_MATRIX>(B, smem, nsm, ls); break;
+      case 7: ierr = launch_block_class<T, 1, KEEP_ALL>(B, smem, nsm, ls); break;
+      default:
+        ierr = i == kBlockClasses - 2 ? launch_block_class<T, 8, KEEP_Z>(B, smem, nsm, ls)
+                                      : launch_block_class<T, 1, KEEP_NONE>(B, smem, nsm, ls);
+    }
+    if (ierr) return ierr;
+    launched++;
+  }
+  for (int i = 0; i < std::min(launched - 1, 3); i++) {
+    SCUDA(cudaEventRecord(s->joined[i], s->side[i]));
+    SCUDA(cudaStreamWaitEvent(st, s->joined[i], 0));
+  }
   return 0;
 }
 
@@ -1083,38 +1705,23 @@ int launch_block(SolverState *s, Krylov &k, const TDyNewtonOptions &o, double to
 // schedule and the others on the tile schedule; its = inner iterations.
 template <class T>
 int solve_scheduled(SolverState *s, Krylov &k, const TDyNewtonOptions &o, double tol2, long long thr,
-                    cudaStream_t st, std::vector<int> &its) {
+                    const std::vector<int> &newt_act, cudaStream_t st, std::vector<int> &its) {
   int ierr;
   const int n = s->n, ns = s->nseg;
   if ((ierr = set_block_split(s, thr, st))) return ierr;
-  init_kernel<T><<<nblk(n, 256), 256, 0, st>>>(n, s->cell_seg, s->newt_active, s->F, (T *)k.b, (T *)k.r, (T *)k.r0,
-                                               (T *)k.p, (T *)k.v, (T *)k.y);
-  {
+  SCUDA(cudaMemsetAsync(s->lin_its, 0, sizeof(int) * ns, st));
+  if (s->n_tile > 0) {
+    init_kernel<T><<<nblk(n, 256), 256, 0, st>>>(n, s->cell_seg, s->newt_active, s->F, (T *)k.b, (T *)k.r, (T *)k.r0,
+                                                 (T *)k.p, (T *)k.v, (T *)k.y);
+    SCUDA(cudaGetLastError());
+  }
+  if (s->n_block > 0 && (ierr = launch_block<T>(s, k, o, tol2, thr, newt_act, st))) return ierr;
+  if (s->n_tile > 0) {
     Emit em(st);
     dot<T>(s, (T *)k.b, (T *)k.b, nullptr, nullptr, S_BNORM2, 0, em);
-  }
-  SCUDA(cudaMemsetAsync(s->lin_its, 0, sizeof(int) * ns, st));
-  init_scalars_kernel<<<nblk(ns, 128), 128, 0, st>>>(ns, s->newt_active, s->block_mask, s->lin_active, s->lin_its,
-                                                     s->scal);
-  SCUDA(cudaGetLastError());
-  if (s->n_block > 0) {
-    switch (k.tpr) {
-      case 1:
-        ierr = launch_block<T, 1>(s, k, o, tol2, st);
-        break;
-      case 2:
-        ierr = launch_block<T, 2>(s, k, o, tol2, st);
-        break;
-      case 4:
-        ierr = launch_block<T, 4>(s, k, o, tol2, st);
-        break;
-      default:
-        ierr = launch_block<T, 8>(s, k, o, tol2, st);
-        break;
-    }
-    if (ierr) return ierr;
-  }
-  if (s->n_tile > 0) {
+    init_scalars_kernel<<<nblk(ns, 128), 128, 0, st>>>(ns, s->newt_active, s->block_mask, s->lin_active, s->lin_its,
+                                                       s->scal);
+    SCUDA(cudaGetLastError());
     std::vector<int> act(ns);
     const int check_every = 8;
     for (int it = 0; it < o.linear_max_it; it += check_every) {
@@ -1143,27 +1750,34 @@ std::mutex g_sched_mutex;
 std::vector<std::pair<long long, long long>> g_sched;  // (class key, split)
 
 template <class T>
-int tune_schedule(SolverState *s, Krylov &k, const TDyNewtonOptions &o, double tol2, cudaStream_t st,
-                  long long *thr) {
+long long sched_key(const SolverState *s) {
   long long maxc = 0;
   for (int g = 0; g < s->nseg; g++) maxc = std::max<long long>(maxc, s->h_seg_off[g + 1] - s->h_seg_off[g]);
   int lg = 0;
   while ((1LL << lg) < maxc) lg++;
   const int cls = s->nseg == 1 ? 0 : (s->nseg < 64 ? 1 : 2);
-  const long long key = ((long long)sizeof(T) << 16) | ((long long)cls << 8) | lg;
-  if (s->block_max_cells != -2) {  // this handle's choice
-    *thr = s->block_max_cells;
-    return 0;
-  }
-  {
+  return ((long long)sizeof(T) << 16) | ((long long)cls << 8) | lg;
+}
+
+// The split already chosen for this handle or its size class; false if none.
+template <class T>
+bool tuned_schedule(SolverState *s, long long *thr) {
+  if (s->block_max_cells == -2) {
+    const long long key = sched_key<T>(s);
     std::lock_guard<std::mutex> lk(g_sched_mutex);
     for (auto &e : g_sched)
-      if (e.first == key) {
-        s->block_max_cells = *thr = e.second;
-        return 0;
-      }
+      if (e.first == key) s->block_max_cells = e.second;
   }
-  std::vector<long long> cand = {-1, LLONG_MAX};
+  *thr = s->block_max_cells;
+  return s->block_max_cells != -2;
+}
+
+template <class T>
+int tune_schedule(SolverState *s, Krylov &k, const TDyNewtonOptions &o, double tol2, const std::vector<int> &act,
+                  cudaStream_t st, long long *thr) {
+  const long long key = sched_key<T>(s);
+  std::vector<long long> cand = {-1};
+  if (s->nslices > 0) cand.push_back(LLONG_MAX);
   for (long long c : {4096LL, 16384LL, 65536LL}) {
     int below = 0;
     for (int g = 0; g < s->nseg; g++) below += (s->h_seg_off[g + 1] - s->h_seg_off[g]) <= c;
@@ -1175,9 +1789,9 @@ int tune_schedule(SolverState *s, Krylov &k, const TDyNewtonOptions &o, double t
   long long best_thr = -1;
   for (long long c : cand) {
     int ierr;
-    if ((ierr = solve_scheduled<T>(s, k, o, tol2, c, st, its))) return ierr;  // warm-up
+    if ((ierr = solve_scheduled<T>(s, k, o, tol2, c, act, st, its))) return ierr;  // warm-up
     const auto t0 = std::chrono::steady_clock::now();
-    if ((ierr = solve_scheduled<T>(s, k, o, tol2, c, st, its))) return ierr;
+    if ((ierr = solve_scheduled<T>(s, k, o, tol2, c, act, st, its))) return ierr;
     const double ms = std::chrono::duration<double, std::milli>(std::chrono::steady_clock::now() - t0).count();
     s->tune_ms.push_back(ms);
     if (ms < best) {
@@ -1193,29 +1807,17 @@ int tune_schedule(SolverState *s, Krylov &k, const TDyNewtonOptions &o, double t
   return 0;
 }
 
+// What the tile schedule needs for the current Jacobian: the CSR copy of its
+// values in the inner precision, the threads per row of its products and the
+// graph of one iteration.  The graph is built with the explicit graph API, not
+// by stream capture: a capture is invalidated by device-wide operations that
+// other threads issue meanwhile (a cudaFree, a device synchronisation), which
+// a server running many handles at once cannot rule out.  The cluster launches
+// depend on this solve's cluster count: rebuild for every solve.
 template <class T>
-int linear_solve(SolverState *s, Krylov &k, const TDyNewtonOptions &o, cudaStream_t st, long long *lin_total,
-                 std::vector<int> &inst_lin_its) {
-  int ierr;
-  if ((ierr = krylov_alloc<T>(s, k, st))) return ierr;
-  if ((ierr = autotune_spmv<T>(s, k, o.spmv_threads, st))) return ierr;  // uses b and v as scratch before they are set
-  const int n = s->n, ns = s->nseg;
-  SCUDA(cudaEventRecord(s->tev[2], st));
-  cast_kernel<T><<<nblk(s->nnz, 256), 256, 0, st>>>(s->nnz, s->J, (T *)k.Jv);
-  s->precond_used = TDY_PRECOND_LINES;
-  if (o.precond == TDY_PRECOND_CLUSTERS && (ierr = cluster_setup<T>(s, k, o.cluster_threshold, st))) return ierr;
-  if (s->precond_used == TDY_PRECOND_LINES)
-    line_factor_kernel<T><<<nblk(s->nlines, 128), 128, 0, st>>>(s->nlines, s->line_off, s->pos_d, s->pos_lo,
-                                                                 s->pos_hi, s->J, (T *)k.la, (T *)k.lcp, (T *)k.linv);
-  SCUDA(cudaEventRecord(s->tev[3], st));
-  const double tol2 = o.linear_rtol * o.linear_rtol;
-  // The graph of one iteration is built with the explicit graph API, not by
-  // stream capture: a capture is invalidated by device-wide operations that
-  // other threads issue meanwhile (a cudaFree, a device synchronisation),
-  // which a server running many handles at once cannot rule out.  The cluster
-  // launches depend on this solve's cluster count: rebuild for every solve.
-  if (!k.graph || s->linear_rtol != o.linear_rtol || k.graph_precond != s->precond_used || k.graph_tpr != k.tpr ||
-      s->precond_used == TDY_PRECOND_CLUSTERS) {
+int tile_setup(SolverState *s, Krylov &k, const TDyNewtonOptions &o, double tol2, cudaStream_t st) {
+  if ((!k.graph || s->linear_rtol != o.linear_rtol || k.graph_precond != s->precond_used || k.graph_tpr != k.tpr ||
+       s->precond_used == TDY_PRECOND_CLUSTERS)) {
     if (k.graph) cudaGraphExecDestroy(k.graph);
     k.graph = nullptr;
     cudaGraph_t g = nullptr;
@@ -1234,19 +1836,61 @@ int linear_solve(SolverState *s, Krylov &k, const TDyNewtonOptions &o, cudaStrea
     k.graph_tpr = k.tpr;
     s->linear_rtol = o.linear_rtol;
   }
-  std::vector<int> its(ns);
-  // the schedule split: chosen by timing on the first solve of this size
-  // class (process-wide), or given by the options; clusters: tile only
+  return 0;
+}
+
+// act: the instances to solve (the host's copy of newt_active)
+template <class T>
+int linear_solve(SolverState *s, Krylov &k, const TDyNewtonOptions &o, const std::vector<int> &act, cudaStream_t st,
+                 long long *lin_total, std::vector<int> &inst_lin_its) {
+  int ierr;
+  if ((ierr = krylov_alloc<T>(s, k, st))) return ierr;
+  // the schedule split: given by the options, chosen before, or (lines, below)
+  // by timing on the first solve of this size class; clusters: tile only
   long long thr = -1;
-  if (s->precond_used == TDY_PRECOND_LINES) {
-    if (o.schedule == TDY_SCHEDULE_TILE)
-      thr = -1;
-    else if (o.schedule == TDY_SCHEDULE_BLOCK)
+  bool tune = false;
+  if (o.precond != TDY_PRECOND_CLUSTERS) {
+    if (o.schedule == TDY_SCHEDULE_BLOCK)
       thr = LLONG_MAX;
-    else if ((ierr = tune_schedule<T>(s, k, o, tol2, st, &thr)))
-      return ierr;
+    else if (o.schedule != TDY_SCHEDULE_TILE)
+      tune = !tuned_schedule<T>(s, &thr);
   }
-  if ((ierr = solve_scheduled<T>(s, k, o, tol2, thr, st, its))) return ierr;
+  bool tile = tune, block = tune && s->nslices > 0;
+  if (!tune)
+    for (int g = 0; g < s->nseg; g++) (on_block(s, thr, g) ? block : tile) = true;
+  if (block) {
+    if ((ierr = sell_setup(s, st))) return ierr;
+    if (!k.sell) {
+      if ((ierr = dmem_alloc(&k.sell, (size_t)s->h_sell_off.back() * sizeof(T), st))) return ierr;
+      s->allocs.push_back(k.sell);
+    }
+  }
+  if (tile) {
+    if (!k.Jv) {
+      if ((ierr = dmem_alloc(&k.Jv, (size_t)s->nnz * sizeof(T), st))) return ierr;
+      s->allocs.push_back(k.Jv);
+    }
+    if ((ierr = autotune_spmv<T>(s, k, o.spmv_threads, st))) return ierr;  // uses b and v as scratch before they are set
+  }
+  const int ns = s->nseg;
+  SCUDA(cudaEventRecord(s->tev[2], st));
+  if (tile) cast_kernel<T><<<nblk(s->nnz, 256), 256, 0, st>>>(s->nnz, s->J, (T *)k.Jv);
+  if (block)
+    sell_fill_kernel<T, double><<<nblk(s->nslices, kSliceWarps), 32 * kSliceWarps, 0, st>>>(
+        s->nslices, s->slice_row, s->slice_end, s->sell_off, s->cell_seg, s->newt_active, s->seg_off, s->rowptr, s->J,
+        (T *)k.sell);
+  s->precond_used = TDY_PRECOND_LINES;
+  if (o.precond == TDY_PRECOND_CLUSTERS && (ierr = cluster_setup<T>(s, k, o.cluster_threshold, st))) return ierr;
+  if (s->precond_used == TDY_PRECOND_LINES)
+    line_factor_kernel<T><<<nblk(s->nlines, 128), 128, 0, st>>>(s->nlines, s->line_off, s->line_cells, s->pos_d,
+                                                                 s->pos_lo, s->pos_hi, s->J, (T *)k.la, (T *)k.lcp,
+                                                                 (T *)k.linv);
+  SCUDA(cudaEventRecord(s->tev[3], st));
+  const double tol2 = o.linear_rtol * o.linear_rtol;
+  if (tile && (ierr = tile_setup<T>(s, k, o, tol2, st))) return ierr;
+  std::vector<int> its(ns);
+  if (tune && (ierr = tune_schedule<T>(s, k, o, tol2, act, st, &thr))) return ierr;
+  if ((ierr = solve_scheduled<T>(s, k, o, tol2, thr, act, st, its))) return ierr;
   SCUDA(cudaEventRecord(s->tev[4], st));
   for (int v : its) *lin_total += v;
   inst_lin_its = its;
@@ -1299,6 +1943,21 @@ int solver_init(_p_TDy *t) {
     seg_chunk.push_back((int)chunk_off.size() - 1);
   }
   s->nchunks = (int)chunk_off.size() - 1;
+  // slices of the block schedule's matrix layout
+  s->h_slice_off.assign(1, 0);
+  s->h_sell_off.assign(1, 0);
+  for (int g = 0; g < s->nseg; g++) {
+    if (seg_off[g + 1] - seg_off[g] <= kBlockCap)
+      for (int i = seg_off[g]; i < seg_off[g + 1]; i += 32) {
+        int width = 0;
+        for (int j = i; j < std::min(i + 32, seg_off[g + 1]); j++)
+          width = std::max(width, su.rowptr[j + 1] - su.rowptr[j]);
+        s->h_slice_row.push_back(i);
+        s->h_sell_off.push_back(s->h_sell_off.back() + 32LL * width);
+      }
+    s->h_slice_off.push_back((int)s->h_slice_row.size());
+  }
+  s->nslices = (int)s->h_slice_row.size();
   s->h_seg_off = seg_off;
   s->h_inst_line_off = inst_line_off;
   s->h_order.resize(s->nseg);
@@ -1339,7 +1998,7 @@ int solver_init(_p_TDy *t) {
   ar.up(&s->inst_line_off, inst_line_off);
   ar.work(&s->block_inst, s->nseg);
   ar.work(&s->block_mask, s->nseg);
-  ar.work(&s->ticket, 1);
+  ar.work(&s->ticket, kBlockClasses);
   if ((ierr = ar.commit(s->st))) return ierr;
   s->allocs.push_back(ar.base);
   // the allocations and uploads complete before any other stream uses them
@@ -1493,7 +2152,7 @@ int device_be_solve(_p_TDy *t, double dt, double *dU, const TDyNewtonOptions &o,
       // so it is the same alone and in a batch.
       TDyNewtonOptions o32 = o;
       o32.linear_max_it = std::min(o.linear_max_it, std::max(20, o.linear_max_it / 4));
-      ierr = linear_solve<float>(s, s->k32, o32, st, &lin_total, lin_its);
+      ierr = linear_solve<float>(s, s->k32, o32, act, st, &lin_total, lin_its);
       if (ierr) return ierr;
       if ((ierr = add_linear_times(s, &t_prec, &t_kry))) return ierr;
       std::vector<int> redo(ns, 0);
@@ -1503,7 +2162,7 @@ int device_be_solve(_p_TDy *t, double dt, double *dU, const TDyNewtonOptions &o,
       if (any_redo) {
         SCUDA(cudaMemcpyAsync(s->newt_active, redo.data(), sizeof(int) * ns, cudaMemcpyHostToDevice, st));
         std::vector<int> lin64;
-        if ((ierr = linear_solve<double>(s, s->k64, o, st, &lin_total, lin64))) return ierr;
+        if ((ierr = linear_solve<double>(s, s->k64, o, redo, st, &lin_total, lin64))) return ierr;
         if ((ierr = add_linear_times(s, &t_prec, &t_kry))) return ierr;
         cast_masked_kernel<<<nblk(n, 256), 256, 0, st>>>(n, s->cell_seg, s->newt_active, (const double *)s->k64.y,
                                                          (float *)s->k32.y);
@@ -1517,7 +2176,7 @@ int device_be_solve(_p_TDy *t, double dt, double *dU, const TDyNewtonOptions &o,
       }
       y = s->k32.y;
     } else {
-      ierr = linear_solve<double>(s, s->k64, o, st, &lin_total, lin_its);
+      ierr = linear_solve<double>(s, s->k64, o, act, st, &lin_total, lin_its);
       if (!ierr) ierr = add_linear_times(s, &t_prec, &t_kry);
       y = s->k64.y;
     }
