@@ -29,17 +29,19 @@ void device_pool_release(int dev, cudaStream_t st, cudaEvent_t ev);
 int device_setup(_p_TDy *t);
 void device_destroy(_p_TDy *t);
 int device_upload_source_sink(_p_TDy *t);
-int device_presolve(_p_TDy *t, const double *dU_prev, void *stream);
+// fp64_curves: the FP64 formulas of the constitutive relations only (the
+// device Newton; see DevArgs)
+int device_presolve(_p_TDy *t, const double *dU_prev, void *stream, bool fp64_curves = false);
 int device_presolve_host(_p_TDy *t, const double *U_prev);
 int device_eval(_p_TDy *t, int form, double time, const double *dU, const double *dUt, double shift, double *dR,
-                double *dJ, void *stream);
+                double *dJ, void *stream, bool fp64_curves = false);
 int device_eval_host(_p_TDy *t, int form, double time, const double *U, const double *Ut, double shift, double *R,
                      double *J);
 int device_launches_per_eval(_p_TDy *t);
 // SNES-form evaluation of the listed instances (blocks) in one launch, one CTA
 // per instance (the same bits as device_eval); the others keep their R and J.
 int device_eval_instances(_p_TDy *t, const double *dU, double *dR, double *dJ, const int *list, int nlist,
-                          void *stream);
+                          void *stream, bool fp64_curves = false);
 bool device_inst_ok(_p_TDy *t);
 int device_synchronize(_p_TDy *t);
 int device_update_state_host(_p_TDy *t, const double *U);

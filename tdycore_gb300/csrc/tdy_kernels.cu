@@ -48,6 +48,7 @@
 #include "tdy_device.h"
 #include "tdy_emit.h"
 #include "tdy_ff.h"
+#include "tdy_pow.h"
 
 namespace tdy {
 
@@ -68,7 +69,7 @@ struct DevArgs {
   // cells
   const double *vol, *poro, *Sr, *sat_param, *rp_param, *ss, *accum_prev;
   const double *lam_sat;  // kr(Se = 1) / mu per cell (saturated cells)
-  double vis;             // water viscosity (constant at Tref and zero salinity)
+  double vis, inv_vis;    // water viscosity (constant at Tref and zero salinity) and 1 / vis
   const int *sat_type, *rp_type;
   // boundary faces
   const int *bnd_cell, *bnd_type, *bnd_has;
@@ -84,6 +85,10 @@ struct DevArgs {
   // canonical interior-hex vertices (SoA, stride nCpad); a launch takes those in [vc0, vc1)
   int nC, nCpad, vc0, vc1;
   const double *Tc;
+  // the curves by the FP64 power functions only: the device Newton's iteration
+  // counts at the rounding floor follow the last bits of the residual, and
+  // stay what they were
+  int fp64_curves;
   int jac_ff;  // Jacobian products of canonical vertices in double-float
   const int *cellc, *facec;
   // generic vertices
@@ -307,11 +312,112 @@ __device__ __forceinline__ void viscosity(int type, double *vis, double *dvis) {
   *dvis = 0.0;
 }
 
+// Saturation and mobility of an unsaturated cell: S, dS/dP, d2S/dP2, kr and
+// dkr/dP.
+struct Curves {
+  double S, dS, d2S, kr, dkr;
+};
+
+// van Genuchten saturation with Mualem relative permeability of the same m,
+// by the identities of their bases: with x = alpha Pc and w = 1 + x^n,
+//   Se = w^-m,  Se^(1/m) = 1/w,  (1 - Se^(1/m))^m = (x^n / w)^m =: t,
+// so kr = sqrt(Se) (1 - t)^2 and, with x^(nm) = x^(n-1),
+//   -dSe/dPc = m n alpha x^(n-1) Se / w,
+//   dkr/dSe = kr / (2 Se) + 2 sqrt(Se) (1 - t) / x.
+// Every power comes from log2 x and log2 w by one exp2_fx (tdy_pow.h): in FP64
+// the four powers and eleven divisions of the plain formulas took a warp 33 k
+// cycles (one cell per lane); the state stage of 204 k unsaturated cells took
+// 0.225 ms and takes 0.035 ms so.
+// The cell's parameters: par = m, alpha, n; p = the Mualem parameters.  False
+// (nothing set) outside the range of the integer powers.
+__device__ __forceinline__ bool vg_mualem(const double *par, const double *p, double Sr, double Pc, bool want_kr,
+                                          bool want_d, bool want_d2, Curves *c) {
+  const double m = par[0], alpha = par[1], n = par[2];
+  const double x = __dmul_rn(Pc, alpha);
+  const int be = (int)((unsigned)__double2hiint(x) >> 20) - 1023;  // (a set sign bit puts it out of range)
+  if (!(be > -300 && be < 300 && m >= 0.00390625 && n <= 32.0 && (abs(be) + 1) * (int)(n + 1.0) < 500)) return false;
+  const fx lx = log2_fx(x), tn = fx_scale(n, lx);
+  const double xn = exp2_fx(tn), w = __dadd_rn(1.0, xn);
+  const fx lw = log2_fx(w), mw = fx_scale(m, lw);
+  const double Se = exp2_fx(fx_neg(mw)), oms = __dadd_rn(1.0, -Sr);
+  c->S = __fma_rn(oms, Se, Sr);
+  if (!want_kr && !want_d) return true;
+  // (the exponent m (n log2 x - log2 w): 1 - t cancels in dry soil)
+  const double t = exp2_fx(fx_scale(m, fx_add(tn, fx_neg(lw))));
+  double g = 0.0, u = 0.0, xi = 0.0, us = 0.0;  // us: x^(n-1) Se
+  if (want_d) {
+    const double wi = exp2_fx(fx_neg(lw)), mn = __dmul_rn(m, n);
+    xi = exp2_fx(fx_neg(lx));
+    u = __dmul_rn(xn, xi);
+    g = __dmul_rn(__dmul_rn(mn, alpha), wi);
+    us = __dmul_rn(u, Se);
+    c->dS = __dmul_rn(__dmul_rn(g, us), oms);
+    if (want_d2) {
+      const double q = __dmul_rn(__dmul_rn(mn, __dmul_rn(__dmul_rn(u, xi), __dmul_rn(alpha, alpha))), __dmul_rn(Se, __dmul_rn(wi, wi)));
+      c->d2S = __dmul_rn(__dmul_rn(oms, q), __dadd_rn(__fma_rn(__dadd_rn(mn, 1.0), xn, -n), 1.0));
+    }
+  }
+  if (!want_kr) return true;
+  if (Se > p[2]) {  // the smoothing cubic (tdycharacteristiccurves.c:607-614)
+    const double dx = p[4], xt = (Se - p[1]) / dx;
+    c->kr = p[5] + xt * (p[6] + xt * (p[7] + xt * p[8]));
+    if (want_d) c->dkr = __dmul_rn((p[6] + xt * (2.0 * p[7] + xt * 3.0 * p[8])) / dx, __dmul_rn(g, us));
+    return true;
+  }
+  const double f = __dadd_rn(1.0, -t), sq = exp2_fx(fx_neg(fx_half(mw)));
+  c->kr = __dmul_rn(sq, __dmul_rn(f, f));
+  if (want_d)
+    c->dkr = __dmul_rn(g, __fma_rn(__dmul_rn(0.5, c->kr), u, __dmul_rn(__dmul_rn(2.0, __dmul_rn(sq, xi)), __dmul_rn(f, us))));
+  return true;
+}
+
+// any curves, in FP64 (out of line: few cells take it, and inlined its powers
+// would set the registers of every kernel)
+__device__ __noinline__ void curves_general(int sat_type, const double *par, int rp_type, const double *p, double Sr,
+                                            double Pc, Curves *c) {
+  saturation(sat_type, par, Sr, Pc, &c->S, &c->dS, &c->d2S);
+  const double Se = (c->S - Sr) / (1.0 - Sr);
+  double dKr_dSe;
+  relperm(rp_type, p, Se, &c->kr, &dKr_dSe);
+  const double dSe_dS = 1.0 / (1.0 - Sr);
+  c->dkr = dKr_dSe * dSe_dS * c->dS;
+}
+
+__device__ __forceinline__ Curves curves_at(const DevArgs &a, int cell, double Pc, bool want_kr, bool want_d,
+                                            bool want_d2) {
+  Curves c = {0.0, 0.0, 0.0, 0.0, 0.0};
+  const double *par = a.sat_param + 3 * (size_t)cell, *p = a.rp_param + 9 * (size_t)cell;
+  const int st = a.sat_type[cell], rt = a.rp_type[cell];
+  const double Sr = a.Sr[cell];
+  if (!(!a.fp64_curves && st == SAT_FUNC_VAN_GENUCHTEN && Pc > 0 && (!want_kr || (rt == REL_PERM_FUNC_MUALEM && p[0] == par[0])) &&
+        vg_mualem(par, p, Sr, Pc, want_kr, want_d, want_d2, &c)))
+    curves_general(st, par, rt, p, Sr, Pc, &c);
+  return c;
+}
+
+// van Genuchten Pc <= 0, Gardner Pc < 0: S = 1, dS = 0
+__device__ __forceinline__ bool saturated_at(int sat_type, double Pc) {
+  return (sat_type == SAT_FUNC_VAN_GENUCHTEN) ? (Pc <= 0) : (Pc < 0);
+}
+
+// S and, with want_d, dS/dP of any cell
+__device__ __forceinline__ Curves cell_saturation(const DevArgs &a, int cell, double Pc, bool want_d) {
+  if (saturated_at(a.sat_type[cell], Pc)) return Curves{1.0, 0.0, 0.0, 0.0, 0.0};
+  return curves_at(a, cell, Pc, false, want_d, false);
+}
+
+// x / vis, correctly rounded but for rare ties, without the FP64 division
+__device__ __forceinline__ double over_vis(const DevArgs &a, double x) {
+  if (a.fp64_curves) return x / a.vis;
+  const double q = __dmul_rn(x, a.inv_vis);
+  return __fma_rn(__fma_rn(-q, a.vis, x), a.inv_vis, q);
+}
+
 // ---------------------------------------------------------------------------
 // 1. cell and boundary-face state
 // Warps take 32-entity chunks in the order chunk = (warp * chunk_mul) mod
 // nchunks (chunk_mul coprime to nchunks): loads stay coalesced within a warp
-// while the unsaturated cells, which cost ~50x more and cluster in space
+// while the unsaturated cells, which cost ~10x more and cluster in space
 // (and therefore in cell numbering), spread over every SM instead of forming
 // a tail of a few slow blocks.
 // entity i: cell i < nc, else boundary face i - nc
@@ -320,46 +426,39 @@ __device__ __forceinline__ void state_entity(const DevArgs &a, int i) {
     const double U = a.U[i];
     const double Pc = a.Pref - U;
     const double P = a.Pref - Pc;
-    const int st = a.sat_type[i];
-    // Saturated cells (van Genuchten Pc <= 0, Gardner Pc < 0): S = 1, dS = 0,
-    // Se = (1 - Sr)/(1 - Sr) = 1 exactly, so kr/mu is the per-cell constant
-    // lam_sat and its pressure derivative is zero.
-    const bool saturated = (st == SAT_FUNC_VAN_GENUCHTEN) ? (Pc <= 0) : (Pc < 0);
-    double S, dS, d2S, lam, dlam;
+    // Saturated cells: Se = (1 - Sr)/(1 - Sr) = 1 exactly, so kr/mu is the
+    // per-cell constant lam_sat and its pressure derivative is zero.
+    double S = 1.0, dS = 0.0, d2S = 0.0, lam, dlam = 0.0;
+    const bool saturated = saturated_at(a.sat_type[i], Pc);
     if (saturated) {
-      S = 1.0;
-      dS = 0.0;
-      d2S = 0.0;
       lam = a.lam_sat[i];
-      dlam = 0.0;
     } else {
-      const double Sr = a.Sr[i];
-      saturation(st, a.sat_param + 3 * (size_t)i, Sr, Pc, &S, &dS, &d2S);
-      double Se = (S - Sr) / (1.0 - Sr);
-      double Kr, dKr_dSe;
-      relperm(a.rp_type[i], a.rp_param + 9 * (size_t)i, Se, &Kr, &dKr_dSe);
-      double dSe_dS = 1.0 / (1.0 - Sr);
-      double dKr_dS = dKr_dSe * dSe_dS;
-      lam = Kr / a.vis;
-      dlam = dKr_dS * dS / a.vis;  // the viscosity does not depend on pressure here
+      const Curves c = curves_at(a, i, Pc, true, a.needJ || a.form == FORM_TS, a.form == FORM_TS && a.needJ);
+      S = c.S;
+      dS = c.dS;
+      d2S = c.d2S;
+      lam = over_vis(a, c.kr);
+      dlam = over_vis(a, c.dkr);  // the viscosity does not depend on pressure here
     }
     double rho, drho, d2rho;
     density(a.rho_type, P, &rho, &drho, &d2rho);
     a.P[i] = P;
-    a.hr[i] = 0.5 * rho;
-    a.hdr[i] = 0.5 * drho;
+    if (a.rho_type != WATER_DENSITY_CONSTANT) {  // (constant: only the other vertices gather rho/2)
+      a.hr[i] = 0.5 * rho;
+      a.hdr[i] = 0.5 * drho;
+    }
     a.lam[i] = lam;
     a.dlam[i] = dlam;
-    a.seep[i] = 0;
     const double poro = a.poro[i], vol = a.vol[i];
-    const double dporo = 0.0;
-    double dmass = rho * dporo * S + drho * poro * S + rho * poro * dS;
+    // d(rho phi S)/dP (the porosity does not depend on pressure)
+    double dmass = rho * poro * dS;
+    if (a.rho_type != WATER_DENSITY_CONSTANT) dmass = drho * poro * S + rho * poro * dS;
     if (a.form == FORM_SNES) {
       const double dtInv = a.shift;  // 1/dt, computed on the host
       double acc = rho * poro * S * vol * dtInv;
       a.acc_a[i] = acc - a.accum_prev[i];
       a.acc_b[i] = a.ss[i];
-      a.jdiag[i] = dmass * vol * dtInv;
+      a.jdiag[i] = saturated && a.rho_type == WATER_DENSITY_CONSTANT ? 0.0 : dmass * vol * dtInv;
     } else if (a.form == FORM_TV) {
       // TDyMPFAOIFunction_TransientVariable (tdympfao_ts_transientvar.c:89-95):
       // Ut holds dM/dt; the Jacobian adds shift * dM/dP * V.
@@ -368,31 +467,24 @@ __device__ __forceinline__ void state_entity(const DevArgs &a, int i) {
       a.jdiag[i] = a.shift * dmass * vol;
     } else {
       const double Ut = a.Ut[i];
-      const double d2poro = 0.0;
-      double d2mass = (dS * rho * dporo + S * drho * dporo + S * rho * d2poro + dS * drho * poro + S * d2rho * poro +
-                       S * drho * dporo + d2S * rho * poro + dS * drho * poro + dS * rho * dporo);
+      // d2(rho phi S)/dP2 with constant porosity
+      const double d2mass = (S * d2rho + 2.0 * (dS * drho) + d2S * rho) * poro;
       a.acc_a[i] = dmass * Ut * vol;
       a.acc_b[i] = a.ss[i] * vol;
       a.jdiag[i] = (a.shift * dmass + d2mass * Ut) * vol;
     }
   } else if (i < a.nc + a.nb) {
     const int b = i - a.nc;
+    if (a.bnd_type[b] == NEUMANN_BC) return;  // no vertex row or column uses it
     const int c = a.bnd_cell[b];
     const double p = a.bnd_has[b] ? a.bnd_val[b] : a.U[c];
     const double Pc = a.Pref - p;
-    const int st = a.sat_type[c];
-    const bool saturated = (st == SAT_FUNC_VAN_GENUCHTEN) ? (Pc <= 0) : (Pc < 0);
     double lam;
-    if (saturated) {
+    if (saturated_at(a.sat_type[c], Pc)) {
       lam = a.lam_sat[c];  // kr(1) / mu with the boundary viscosity (the same constant)
     } else {
-      const double Sr = a.Sr[c];
-      double S, dS, d2S;
-      saturation(st, a.sat_param + 3 * (size_t)c, Sr, Pc, &S, &dS, &d2S);
-      double Se = (S - Sr) / (1.0 - Sr);
-      double Kr, dKr;
-      relperm(a.rp_type[c], a.rp_param + 9 * (size_t)c, Se, &Kr, &dKr);
-      lam = Kr / a.bnd_vis[b];
+      const Curves cv = curves_at(a, c, Pc, true, false, false);
+      lam = cv.kr / a.bnd_vis[b];
     }
     a.P[i] = p;
     a.hr[i] = 0.5 * a.bnd_rho[b];
@@ -411,15 +503,21 @@ __global__ void __launch_bounds__(256) state_kernel(DevArgs a, int e0, int e1, i
   if (i < e1) state_entity(a, i);
 }
 
+// rho/2 and its derivative of every entity for the constant density
+__global__ void __launch_bounds__(256) const_density_kernel(int n, double *hr, double *hdr) {
+  const int i = blockIdx.x * blockDim.x + threadIdx.x;
+  if (i >= n) return;
+  hr[i] = 0.5 * kRhoConst;
+  hdr[i] = 0.0;
+}
+
 // Accumulation at the previous solution (TDyMPFAOSNESPreSolve,
 // tdympfao_snes.c:19-64).
 __global__ void __launch_bounds__(256) presolve_kernel(DevArgs a, const double *Uprev, double *accum_prev) {
   int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= a.nc) return;
-  const double Sr = a.Sr[i];
   const double Pc = a.Pref - Uprev[i];
-  double S, dS, d2S;
-  saturation(a.sat_type[i], a.sat_param + 3 * (size_t)i, Sr, Pc, &S, &dS, &d2S);
+  const double S = cell_saturation(a, i, Pc, false).S;
   double rho, drho, d2rho;
   density(a.rho_type, a.Pref - Pc, &rho, &drho, &d2rho);
   accum_prev[i] = rho * a.poro[i] * S * a.vol[i] / a.dt;
@@ -430,15 +528,13 @@ __global__ void __launch_bounds__(256) presolve_kernel(DevArgs a, const double *
 __global__ void __launch_bounds__(256) tv_kernel(DevArgs a, const double *U, double *C, double *dC) {
   int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= a.nc) return;
-  const double Sr = a.Sr[i];
   const double Pc = a.Pref - U[i];
-  double S, dS, d2S;
-  saturation(a.sat_type[i], a.sat_param + 3 * (size_t)i, Sr, Pc, &S, &dS, &d2S);
+  const Curves c = cell_saturation(a, i, Pc, dC != nullptr);
   double rho, drho, d2rho;
   density(a.rho_type, a.Pref - Pc, &rho, &drho, &d2rho);
   const double poro = a.poro[i], vol = a.vol[i];
-  if (C) C[i] = rho * poro * S * vol;
-  if (dC) dC[i] = (rho * 0.0 * S + drho * poro * S + rho * poro * dS) * vol;
+  if (C) C[i] = rho * poro * c.S * vol;
+  if (dC) dC[i] = (drho * poro * c.S + rho * poro * c.dS) * vol;
 }
 
 // DAE form (TDyMPFAOIFunction_DAE, tdympfao_ts_dae.c:13-84): split the
@@ -464,10 +560,8 @@ __global__ void __launch_bounds__(256) dae_merge_kernel(int n, const double *U2,
 __global__ void __launch_bounds__(256) diag_kernel(DevArgs a, double *Sout, double *mass) {
   int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= a.nc) return;
-  const double Sr = a.Sr[i];
   const double Pc = a.Pref - a.U[i];
-  double S, dS, d2S;
-  saturation(a.sat_type[i], a.sat_param + 3 * (size_t)i, Sr, Pc, &S, &dS, &d2S);
+  const double S = cell_saturation(a, i, Pc, false).S;
   double rho, drho, d2rho;
   density(a.rho_type, a.Pref - Pc, &rho, &drho, &d2rho);
   Sout[i] = S;
@@ -1603,13 +1697,18 @@ int device_setup(_p_TDy *t) {
   ar.up(&a.vol, m.cell_vol);
   ar.up(&a.poro, t->mat.porosity);
   ar.up(&a.Sr, t->mat.Sr);
-  ar.up(&a.sat_param, t->mat.sat_param);
+  // (van Genuchten: the third slot holds n = 1 / (1 - m))
+  std::vector<double> sat_param = t->mat.sat_param;
+  for (int c = 0; c < m.nc; c++)
+    if (t->mat.sat_type[c] == SAT_FUNC_VAN_GENUCHTEN) sat_param[3 * (size_t)c + 2] = 1.0 / (1.0 - sat_param[3 * (size_t)c]);
+  ar.up(&a.sat_param, sat_param);
   ar.up(&a.rp_param, t->mat.relperm_param);
   ar.up(&a.ss, t->mat.source_sink);
   ar.up(&a.sat_type, t->mat.sat_type);
   ar.up(&a.rp_type, t->mat.relperm_type);
   ar.up(&a.lam_sat, t->mat.lam_sat);
   a.vis = t->mat.vis;
+  a.inv_vis = 1.0 / t->mat.vis;
   std::vector<int> bnd_cell(m.nb);
   for (int b = 0; b < m.nb; b++) bnd_cell[b] = m.face_cell1[m.bnd_face[b]];
   ar.up(&a.bnd_cell, bnd_cell);
@@ -1700,6 +1799,12 @@ int device_setup(_p_TDy *t) {
   if ((ierr = ar.commit(d->stream))) return ierr;
   d->allocs.push_back(ar.base);
   CUDA_TRY(cudaMemsetAsync(accum_prev, 0, sizeof(double) * m.nc, d->stream));
+  // what no evaluation changes: no cell seeps; constant density
+  CUDA_TRY(cudaMemsetAsync(a.seep, 0, next, d->stream));
+  if (a.rho_type == WATER_DENSITY_CONSTANT) {
+    const_density_kernel<<<(unsigned)((next + 255) / 256), 256, 0, d->stream>>>(next, a.hr, a.hdr);
+    CUDA_TRY(cudaGetLastError());
+  }
   a.accum_prev = accum_prev;
   if (t->opt.setup_on_device &&
       (ierr = device_canon_trans(t, a.cellc, a.facec, const_cast<double *>(a.Tc), d->stream)))
@@ -1776,11 +1881,12 @@ static int chunk_multiplier(int n) {
   return (int)(m % n);
 }
 
-int device_presolve(_p_TDy *t, const double *dUprev, void *stream) {
+int device_presolve(_p_TDy *t, const double *dUprev, void *stream, bool fp64_curves) {
   DeviceState *d = t->dev;
   cudaStream_t st = stream ? (cudaStream_t)stream : d->stream;
   DevArgs a = d->a;
   a.dt = t->dtime;
+  a.fp64_curves = fp64_curves;
   presolve_kernel<<<nblocks(a.nc, 256), 256, 0, st>>>(a, dUprev, (double *)a.accum_prev);
   CUDA_TRY(cudaGetLastError());
   return note_stream(d, st);
@@ -1873,7 +1979,7 @@ static int launch_eval(const DevArgs &a, cudaStream_t st, cudaEvent_t *events) {
 
 // The arguments of one evaluation.
 static int eval_args(_p_TDy *t, int form, const double *dU, const double *dUt, double shift, double *dR, double *dJ,
-                     DevArgs *out) {
+                     DevArgs *out, bool fp64_curves = false) {
   DeviceState *d = t->dev;
   if (form == FORM_SNES && !(t->dtime > 0.0))
     return set_error(TDY_ERR_USER, "SNES form needs TDySetDtimeForSNESSolver before evaluation");
@@ -1887,17 +1993,18 @@ static int eval_args(_p_TDy *t, int form, const double *dU, const double *dUt, d
   a.needJ = dJ != nullptr;
   a.R = dR;
   a.J = dJ;
+  a.fp64_curves = fp64_curves;
   *out = a;
   return 0;
 }
 
 int device_eval(_p_TDy *t, int form, double time, const double *dU, const double *dUt, double shift, double *dR,
-                double *dJ, void *stream) {
+                double *dJ, void *stream, bool fp64_curves) {
   (void)time;
   DeviceState *d = t->dev;
   cudaStream_t st = stream ? (cudaStream_t)stream : d->stream;
   DevArgs a;
-  int ierr = eval_args(t, form, dU, dUt, shift, dR, dJ, &a);
+  int ierr = eval_args(t, form, dU, dUt, shift, dR, dJ, &a, fp64_curves);
   if (ierr) return ierr;
   ierr = launch_eval(a, st, d->timers ? d->ev : nullptr);
   if (ierr) return ierr;
@@ -1920,13 +2027,13 @@ int device_eval(_p_TDy *t, int form, double time, const double *dU, const double
 static size_t g_inst_smem_granted[kMaxDevices] = {};
 
 int device_eval_instances(_p_TDy *t, const double *dU, double *dR, double *dJ, const int *list, int nlist,
-                          void *stream) {
+                          void *stream, bool fp64_curves) {
   DeviceState *d = t->dev;
   if (!d->inst_ok) return set_error(TDY_ERR_SUP, "instance schedule unavailable for this handle");
   if (nlist <= 0) return 0;
   cudaStream_t st = stream ? (cudaStream_t)stream : d->stream;
   DevArgs a;
-  int ierr = eval_args(t, FORM_SNES, dU, nullptr, 0.0, dR, dJ, &a);
+  int ierr = eval_args(t, FORM_SNES, dU, nullptr, 0.0, dR, dJ, &a, fp64_curves);
   if (ierr) return ierr;
   using Kern = void (*)(DevArgs, const InstRange *, const int *, int, int *);
   const Kern kerns[6] = {instance_eval_kernel<RHO_CONST, false>,   instance_eval_kernel<RHO_CONST, true>,

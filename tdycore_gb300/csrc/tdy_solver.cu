@@ -2039,7 +2039,7 @@ int device_be_solve(_p_TDy *t, double dt, double *dU, const TDyNewtonOptions &o,
   cudaStream_t st = (cudaStream_t)(stream ? stream : device_default_stream(t));
   const int n = s->n, ns = s->nseg;
   t->dtime = dt;
-  if ((ierr = device_presolve(t, dU, st))) return ierr;
+  if ((ierr = device_presolve(t, dU, st, true))) return ierr;
   SCUDA(cudaMemcpyAsync(s->x, dU, sizeof(double) * n, cudaMemcpyDeviceToDevice, st));
   SCUDA(cudaMemcpyAsync(s->xb, dU, sizeof(double) * n, cudaMemcpyDeviceToDevice, st));
   std::vector<double> f0(ns, 0.0), fn(ns, 0.0), g2(ns, 0.0), lam(ns, 1.0);
@@ -2074,8 +2074,8 @@ int device_be_solve(_p_TDy *t, double dt, double *dU, const TDyNewtonOptions &o,
       for (int mode = 0; mode < 2; mode++) {
         for (int rep = 0; rep < 2; rep++) {  // the first run warms up
           SCUDA(cudaEventRecord(e0, st));
-          e = mode == 0 ? device_eval(t, FORM_SNES, 0.0, s->x, nullptr, 0.0, s->F, s->J, st)
-                        : device_eval_instances(t, s->x, s->F, s->J, all_inst.data(), ns, st);
+          e = mode == 0 ? device_eval(t, FORM_SNES, 0.0, s->x, nullptr, 0.0, s->F, s->J, st, true)
+                        : device_eval_instances(t, s->x, s->F, s->J, all_inst.data(), ns, st, true);
           if (e) return e;
           SCUDA(cudaEventRecord(e1, st));
           SCUDA(cudaEventSynchronize(e1));
@@ -2090,8 +2090,8 @@ int device_be_solve(_p_TDy *t, double dt, double *dU, const TDyNewtonOptions &o,
       return 0;
     }
     if (s->eval_mode < 0) s->eval_mode = 0;
-    return s->eval_mode == 1 ? device_eval_instances(t, s->x, s->F, s->J, all_inst.data(), ns, st)
-                             : device_eval(t, FORM_SNES, 0.0, s->x, nullptr, 0.0, s->F, s->J, st);
+    return s->eval_mode == 1 ? device_eval_instances(t, s->x, s->F, s->J, all_inst.data(), ns, st, true)
+                             : device_eval(t, FORM_SNES, 0.0, s->x, nullptr, 0.0, s->F, s->J, st, true);
   };
   auto evaluate = [&](const std::vector<int> *sub = nullptr) -> int {
     int e;
@@ -2100,7 +2100,7 @@ int device_be_solve(_p_TDy *t, double dt, double *dU, const TDyNewtonOptions &o,
       for (int g : *sub) part = part && s->h_seg_off[g + 1] - s->h_seg_off[g] <= 65536;
     SCUDA(cudaEventRecord(s->tev[0], st));
     if (part)
-      e = device_eval_instances(t, s->x, s->F, s->J, sub->data(), (int)sub->size(), st);
+      e = device_eval_instances(t, s->x, s->F, s->J, sub->data(), (int)sub->size(), st, true);
     else
       e = eval_all();
     if (e) return e;
