@@ -274,8 +274,7 @@ typedef struct {
   long long block_max_cells;    /* last inner solve: the split (instances up to this many cells on the block
                                    schedule; -1 none) */
   int fp64_fallback;            /* 1 if Newton went past fp32_max_it and finished with FP64 inner solves */
-  int eval_schedule;            /* evaluation of every instance: 0 three-stage launches, 1 one CTA per
-                                   instance (timed on the handle's first evaluation; the same bits) */
+  int eval_schedule;            /* 0: three-stage launches (the only evaluation) */
   double eval_s;                /* seconds on the solve's stream in F+J evaluations (line-search trials
                                    included) */
   double precond_s;             /* ... in Jacobian copies to the inner solve's precision and
@@ -337,9 +336,8 @@ TDyErrorCode TDyMPFAOIFunctionIJacobianDevice(TDy tdy, double t, const double *d
 TDyErrorCode TDyPreSolveSNESSolverDevice(TDy tdy, const double *dU_prev, void *stream);
 /* Extension for batched handles (TDySetExtrudedMeshes; no reference
  * counterpart): the SNES residual and Jacobian of the listed instances only
- * (host array of ninst instance indices), in one launch with one CTA per
- * instance at a time; the other instances' rows of dR and dJ are left as they
- * are.  Each listed instance gets the same bits as from
+ * (host array of ninst instance indices); the other instances' rows of dR
+ * and dJ are left as they are.  Each listed instance gets the same bits as from
  * TDyMPFAOSNESFunctionJacobianDevice.  For Newton loops in which only some
  * instances still iterate.  TDY_ERR_SUP when the handle's rows are longer
  * than 96 entries. */

@@ -681,8 +681,8 @@ class TDy:
               "TDyMPFAOSNESFunctionJacobianDevice")
 
     def snes_function_jacobian_device_instances(self, dU, dR, dJ, instances, stream=None):
-        """SNES R and J of the listed instances of a batched handle only (one
-        CTA per instance); the other rows of dR and dJ are left as they are."""
+        """SNES R and J of the listed instances of a batched handle only;
+        the other rows of dR and dJ are left as they are."""
         lst = _i32(instances)
         check(lib.TDyMPFAOSNESFunctionJacobianDeviceInstances(self._h, self._ptr(dU), self._ptr(dR), self._ptr(dJ),
                                                               lst.size, lst.ctypes.data_as(_ip),

@@ -38,8 +38,8 @@ int device_eval(_p_TDy *t, int form, double time, const double *dU, const double
 int device_eval_host(_p_TDy *t, int form, double time, const double *U, const double *Ut, double shift, double *R,
                      double *J);
 int device_launches_per_eval(_p_TDy *t);
-// SNES-form evaluation of the listed instances (blocks) in one launch, one CTA
-// per instance (the same bits as device_eval); the others keep their R and J.
+// SNES-form evaluation of the listed instances (blocks), the same bits as
+// device_eval; the others keep their R and J.
 int device_eval_instances(_p_TDy *t, const double *dU, double *dR, double *dJ, const int *list, int nlist,
                           void *stream, bool fp64_curves = false);
 bool device_inst_ok(_p_TDy *t);

@@ -105,19 +105,19 @@ struct DevArgs {
   const long long *cv_jbase, *cv_rbase;
   const unsigned char *cv_slots;
   int max_row_nnz;
+  // instances: of each cell, and (a call on some instances only, else null)
+  // which are evaluated; the others' entities are skipped
+  const int *cell_inst, *inst_on;
   int nS, nSpad, ngc;
   const int *sc_cells, *sc_vc, *gc_cells;
   // outputs
   double *R, *J;
 };
 
-// The entities of one instance (block of a batched handle): cells [c0, c1),
-// boundary faces [b0, b1), canonical vertices [vc0, vc1), other vertices
-// gen_vertex[g0, g1), structured cells sc_cells[s0, s1), other cells
-// gc_cells[gc0, gc1).
-struct InstRange {
-  int c0, c1, b0, b1, vc0, vc1, g0, g1, s0, s1, gc0, gc1;
-};
+// whether the instance of a cell is evaluated
+__device__ __forceinline__ bool inst_skipped(const DevArgs &a, int cell) {
+  return a.inst_on && !a.inst_on[a.cell_inst[cell]];
+}
 
 // timer groups: the state kernel, the vertex kernels, the cell kernels
 static const char *const kKernelNames[3] = {"state_kernel", "vertex_kernel", "cell_kernel"};
@@ -168,14 +168,9 @@ struct DeviceState {
   // recorded after its last enqueue: TDyDestroy waits for them before the
   // stream-ordered frees (which do not synchronise the device)
   std::vector<std::pair<cudaStream_t, cudaEvent_t>> user_streams;
-  // instance schedule (handles whose blocks are laid out contiguously):
-  // per-instance ranges, the list of a call, its ticket; smem bytes per CTA
-  InstRange *inst_rng = nullptr;
-  int *inst_list = nullptr, *inst_ticket = nullptr;
-  std::vector<InstRange> h_inst_rng;
-  std::vector<long long> h_inst_cells;
-  std::vector<int> h_list;
-  size_t inst_smem = 0;
+  // calls on some instances: their flags on the device, and the host's copy
+  int *inst_on = nullptr;
+  std::vector<int> h_on;
   bool inst_ok = false;
   // recorded after every allocation-free evaluation (created at set-up, so
   // that call creates nothing); such calls never overlap, so the last one
@@ -423,6 +418,7 @@ __device__ __forceinline__ double over_vis(const DevArgs &a, double x) {
 // entity i: cell i < nc, else boundary face i - nc
 __device__ __forceinline__ void state_entity(const DevArgs &a, int i) {
   if (i < a.nc) {
+    if (inst_skipped(a, i)) return;
     const double U = a.U[i];
     const double Pc = a.Pref - U;
     const double P = a.Pref - Pc;
@@ -477,6 +473,7 @@ __device__ __forceinline__ void state_entity(const DevArgs &a, int i) {
     const int b = i - a.nc;
     if (a.bnd_type[b] == NEUMANN_BC) return;  // no vertex row or column uses it
     const int c = a.bnd_cell[b];
+    if (inst_skipped(a, c)) return;
     const double p = a.bnd_has[b] ? a.bnd_val[b] : a.U[c];
     const double Pc = a.Pref - p;
     double lam;
@@ -978,6 +975,7 @@ __device__ __forceinline__ void generic_vertex_one(const DevArgs &a, int g) {
   const int nint = a.v_nint[v];
   const int r0 = a.v_row_off[v], nrow = a.v_row_off[v + 1] - r0;
   const int c0 = a.v_col_off[v], ncol = a.v_col_off[v + 1] - c0;
+  if (inst_skipped(a, a.col_ext[c0])) return;
   const double *T = a.trans + a.v_trans_off[v];
   double *Jv = a.scratch + a.v_jv_off[v];
   double *Rv = Jv + nint * nint;
@@ -1059,6 +1057,7 @@ __device__ __forceinline__ void generic_vertex_warp(const DevArgs &a, int block)
   const int nint = a.v_nint[v];
   const int r0 = a.v_row_off[v], nrow = a.v_row_off[v + 1] - r0;
   const int c0 = a.v_col_off[v], ncol = a.v_col_off[v + 1] - c0;
+  if (inst_skipped(a, a.col_ext[c0])) return;  // whole warp
   const double *T = a.trans + a.v_trans_off[v];
   double *Jv = a.scratch + a.v_jv_off[v];
   double *Rv = Jv + nint * nint;
@@ -1165,7 +1164,7 @@ template <int RHO, bool FFJ>
 __global__ void __launch_bounds__(128) vertex_kernel(DevArgs a, int gen_blocks) {
   if ((int)blockIdx.x >= gen_blocks) {
     const int vc = a.vc0 + ((int)blockIdx.x - gen_blocks) * blockDim.x + threadIdx.x;
-    if (vc < a.vc1) canon_vertex_at<RHO, FFJ>(a, vc, threadIdx.x);
+    if (vc < a.vc1 && !inst_skipped(a, a.cellc[vc])) canon_vertex_at<RHO, FFJ>(a, vc, threadIdx.x);
   } else {
     const int g = blockIdx.x * blockDim.x + threadIdx.x;
     if (g < a.ngen) generic_vertex_one(a, g);
@@ -1180,7 +1179,7 @@ __global__ void __launch_bounds__(kPairThreads, 7) vertex_pair_kernel(DevArgs a,
   if ((int)blockIdx.x >= gen_blocks) {
     const int slot = threadIdx.x >> 1, h = threadIdx.x & 1;
     const int vc = a.vc0 + ((int)blockIdx.x - gen_blocks) * (kPairThreads / 2) + slot;
-    if (vc < a.vc1) canon_vertex_pair<RHO>(a, vc, slot, h, kPairThreads / 2);
+    if (vc < a.vc1 && !inst_skipped(a, a.cellc[vc])) canon_vertex_pair<RHO>(a, vc, slot, h, kPairThreads / 2);
   } else {
     const int g = blockIdx.x * blockDim.x + threadIdx.x;
     if (g < a.ngen) generic_vertex_one(a, g);
@@ -1204,8 +1203,10 @@ __device__ __forceinline__ void struct_cell_at(const DevArgs &a, int sidx, int s
   extern __shared__ double rowbuf[];
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   if (sidx - lane >= s_end) return;  // whole warp out of range
-  const bool active = sidx < s_end;
+  bool active = sidx < s_end;
   const int i = active ? a.sc_cells[sidx] : 0;
+  active = active && !inst_skipped(a, i);
+  if (a.inst_on && !__any_sync(0xffffffffu, active)) return;
   const long long P = a.nCpad, Q = a.nSpad;
   const double *S = a.scratch;
   double row[27];
@@ -1267,8 +1268,9 @@ __device__ __forceinline__ void generic_cell_at(const DevArgs &a, int gidx, int 
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const int g0 = gidx - lane;
   if (g0 >= g_end) return;  // whole warp out of range
-  const bool active = gidx < g_end;
+  bool active = gidx < g_end;
   const int i = active ? a.gc_cells[gidx] : -1;
+  active = active && !inst_skipped(a, i);
   if (a.needR && active) {
     const int k0 = a.cv_off[i], k1 = a.cv_off[i + 1];
     double s = 0.0;
@@ -1317,6 +1319,7 @@ __device__ __forceinline__ void generic_cell_warp(const DevArgs &a, int block) {
   if (gidx >= a.ngc) return;  // the second half of the last warp
   const unsigned mask = 0xffffu << (16 * half);
   const int i = a.gc_cells[gidx];
+  if (inst_skipped(a, i)) return;  // whole half-warp
   const int k0 = a.cv_off[i], k1 = a.cv_off[i + 1];
   if (a.needR && hl == 0) {
     double s = 0.0;
@@ -1353,44 +1356,6 @@ __global__ void __launch_bounds__(64) cell_kernel(DevArgs a, int struct_blocks) 
 }
 
 __global__ void __launch_bounds__(32 * kCellWarps) generic_cell_kernel(DevArgs a) { generic_cell_warp(a, blockIdx.x); }
-
-// ---------------------------------------------------------------------------
-// 5. instance schedule: one launch evaluates a list of instances (the blocks
-// of a batched handle), one CTA per instance at a time, taken from a ticket
-// counter; the CTA runs the instance's state, vertex and cell stages with
-// block barriers between them.  Every entity goes through the same device
-// function as in the three-stage launches (vertices and other cells in their
-// thread forms, which give the warp forms' bits), so an instance gets the same
-// bits from either schedule.  The instances not in the list keep their
-// previous R and J.  256 threads with at most 128 registers each (a little
-// spilling in the heaviest stage): measured on 4096 config-4 instances,
-// 11.8 ms for all of them and 2.2 ms for 64, against 14.5 and 3.0 ms with 128
-// threads at 251 registers, and 17.5 ms for the three-stage launches.
-constexpr int kInstThreads = 256;
-
-template <int RHO, bool FFJ>
-__global__ void __launch_bounds__(kInstThreads, 2) instance_eval_kernel(DevArgs a, const InstRange *rng, const int *list,
-                                                                     int nlist, int *ticket) {
-  __shared__ int cur;
-  const int tid = threadIdx.x, bs = blockDim.x;
-  for (;;) {
-    if (tid == 0) cur = atomicAdd(ticket, 1);
-    __syncthreads();
-    const int k = cur;
-    __syncthreads();  // every thread has read the ticket before the next one is drawn
-    if (k >= nlist) return;
-    const InstRange R = rng[list[k]];
-    for (int i = R.c0 + tid; i < R.c1; i += bs) state_entity(a, i);
-    for (int b = R.b0 + tid; b < R.b1; b += bs) state_entity(a, a.nc + b);
-    __syncthreads();
-    for (int vc = R.vc0 + tid; vc < R.vc1; vc += bs) canon_vertex_at<RHO, FFJ>(a, vc, tid);
-    for (int g = R.g0 + tid; g < R.g1; g += bs) generic_vertex_one(a, g);
-    __syncthreads();
-    for (int base = R.s0; base < R.s1; base += bs) struct_cell_at(a, base + tid, R.s1);
-    for (int base = R.gc0; base < R.gc1; base += bs) generic_cell_at(a, base + tid, R.gc1);
-    __syncthreads();
-  }
-}
 
 // ---------------------------------------------------------------------------
 // Host side
@@ -1536,65 +1501,6 @@ static void build_slabs(_p_TDy *t, DeviceState *d) {
     sl.j1 = s.rowptr[cut[k + 1]];
     d->slabs.push_back(sl);
   }
-}
-
-// Entity ranges of each block of the handle for the instance schedule; false
-// when some list does not run through the blocks in order (then the handle
-// evaluates with the three-stage launches only).
-static bool build_inst_ranges(const _p_TDy *t, std::vector<InstRange> &out, std::vector<long long> &cells) {
-  const Mesh &m = t->mesh;
-  const MPFAOSetup &s = t->setup;
-  const int nblk = (int)t->mesh_blocks.size();
-  std::vector<int> cb(nblk + 1, 0), vb(nblk + 1, 0);
-  for (int b = 0; b < nblk; b++) {
-    const ExtrudedInput &e = t->mesh_blocks[b];
-    cb[b + 1] = cb[b] + e.nc2 * e.nlayers;
-    vb[b + 1] = vb[b] + e.nv2 * (e.nlayers + 1);
-  }
-  if (cb[nblk] != m.nc || vb[nblk] != m.nv) return false;
-  auto block_of = [](const std::vector<int> &bounds, int x) {
-    return (int)(std::upper_bound(bounds.begin(), bounds.end(), x) - bounds.begin()) - 1;
-  };
-  // [first, last) position in `list` of the items of each block; false if unordered
-  auto ranges = [&](const std::vector<int> &list, const std::vector<int> &bounds, std::vector<int> &lo,
-                    std::vector<int> &hi, auto key) {
-    lo.assign(nblk, 0);
-    hi.assign(nblk, 0);
-    int prev = 0;
-    std::vector<int> first(nblk, -1), last(nblk, -1);
-    for (int i = 0; i < (int)list.size(); i++) {
-      const int b = block_of(bounds, key(list[i]));
-      if (b < prev) return false;
-      prev = b;
-      if (first[b] < 0) first[b] = i;
-      last[b] = i + 1;
-    }
-    int pos = 0;
-    for (int b = 0; b < nblk; b++) {
-      lo[b] = first[b] < 0 ? pos : first[b];
-      hi[b] = first[b] < 0 ? pos : last[b];
-      pos = hi[b];
-    }
-    return true;
-  };
-  auto ident = [](int x) { return x; };
-  std::vector<int> bcell(m.nb);
-  for (int b = 0; b < m.nb; b++) bcell[b] = m.face_cell1[m.bnd_face[b]];
-  std::vector<int> bidx(m.nb);
-  for (int b = 0; b < m.nb; b++) bidx[b] = b;
-  std::vector<int> blo, bhi, clo, chi, glo, ghi, slo, shi, gclo, gchi;
-  if (!ranges(bidx, cb, blo, bhi, [&](int b) { return bcell[b]; })) return false;
-  if (!ranges(s.canon_vertex, vb, clo, chi, ident)) return false;
-  if (!ranges(s.gen_vertex, vb, glo, ghi, ident)) return false;
-  if (!ranges(s.sc_cells, cb, slo, shi, ident)) return false;
-  if (!ranges(s.gc_cells, cb, gclo, gchi, ident)) return false;
-  out.resize(nblk);
-  cells.resize(nblk);
-  for (int b = 0; b < nblk; b++) {
-    out[b] = InstRange{cb[b], cb[b + 1], blo[b], bhi[b], clo[b], chi[b], glo[b], ghi[b], slo[b], shi[b], gclo[b], gchi[b]};
-    cells[b] = cb[b + 1] - cb[b];
-  }
-  return true;
 }
 
 static int noalloc_resolve(int dev);
@@ -1787,14 +1693,13 @@ int device_setup(_p_TDy *t) {
   ar.work(&d->dJ, d->nnz);
   ar.work(&d->diagS, m.nc);
   ar.work(&d->diagMass, m.nc);
-  // instance schedule: contiguous blocks and rows short enough for one CTA's
-  // shared rows (canonical vertices' 36 per thread, the cell rows)
-  d->inst_smem = (size_t)std::max(36, std::max(27, s.max_row_nnz)) * kInstThreads * sizeof(double);
-  d->inst_ok = s.max_row_nnz <= 96 && build_inst_ranges(t, d->h_inst_rng, d->h_inst_cells);
-  if (d->inst_ok) {
-    ar.up(&d->inst_rng, d->h_inst_rng);
-    ar.work(&d->inst_list, d->h_inst_rng.size());
-    ar.work(&d->inst_ticket, 1);
+  d->inst_ok = s.max_row_nnz <= 96;
+  std::vector<int> cell_inst;
+  if (t->mesh_blocks.size() > 1) {
+    for (size_t b = 0; b < t->mesh_blocks.size(); b++)
+      cell_inst.insert(cell_inst.end(), (size_t)t->mesh_blocks[b].nc2 * t->mesh_blocks[b].nlayers, (int)b);
+    ar.up(&a.cell_inst, cell_inst);
+    ar.work(&d->inst_on, t->mesh_blocks.size());
   }
   if ((ierr = ar.commit(d->stream))) return ierr;
   d->allocs.push_back(ar.base);
@@ -2021,42 +1926,26 @@ int device_eval(_p_TDy *t, int form, double time, const double *dU, const double
   return 0;
 }
 
-// Instance-schedule evaluation (SNES form) of the listed instances (blocks);
-// the others keep their R and J.  TDY_ERR_SUP when the handle has no
-// instance ranges (blocks not contiguous, or rows too long).
-static size_t g_inst_smem_granted[kMaxDevices] = {};
-
+// Evaluation (SNES form) of the listed instances (blocks): the three stages
+// with the other instances' entities skipped, which keep their R and J.  The
+// skipped threads cost a load and a test each; one CTA per instance, which no
+// launch outlasts, took longer than an evaluation of every instance.
 int device_eval_instances(_p_TDy *t, const double *dU, double *dR, double *dJ, const int *list, int nlist,
                           void *stream, bool fp64_curves) {
   DeviceState *d = t->dev;
-  if (!d->inst_ok) return set_error(TDY_ERR_SUP, "instance schedule unavailable for this handle");
+  if (!d->inst_ok) return set_error(TDY_ERR_SUP, "rows of more than 96 entries: no evaluation of single instances");
   if (nlist <= 0) return 0;
   cudaStream_t st = stream ? (cudaStream_t)stream : d->stream;
   DevArgs a;
   int ierr = eval_args(t, FORM_SNES, dU, nullptr, 0.0, dR, dJ, &a, fp64_curves);
   if (ierr) return ierr;
-  using Kern = void (*)(DevArgs, const InstRange *, const int *, int, int *);
-  const Kern kerns[6] = {instance_eval_kernel<RHO_CONST, false>,   instance_eval_kernel<RHO_CONST, true>,
-                         instance_eval_kernel<RHO_NODERIV, false>, instance_eval_kernel<RHO_NODERIV, true>,
-                         instance_eval_kernel<RHO_EXP, false>,     instance_eval_kernel<RHO_EXP, true>};
-  const Kern kern = kerns[2 * rho_mode(a) + (a.jac_ff ? 1 : 0)];
-  if (d->inst_smem > 48 * 1024) {
-    std::lock_guard<std::mutex> lk(g_dev_mutex);
-    if (d->inst_smem > g_inst_smem_granted[d->device]) {
-      for (Kern k : kerns)
-        CUDA_TRY(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)d->inst_smem));
-      g_inst_smem_granted[d->device] = d->inst_smem;
-    }
+  if (d->inst_on) {
+    d->h_on.assign(t->mesh_blocks.size(), 0);
+    for (int k = 0; k < nlist; k++) d->h_on[list[k]] = 1;
+    CUDA_TRY(cudaMemcpyAsync(d->inst_on, d->h_on.data(), sizeof(int) * d->h_on.size(), cudaMemcpyHostToDevice, st));
+    a.inst_on = d->inst_on;
   }
-  int nsm = 0, per_sm = 0;
-  CUDA_TRY(cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, d->device));
-  CUDA_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, kInstThreads, d->inst_smem));
-  const int grid = std::max(1, std::min(nlist, nsm * std::max(per_sm, 1)));
-  d->h_list.assign(list, list + nlist);  // read by the copy before the caller's next synchronisation
-  CUDA_TRY(cudaMemcpyAsync(d->inst_list, d->h_list.data(), sizeof(int) * nlist, cudaMemcpyHostToDevice, st));
-  CUDA_TRY(cudaMemsetAsync(d->inst_ticket, 0, sizeof(int), st));
-  kern<<<grid, kInstThreads, d->inst_smem, st>>>(a, d->inst_rng, d->inst_list, nlist, d->inst_ticket);
-  CUDA_TRY(cudaGetLastError());
+  if ((ierr = launch_eval(a, st, nullptr))) return ierr;
   return note_stream(d, st);
 }
 

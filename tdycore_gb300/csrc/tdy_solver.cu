@@ -119,14 +119,9 @@ struct SolverState {
   long long block_max_cells = -2, mask_for = -3;
   int n_block = 0, n_tile = 0;
   std::vector<double> tune_ms;  // measured candidates of the last tuning (ms per linear solve)
-  // evaluation of every instance: -1 not chosen, 0 three-stage launches,
-  // 1 instance schedule (timed on the first evaluation; the same bits)
-  int eval_mode = -1;
-  double eval_ms[2] = {0.0, 0.0};
   // phase timers on the solve's stream: evaluation, Jacobian cast and
   // preconditioner set-up, Krylov iterations (events of the current phase)
   cudaEvent_t tev[5] = {nullptr, nullptr, nullptr, nullptr, nullptr};
-  std::vector<long long> h_inst_cells;
   // device memory: stream-ordered on the handle's stream (allocated there and
   // synchronised at init; freed there when the solver is destroyed, after
   // every solve has synchronised its stream)
@@ -2062,47 +2057,14 @@ int device_be_solve(_p_TDy *t, double dt, double *dU, const TDyNewtonOptions &o,
   // the squared per-instance residual norms into g2
   // `sub` (host list of instances, or null for all): only those instances'
   // states changed since the last evaluation, the others keep F and J
-  std::vector<int> all_inst(ns);
-  for (int g = 0; g < ns; g++) all_inst[g] = g;
-  auto eval_all = [&]() -> int {
-    int e;
-    if (s->eval_mode < 0 && device_inst_ok(t) && ns > 1) {
-      // time both schedules once on this evaluation (they give the same bits)
-      cudaEvent_t e0, e1;
-      SCUDA(cudaEventCreate(&e0));
-      SCUDA(cudaEventCreate(&e1));
-      for (int mode = 0; mode < 2; mode++) {
-        for (int rep = 0; rep < 2; rep++) {  // the first run warms up
-          SCUDA(cudaEventRecord(e0, st));
-          e = mode == 0 ? device_eval(t, FORM_SNES, 0.0, s->x, nullptr, 0.0, s->F, s->J, st, true)
-                        : device_eval_instances(t, s->x, s->F, s->J, all_inst.data(), ns, st, true);
-          if (e) return e;
-          SCUDA(cudaEventRecord(e1, st));
-          SCUDA(cudaEventSynchronize(e1));
-          float ms = 0.f;
-          SCUDA(cudaEventElapsedTime(&ms, e0, e1));
-          s->eval_ms[mode] = ms;
-        }
-      }
-      cudaEventDestroy(e0);
-      cudaEventDestroy(e1);
-      s->eval_mode = s->eval_ms[1] < s->eval_ms[0] ? 1 : 0;
-      return 0;
-    }
-    if (s->eval_mode < 0) s->eval_mode = 0;
-    return s->eval_mode == 1 ? device_eval_instances(t, s->x, s->F, s->J, all_inst.data(), ns, st, true)
-                             : device_eval(t, FORM_SNES, 0.0, s->x, nullptr, 0.0, s->F, s->J, st, true);
-  };
   auto evaluate = [&](const std::vector<int> *sub = nullptr) -> int {
     int e;
-    bool part = sub && (int)sub->size() < ns && device_inst_ok(t);
-    if (part)  // one CTA per instance: only for instances small enough for one SM
-      for (int g : *sub) part = part && s->h_seg_off[g + 1] - s->h_seg_off[g] <= 65536;
+    const bool part = sub && (int)sub->size() < ns && device_inst_ok(t);
     SCUDA(cudaEventRecord(s->tev[0], st));
     if (part)
       e = device_eval_instances(t, s->x, s->F, s->J, sub->data(), (int)sub->size(), st, true);
     else
-      e = eval_all();
+      e = device_eval(t, FORM_SNES, 0.0, s->x, nullptr, 0.0, s->F, s->J, st, true);
     if (e) return e;
     SCUDA(cudaEventRecord(s->tev[1], st));
     seg_dot<double, double>(s, s->F, s->F, nullptr, nullptr, s->fn2, nullptr, st);
@@ -2313,7 +2275,7 @@ int device_be_solve(_p_TDy *t, double dt, double *dU, const TDyNewtonOptions &o,
     stats->cluster_cells = s->precond_used == TDY_PRECOND_CLUSTERS ? s->ncl_cells : 0;
     stats->cluster_cells_diagonal = s->precond_used == TDY_PRECOND_CLUSTERS ? s->ncl_big_cells : 0;
     stats->fp64_fallback = fell_back;
-    stats->eval_schedule = s->eval_mode;
+    stats->eval_schedule = 0;
     stats->eval_s = 1e-3 * t_eval;
     stats->precond_s = 1e-3 * t_prec;
     stats->krylov_s = 1e-3 * t_kry;
