@@ -17,10 +17,8 @@
 //        J_v[nint][nint] (rows and columns: the vertex's internal cells) to a
 //        scratch area it alone owns.  Interior hexahedral vertices use a fixed
 //        octant layout (rows and columns known at compile time, structure-of-
-//        arrays storage read with coalesced loads, one thread each, in
-//        vertex_kernel); the others use per-vertex blocks, one thread each in
-//        the first blocks of vertex_kernel when canonical vertices dominate,
-//        else one warp each in generic_vertex_kernel (a launch of its own).
+//        arrays storage read with coalesced loads); the others use per-vertex
+//        blocks, a few lanes each, in the first blocks of the same launch.
 //   3. cells: sum, in a fixed order, the partials of the cell's vertices into
 //        R[cell] and into the cell's row of the fixed CSR pattern, then add
 //        the accumulation terms (cell_kernel: structured cells, and the
@@ -58,6 +56,14 @@ namespace tdy {
 // generic cell kernel stages one row per warp in shared memory)
 #define TDY_MAX_ROW_NNZ 255
 
+// An other (not canonical) vertex: its rows, columns and internal cells in the
+// packed arrays g_row*, g_col and g_cell, its Trans block and its partials.
+struct __align__(16) GenVertex {
+  long long trans, jv;
+  int row0, col0, cell0;
+  unsigned char nrow, ncol, nint, pad;
+};
+
 struct DevArgs {
   int nc, nb, nv;
   int form;
@@ -79,9 +85,7 @@ struct DevArgs {
   double *P, *hr, *hdr, *lam, *dlam;
   unsigned char *seep;
   double *acc_a, *acc_b, *jdiag;
-  // faces
-  const int *f_up, *f_dn;
-  const double *G;
+  const double *G;  // per face
   // canonical interior-hex vertices (SoA, stride nCpad); a launch takes those in [vc0, vc1)
   int nC, nCpad, vc0, vc1;
   const double *Tc;
@@ -91,13 +95,13 @@ struct DevArgs {
   int fp64_curves;
   int jac_ff;  // Jacobian products of canonical vertices in double-float
   const int *cellc, *facec;
-  // generic vertices
-  int ngen;
-  int gen_warp_doubles;  // shared memory of one generic-vertex warp (doubles)
-  const int *gen_vertex;
-  const int *v_row_off, *v_col_off, *v_nint;
-  const long long *v_trans_off, *v_jv_off;
-  const int *row_face, *row_lup, *row_ldn, *col_ext;
+  // other vertices: gen_lanes threads each, gen_doubles of shared memory
+  int ngen, gen_lanes, gen_apart, gen_doubles, gen_max_row, gen_max_col;
+  const GenVertex *gen;
+  const int *g_col;      // extended index of a column
+  const double *g_rowG;  // gravity coefficient of a row
+  const uchar2 *g_rowc;  // columns of a row's up and down sides
+  const uint2 *g_cell;   // of an internal cell: see gen_cell_program
   const double *trans;
   double *scratch;
   // cell gather
@@ -926,248 +930,192 @@ __device__ __forceinline__ void canon_vertex_pair(const DevArgs &a, int vc, int 
   }
 }
 
-// Entry (c, b) of another vertex's J_v in double-float: the rows r of
-// local cell c, in row order, each add -+w_r T_rb and, where b is the row's
-// up or down cell, -+E; every product at the entry's own power-of-two scale
-// (the largest exponent among its terms), as for the canonical vertices.
-// row_of(k), k < kn, lists the rows to scan; rows not touching c are skipped.
-template <class RowOf>
-__device__ __forceinline__ double gen_entry_ff(int c, int b, int kn, RowOf row_of, const int *lup, const int *ldn,
-                                               const double *w, const double *Eu, const double *Ed, const double *T,
-                                               int ncol) {
-  int mb = 0;
-  for (int k = 0; k < kn; k++) {
-    const int r = row_of(k), lu = lup[r], ld = ldn[r];
-    if (lu != c && ld != c) continue;
-    mb = max(mb, d_bexp(w[r]) + d_bexp(T[(size_t)r * ncol + b]) - 1023);
-    if (b == lu) mb = max(mb, d_bexp(Eu[r]));
-    if (b == ld) mb = max(mb, d_bexp(Ed[r]));
+// ---------------------------------------------------------------------------
+// 3. other vertices (boundary, prismatic, irregular): gen_lanes threads each
+// (pack_generic).  The
+// lanes load the columns' state into shared memory, take the rows (T.P and
+// upwinding: FP64, whose instructions cost a warp the same with few lanes
+// active as with all), then the entries of J_v.  A cell has three faces at a
+// vertex, so an entry has at most three rows; which, with which signs, and the
+// cells on their other sides come packed (gen_cell_program).  Every entry
+// (c, b) is summed over the rows of cell c in row order, each row's T term
+// before its upwind-derivative term.  One warp per vertex with row lists
+// built on the fly took 0.41 ms for 108 k prismatic vertices and 0.74 ms for
+// 532 k boundary vertices of 512 columns.
+
+// bytes: rows 0-2 (255: none), flags (bit k: the cell is row k's up cell),
+// then the local cell on the other side of each row (255: the boundary)
+struct GenCell {
+  int row[3], other[3];
+  unsigned flags;
+};
+__device__ __forceinline__ GenCell gen_cell(uint2 u) {
+  GenCell c;
+#pragma unroll
+  for (int k = 0; k < 3; k++) {
+    c.row[k] = (u.x >> (8 * k)) & 255u;
+    c.other[k] = (u.y >> (8 * k)) & 255u;
   }
-  ff acc = {0.0f, 0.0f};
-  for (int k = 0; k < kn; k++) {
-    const int r = row_of(k), lu = lup[r], ld = ldn[r];
-    if (lu != c && ld != c) continue;
-    const bool isup = lu == c;
-    const double wr = w[r], t = T[(size_t)r * ncol + b];
-    const int bw = d_bexp(wr);
-    const ff p = ff_mul(ff_split_scaled(wr, bw, 1023 - bw), ff_split_scaled(t, d_bexp(t), bw - mb));
-    ff_acc(acc, isup ? ff_neg(p) : p);
-    if (b == lu || b == ld) {
-      const double et = b == lu ? Eu[r] : Ed[r];
-      const ff ef = ff_split_scaled(et, d_bexp(et), 1023 - mb);
-      ff_acc(acc, isup ? ff_neg(ef) : ef);
-    }
-  }
-  return ff_to_d(acc, mb - 1023);
+  c.flags = u.x >> 24;
+  return c;
 }
 
-// ---------------------------------------------------------------------------
-// 3. other vertices.  Both forms below sum every Jacobian entry (c, b) of a
-// vertex block over the rows whose faces touch local cell c in row order,
-// each row's T term before its upwind-derivative terms, so they give the
-// same bits.
-//
-// (a) one thread per vertex, for meshes that are mostly canonical hexahedra
-// (their other vertices are few and small, and share the canonical launch)
-// other vertex gen_vertex[g], one thread
-__device__ __forceinline__ void generic_vertex_one(const DevArgs &a, int g) {
-  const int v = a.gen_vertex[g];
-  const int nint = a.v_nint[v];
-  const int r0 = a.v_row_off[v], nrow = a.v_row_off[v + 1] - r0;
-  const int c0 = a.v_col_off[v], ncol = a.v_col_off[v + 1] - c0;
-  if (inst_skipped(a, a.col_ext[c0])) return;
-  const double *T = a.trans + a.v_trans_off[v];
-  double *Jv = a.scratch + a.v_jv_off[v];
-  double *Rv = Jv + nint * nint;
-
-  double w[TDY_MAX_ROWS], Eu[TDY_MAX_ROWS], Ed[TDY_MAX_ROWS], fl[TDY_MAX_ROWS];
-  for (int r = 0; r < nrow; r++) {
-    const double *Tr = T + (size_t)r * ncol;
+template <bool FFJ>
+__device__ __forceinline__ void generic_vertex_group(const DevArgs &a, int block) {
+  extern __shared__ double sh[];
+  const int L = a.gen_lanes, grp = threadIdx.x / L, lane = threadIdx.x & (L - 1);
+  const int g = block * (128 / L) + grp;
+  if (g >= a.ngen) return;  // whole group
+  const unsigned mask = L == 32 ? 0xffffffffu : ((1u << L) - 1u) << (threadIdx.x & 31 & ~(L - 1));
+  const GenVertex d = a.gen[g];
+  const int *ce = a.g_col + d.col0;
+  if (inst_skipped(a, ce[0])) return;  // whole group
+  const int nrow = d.nrow, ncol = d.ncol, nint = d.nint, R = a.gen_max_row, C = a.gen_max_col;
+  const bool vary = a.rho_type != WATER_DENSITY_CONSTANT;
+  const double *T = a.trans + d.trans;
+  double *Jv = a.scratch + d.jv;
+  // per column: P, kr/mu and its derivative (rho/2 and its derivative where
+  // the density varies), seepage; per row: flux, w, E_up, E_dn, exponent of w
+  double *sP = sh + (size_t)grp * a.gen_doubles, *sl = sP + C, *sd = sl + C, *sh2 = sd + C, *shd = sh2 + (vary ? C : 0);
+  double *fl = shd + (vary ? C : 0), *w = fl + R, *Eu = w + R, *Ed = Eu + R;
+  float2 *wf = reinterpret_cast<float2 *>(w);
+  int *bw = reinterpret_cast<int *>(Ed + R);
+  unsigned char *sp = reinterpret_cast<unsigned char *>(bw + R);
+  for (int c = lane; c < ncol; c += L) {
+    const int e = ce[c];
+    sP[c] = a.P[e];
+    sl[c] = a.lam[e];
+    sd[c] = a.dlam[e];
+    if (vary) {
+      sh2[c] = a.hr[e];
+      shd[c] = a.hdr[e];
+    }
+    sp[c] = a.seep[e];
+  }
+  __syncwarp(mask);
+  for (int r = lane; r < nrow; r += L) {
+    const double *Tr = T + r * ncol;
     double TP = 0.0;
-    for (int c = 0; c < ncol; c++) TP = __fma_rn(Tr[c], a.P[a.col_ext[c0 + c]], TP);
-    const int f = a.row_face[r0 + r];
-    const int up = a.f_up[f], dn = a.f_dn[f];
-    const double G = a.G[f];
-    const double den = __dadd_rn(a.hr[up], a.hr[dn]);
+#pragma unroll 4
+    for (int c = 0; c < ncol; c++) TP = __fma_rn(Tr[c], sP[c], TP);
+    const uchar2 ud = a.g_rowc[d.row0 + r];
+    const int up = ud.x, dn = ud.y;
+    const double G = a.g_rowG[d.row0 + r];
+    const double den = vary ? __dadd_rn(sh2[up], sh2[dn]) : kRhoConst;
     const double q = __fma_rn(den, G, TP);
-    const bool flowdn = q < 0.0;
+    const bool flowdn = dneg(q);
     const int u = flowdn ? up : dn;
-    const double lm = a.lam[u];
-    const bool zero = a.seep[u] != 0;
+    const double lm = sl[u];
+    const bool zero = sp[u] != 0;
     const double wr = zero ? 0.0 : __dmul_rn(den, lm);
     fl[r] = -__dmul_rn(wr, q);
     if (a.needJ) {
-      w[r] = wr;
-      if (zero) {
-        Eu[r] = 0.0;
-        Ed[r] = 0.0;
+      double eu = 0.0, ed = 0.0;
+      if (!zero) {
+        if (vary) {
+          const double dlu = flowdn ? sd[up] : 0.0, dld = flowdn ? 0.0 : sd[dn];
+          const double g2 = q + den * G;
+          eu = shd[up] * lm * g2 + den * dlu * q;
+          ed = shd[dn] * lm * g2 + den * dld * q;
+        } else {
+          const double e = __dmul_rn(__dmul_rn(den, sd[u]), q);
+          eu = flowdn ? e : 0.0;
+          ed = flowdn ? 0.0 : e;
+        }
+      }
+      Eu[r] = eu;
+      Ed[r] = ed;
+      if (FFJ) {
+        const int b = d_bexp(wr);
+        const ff f = ff_split_scaled(wr, b, 1023 - b);
+        wf[r] = make_float2(f.h, f.l);
+        bw[r] = b;
       } else {
-        const double dlu = flowdn ? a.dlam[up] : 0.0, dld = flowdn ? 0.0 : a.dlam[dn];
-        const double g2 = q + den * G;
-        Eu[r] = a.hdr[up] * lm * g2 + den * dlu * q;
-        Ed[r] = a.hdr[dn] * lm * g2 + den * dld * q;
+        w[r] = wr;
       }
     }
   }
+  __syncwarp(mask);
+  const uint2 *prog = a.g_cell + d.cell0;
   if (a.needR) {
-    for (int c = 0; c < nint; c++) {
+    for (int c = lane; c < nint; c += L) {
+      const GenCell gc = gen_cell(prog[c]);
       double s = 0.0;
-      for (int r = 0; r < nrow; r++) {
-        if (a.row_lup[r0 + r] == c) s += fl[r];
-        if (a.row_ldn[r0 + r] == c) s -= fl[r];
-      }
-      Rv[c] = s;
-    }
-  }
-  if (a.needJ && a.jac_ff) {
-    for (int c = 0; c < nint; c++)
-      for (int b = 0; b < nint; b++)
-        Jv[c * nint + b] = gen_entry_ff(c, b, nrow, [](int k) { return k; }, a.row_lup + r0, a.row_ldn + r0, w, Eu, Ed,
-                                        T, ncol);
-  } else if (a.needJ) {
-    for (int c = 0; c < nint; c++) {
-      for (int b = 0; b < nint; b++) Jv[c * nint + b] = 0.0;
-      for (int r = 0; r < nrow; r++) {
-        const int lu = a.row_lup[r0 + r], ld = a.row_ldn[r0 + r];
-        if (lu != c && ld != c) continue;
-        const double sw = (lu == c) ? -w[r] : w[r];
-        const double *Tr = T + (size_t)r * ncol;
-        for (int b = 0; b < nint; b++) Jv[c * nint + b] = fma(sw, Tr[b], Jv[c * nint + b]);
-        const double s = (lu == c) ? -1.0 : 1.0;
-        if (lu >= 0) Jv[c * nint + lu] += s * Eu[r];
-        if (ld >= 0) Jv[c * nint + ld] += s * Ed[r];
-      }
-    }
-  }
-}
-
-// (b) one warp per vertex, for meshes without canonical vertices.  Lanes
-// take the rows for the transmissibility products and upwinding, then the
-// entries of the block; the rows of each local cell come from a list built
-// in shared memory, so the lanes of an entry pass stay in step.
-constexpr int kGenWarps = 4;     // warps (vertices) per 128-thread block
-constexpr int kGenCellRows = 8;  // rows per local cell in the list; more take the scan
-
-__device__ __forceinline__ void generic_vertex_warp(const DevArgs &a, int block) {
-  extern __shared__ double gsh[];  // [kGenWarps][gen_warp_doubles]
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int g = block * kGenWarps + warp;
-  if (g >= a.ngen) return;  // whole warp
-  const int v = a.gen_vertex[g];
-  const int nint = a.v_nint[v];
-  const int r0 = a.v_row_off[v], nrow = a.v_row_off[v + 1] - r0;
-  const int c0 = a.v_col_off[v], ncol = a.v_col_off[v + 1] - c0;
-  if (inst_skipped(a, a.col_ext[c0])) return;  // whole warp
-  const double *T = a.trans + a.v_trans_off[v];
-  double *Jv = a.scratch + a.v_jv_off[v];
-  double *Rv = Jv + nint * nint;
-  double *w = gsh + (size_t)warp * a.gen_warp_doubles;
-  double *Eu = w + TDY_MAX_ROWS, *Ed = Eu + TDY_MAX_ROWS, *fl = Ed + TDY_MAX_ROWS;
-  int *lup = reinterpret_cast<int *>(fl + TDY_MAX_ROWS), *ldn = lup + TDY_MAX_ROWS;
-  unsigned char *cnt = reinterpret_cast<unsigned char *>(ldn + TDY_MAX_ROWS);  // [TDY_MAX_NINT]
-  unsigned char *lst = cnt + TDY_MAX_NINT;                                    // [TDY_MAX_NINT][kGenCellRows]
-
-  for (int r = lane; r < nrow; r += 32) {
-    const double *Tr = T + (size_t)r * ncol;
-    double TP = 0.0;
-    for (int c = 0; c < ncol; c++) TP = __fma_rn(Tr[c], a.P[a.col_ext[c0 + c]], TP);
-    const int f = a.row_face[r0 + r];
-    const int up = a.f_up[f], dn = a.f_dn[f];
-    const double G = a.G[f];
-    const double den = __dadd_rn(a.hr[up], a.hr[dn]);
-    const double q = __fma_rn(den, G, TP);
-    const bool flowdn = q < 0.0;
-    const int u = flowdn ? up : dn;
-    const double lm = a.lam[u];
-    const bool zero = a.seep[u] != 0;
-    const double wr = zero ? 0.0 : __dmul_rn(den, lm);
-    fl[r] = -__dmul_rn(wr, q);
-    w[r] = wr;
-    if (zero) {
-      Eu[r] = 0.0;
-      Ed[r] = 0.0;
-    } else {
-      const double dlu = flowdn ? a.dlam[up] : 0.0, dld = flowdn ? 0.0 : a.dlam[dn];
-      const double g2 = q + den * G;
-      Eu[r] = a.hdr[up] * lm * g2 + den * dlu * q;
-      Ed[r] = a.hdr[dn] * lm * g2 + den * dld * q;
-    }
-    lup[r] = a.row_lup[r0 + r];
-    ldn[r] = a.row_ldn[r0 + r];
-  }
-  __syncwarp();
-  // rows of each local cell, in row order (count 255: more than the list holds)
-  for (int c = lane; c < nint; c += 32) {
-    int k = 0;
-    for (int r = 0; r < nrow; r++)
-      if (lup[r] == c || ldn[r] == c) {
-        if (k < kGenCellRows) lst[c * kGenCellRows + k] = (unsigned char)r;
-        k++;
-      }
-    cnt[c] = (unsigned char)(k <= kGenCellRows ? k : 255);
-  }
-  __syncwarp();
-  // The FP64 pipe is the bound here (a warp-wide FP64 instruction costs as
-  // many issue slots as it has lanes, active or not): walk only each cell's
-  // own rows, and pick signs and upwind terms by integer selects.
-  if (a.needR) {
-    for (int c = lane; c < nint; c += 32) {
-      const int kc = cnt[c];
-      const int kn = kc == 255 ? nrow : kc;
-      double s = 0.0;
-      for (int k = 0; k < kn; k++) {
-        const int r = kc == 255 ? k : lst[c * kGenCellRows + k];
-        if (lup[r] == c) s += fl[r];
-        if (ldn[r] == c) s -= fl[r];
-      }
-      Rv[c] = s;
+#pragma unroll
+      for (int k = 0; k < 3; k++)
+        if (gc.row[k] != 255) s += (gc.flags >> k & 1) ? fl[gc.row[k]] : -fl[gc.row[k]];
+      Jv[nint * nint + c] = s;
     }
   }
   if (!a.needJ) return;
-  const int nn = nint * nint;
-  if (a.jac_ff) {
-    for (int e = lane; e < nn; e += 32) {
-      const int c = e / nint, b = e - c * nint;
-      const int kc = cnt[c];
-      const unsigned char *lc = lst + c * kGenCellRows;
-      Jv[e] = gen_entry_ff(c, b, kc == 255 ? nrow : kc, [&](int k) { return kc == 255 ? k : (int)lc[k]; }, lup, ldn,
-                           w, Eu, Ed, T, ncol);
+  int c = 0, b = lane;
+  for (;; b += L) {
+    while (b >= nint) {
+      b -= nint;
+      c++;
     }
-    return;
-  }
-  for (int e = lane; e < nn; e += 32) {
-    const int c = e / nint, b = e - c * nint;
-    const int kc = cnt[c];
-    const int kn = kc == 255 ? nrow : kc;
-    double J = 0.0;
-    for (int k = 0; k < kn; k++) {
-      const int r = kc == 255 ? k : lst[c * kGenCellRows + k];
-      const int lu = lup[r], ld = ldn[r];
-      if (lu != c && ld != c) continue;  // only in the scan
-      const bool isup = lu == c;
-      const double wr = w[r], eu = Eu[r], ed = Ed[r];
-      J = fma(isup ? -wr : wr, T[(size_t)r * ncol + b], J);
-      // at most one of b == lu, b == ld holds
-      const double et = (b == lu) ? eu : ((b == ld) ? ed : 0.0);
-      J += isup ? -et : et;
+    if (c >= nint) break;
+    const GenCell gc = gen_cell(prog[c]);
+    if (FFJ) {
+      // every product at the entry's own power-of-two scale, as for the
+      // canonical vertices
+      int mb = 0;
+      double t[3], e[3];
+#pragma unroll
+      for (int k = 0; k < 3; k++) {
+        t[k] = e[k] = 0.0;
+        if (gc.row[k] == 255) continue;
+        const int r = gc.row[k];
+        const bool isup = gc.flags >> k & 1;
+        t[k] = T[r * ncol + b];
+        mb = max(mb, bw[r] + d_bexp(t[k]) - 1023);
+        if (b == c || b == gc.other[k]) {
+          e[k] = (b == c) == isup ? Eu[r] : Ed[r];
+          mb = max(mb, d_bexp(e[k]));
+        }
+      }
+      ff acc = {0.0f, 0.0f};
+#pragma unroll
+      for (int k = 0; k < 3; k++) {
+        if (gc.row[k] == 255) continue;
+        const int r = gc.row[k];
+        const bool isup = gc.flags >> k & 1;
+        const float2 f = wf[r];
+        const ff p = ff_mul(ff{f.x, f.y}, ff_split_scaled(t[k], d_bexp(t[k]), bw[r] - mb));
+        ff_acc(acc, isup ? ff_neg(p) : p);
+        if (b == c || b == gc.other[k]) {
+          const ff ef = ff_split_scaled(e[k], d_bexp(e[k]), 1023 - mb);
+          ff_acc(acc, isup ? ff_neg(ef) : ef);
+        }
+      }
+      Jv[c * nint + b] = ff_to_d(acc, mb - 1023);
+    } else {
+      double J = 0.0;
+#pragma unroll
+      for (int k = 0; k < 3; k++) {
+        if (gc.row[k] == 255) continue;
+        const int r = gc.row[k];
+        const bool isup = gc.flags >> k & 1;
+        J = __fma_rn(isup ? -w[r] : w[r], T[r * ncol + b], J);
+        if (b == c || b == gc.other[k]) {
+          const double et = (b == c) == isup ? Eu[r] : Ed[r];
+          J = __dadd_rn(J, isup ? -et : et);
+        }
+      }
+      Jv[c * nint + b] = J;
     }
-    Jv[e] = J;
   }
 }
 
-// Canonical vertices (one thread each, register-heavy) share their launch
-// with the thread form of the other vertices, which take the first blocks so
-// they overlap the canonical ones; meshes without canonical vertices launch
-// the warp form on its own (a light kernel with high occupancy for its
-// latency-bound gathers).
+// The other vertices take the first blocks of the canonical vertices' launch,
+// so they overlap and the chain of their rows is off the launch's tail.
 template <int RHO, bool FFJ>
 __global__ void __launch_bounds__(128) vertex_kernel(DevArgs a, int gen_blocks) {
   if ((int)blockIdx.x >= gen_blocks) {
     const int vc = a.vc0 + ((int)blockIdx.x - gen_blocks) * blockDim.x + threadIdx.x;
     if (vc < a.vc1 && !inst_skipped(a, a.cellc[vc])) canon_vertex_at<RHO, FFJ>(a, vc, threadIdx.x);
   } else {
-    const int g = blockIdx.x * blockDim.x + threadIdx.x;
-    if (g < a.ngen) generic_vertex_one(a, g);
+    generic_vertex_group<FFJ>(a, blockIdx.x);
   }
 }
 
@@ -1181,12 +1129,14 @@ __global__ void __launch_bounds__(kPairThreads, 7) vertex_pair_kernel(DevArgs a,
     const int vc = a.vc0 + ((int)blockIdx.x - gen_blocks) * (kPairThreads / 2) + slot;
     if (vc < a.vc1 && !inst_skipped(a, a.cellc[vc])) canon_vertex_pair<RHO>(a, vc, slot, h, kPairThreads / 2);
   } else {
-    const int g = blockIdx.x * blockDim.x + threadIdx.x;
-    if (g < a.ngen) generic_vertex_one(a, g);
+    generic_vertex_group<true>(a, blockIdx.x);
   }
 }
 
-__global__ void __launch_bounds__(128) generic_vertex_kernel(DevArgs a) { generic_vertex_warp(a, blockIdx.x); }
+template <bool FFJ>
+__global__ void __launch_bounds__(128) generic_vertex_kernel(DevArgs a) {
+  generic_vertex_group<FFJ>(a, blockIdx.x);
+}
 
 // ---------------------------------------------------------------------------
 // 4. per-cell deterministic gather into R and the CSR row.
@@ -1573,6 +1523,79 @@ int device_pool_stream(cudaStream_t *st) { return pool_stream(st); }
 int device_pool_event(cudaEvent_t *ev) { return pool_event(ev); }
 void device_pool_release(int dev, cudaStream_t st, cudaEvent_t ev) { pool_release(dev, st, ev); }
 
+// The other vertices' descriptions (GenVertex, gen_cell) in gen_vertex order,
+// and the lanes and shared memory they take.
+static int pack_generic(const _p_TDy *t, std::vector<GenVertex> &gen, std::vector<int> &g_col,
+                        std::vector<double> &g_rowG, std::vector<uchar2> &g_rowc, std::vector<uint2> &g_cell,
+                        DevArgs *a) {
+  const Mesh &m = t->mesh;
+  const MPFAOSetup &s = t->setup;
+  int max_row = 1, max_col = 1;
+  long long trans = 0;
+  for (int v : s.gen_vertex) {
+    GenVertex d;
+    const int r0 = s.v_row_off[v], nrow = s.v_row_off[v + 1] - r0;
+    const int c0 = s.v_col_off[v], ncol = s.v_col_off[v + 1] - c0, nint = s.v_nint[v];
+    if (ncol > 255) return set_error(TDY_ERR_SUP, "vertex %d has %d columns (max 255)", v, ncol);
+    d.trans = s.v_trans_off[v];
+    d.jv = s.v_jv_off[v];
+    d.row0 = (int)g_rowG.size();
+    d.col0 = (int)g_col.size();
+    d.cell0 = (int)g_cell.size();
+    d.nrow = (unsigned char)nrow;
+    d.ncol = (unsigned char)ncol;
+    d.nint = (unsigned char)nint;
+    d.pad = 0;
+    gen.push_back(d);
+    g_col.insert(g_col.end(), s.col_ext.begin() + c0, s.col_ext.begin() + c0 + ncol);
+    g_cell.insert(g_cell.end(), nint, make_uint2(0x00ffffffu, 0x00ffffffu));
+    uint2 *cells = g_cell.data() + d.cell0;
+    std::vector<int> count(nint, 0);
+    auto add = [&](int c, int r, bool up, int other) {
+      if (c < 0) return true;
+      const int k = count[c]++;
+      if (k >= 3) return false;
+      cells[c].x = (cells[c].x & ~(255u << (8 * k))) | ((unsigned)r << (8 * k)) | (up ? 1u << (24 + k) : 0u);
+      cells[c].y = (cells[c].y & ~(255u << (8 * k))) | ((unsigned)(other < 0 ? 255 : other) << (8 * k));
+      return true;
+    };
+    for (int r = 0; r < nrow; r++) {
+      const int f = s.row_face[r0 + r], lu = s.row_lup[r0 + r], ld = s.row_ldn[r0 + r];
+      // the column of a boundary side: the face's Dirichlet column
+      int bc = -1;
+      if (lu < 0 || ld < 0)
+        for (int c = nint; c < ncol; c++)
+          if (s.col_ext[c0 + c] == m.nc + m.face_bnd[f]) bc = c;
+      if ((lu < 0 || ld < 0) && bc < 0) return set_error(TDY_ERR_LIB, "vertex %d: row without its boundary column", v);
+      g_rowG.push_back(s.gravdis[f]);
+      g_rowc.push_back(make_uchar2((unsigned char)(lu < 0 ? bc : lu), (unsigned char)(ld < 0 ? bc : ld)));
+      if (!add(lu, r, true, ld) || !add(ld, r, false, lu))
+        return set_error(TDY_ERR_SUP, "vertex %d: a cell with more than 3 rows", v);
+    }
+    max_row = std::max(max_row, nrow);
+    max_col = std::max(max_col, ncol);
+    trans += (long long)nrow * ncol;
+  }
+  a->ngen = (int)gen.size();
+  a->gen_max_row = max_row;
+  a->gen_max_col = max_col;
+  // per column 3 doubles (5 where the density varies) and a byte; per row 4
+  // doubles and an int
+  const bool vary = a->rho_type != WATER_DENSITY_CONSTANT;
+  a->gen_doubles = (vary ? 5 : 3) * max_col + 4 * max_row + (4 * max_row + max_col + 7) / 8;
+  // 4 lanes where a vertex's Trans is small (hexahedra's boundary: 4 rows, 4
+  // columns; 532 k of them 0.34 ms, 0.43 with 8 lanes, 0.76 with 32), a warp
+  // where it is large (prisms: 18 x 12; 108 k of them 0.31 ms, 0.36 with 16
+  // lanes, 0.50 with 8): it is read for the rows and again for J_v, and more
+  // vertices in flight push it out of L1.  A launch of their own where they
+  // are the many (48 registers: 0.31 ms against 0.39 ms in the first blocks of
+  // the canonical ones), not where a launch costs more (10 x 10 x 10 cells).
+  a->gen_lanes = trans <= 64LL * a->ngen ? 4 : 32;
+  a->gen_apart = a->ngen > s.nC && a->ngen > 20000;
+  while (a->gen_lanes < 32 && (size_t)(128 / a->gen_lanes) * a->gen_doubles * sizeof(double) > 40 * 1024) a->gen_lanes *= 2;
+  return 0;
+}
+
 int device_setup(_p_TDy *t) {
   const Mesh &m = t->mesh;
   const MPFAOSetup &s = t->setup;
@@ -1623,14 +1646,6 @@ int device_setup(_p_TDy *t) {
   ar.up(&a.bnd_val, t->bnd.value);
   ar.up(&a.bnd_rho, t->bnd.rho);
   ar.up(&a.bnd_vis, t->bnd.vis);
-  std::vector<int> fup(m.nf), fdn(m.nf);
-  for (int f = 0; f < m.nf; f++) {
-    int u = m.face_cell0[f], w = m.face_cell1[f];
-    fup[f] = u >= 0 ? u : m.nc + (-u - 1);
-    fdn[f] = w >= 0 ? w : m.nc + (-w - 1);
-  }
-  ar.up(&a.f_up, fup);
-  ar.up(&a.f_dn, fdn);
   ar.up(&a.G, s.gravdis);
   a.nC = s.nC;
   a.vc0 = 0;
@@ -1643,20 +1658,17 @@ int device_setup(_p_TDy *t) {
   a.jac_ff = t->opt.jacobian_arithmetic == JACOBIAN_DOUBLE_FLOAT;
   ar.up(&a.cellc, s.cellc);
   ar.up(&a.facec, s.facec);
-  a.ngen = (int)s.gen_vertex.size();
-  // per row: w, E_up, E_dn, flux (doubles) and the two local-cell indices
-  // (ints); per local cell: a row count and a list of kGenCellRows rows (bytes)
-  a.gen_warp_doubles = 5 * TDY_MAX_ROWS + (TDY_MAX_NINT * (1 + kGenCellRows) + 7) / 8;
-  ar.up(&a.gen_vertex, s.gen_vertex);
-  ar.up(&a.v_row_off, s.v_row_off);
-  ar.up(&a.v_col_off, s.v_col_off);
-  ar.up(&a.v_nint, s.v_nint);
-  ar.up(&a.v_trans_off, s.v_trans_off);
-  ar.up(&a.v_jv_off, s.v_jv_off);
-  ar.up(&a.row_face, s.row_face);
-  ar.up(&a.row_lup, s.row_lup);
-  ar.up(&a.row_ldn, s.row_ldn);
-  ar.up(&a.col_ext, s.col_ext);
+  std::vector<GenVertex> gen;
+  std::vector<int> g_col;
+  std::vector<double> g_rowG;
+  std::vector<uchar2> g_rowc;
+  std::vector<uint2> g_cell;
+  if ((ierr = pack_generic(t, gen, g_col, g_rowG, g_rowc, g_cell, &a))) return ierr;
+  ar.up(&a.gen, gen);
+  ar.up(&a.g_col, g_col);
+  ar.up(&a.g_rowG, g_rowG);
+  ar.up(&a.g_rowc, g_rowc);
+  ar.up(&a.g_cell, g_cell);
   ar.up(&a.trans, s.trans);
   ar.up(&a.rowptr, s.rowptr);
   ar.up(&a.cv_off, s.cv_off);
@@ -1815,37 +1827,38 @@ static void launch_state_range(const DevArgs &a, int e0, int e1, Emit &e) {
 }
 static void launch_state(const DevArgs &a, Emit &e) { launch_state_range(a, 0, a.nc + a.nb, e); }
 
-// Vertex stage over the vertices a names (gen_vertex/ngen, [vc0, vc1)).
-// gen_warp: mostly other vertices (e.g. prisms, whose valence-4 vertices are
-// canonical): the warp form in its own launch, then the canonical ones; else
-// one launch with the thread form in the first blocks.  The choice is made
-// once per mesh, so a slab launches the same form as the whole evaluation.
+// Vertex stage over the vertices a names (gen/ngen, [vc0, vc1)).
 static int rho_mode(const DevArgs &a) {
   return a.rho_type == WATER_DENSITY_CONSTANT ? RHO_CONST
          : a.rho_type == WATER_DENSITY_EXPONENTIAL ? RHO_EXP
                                                    : RHO_NODERIV;
 }
 
-static void launch_vertices(const DevArgs &a, bool gen_warp, Emit &e) {
-  if (gen_warp && a.ngen > 0)
-    e(generic_vertex_kernel, nblocks(a.ngen, kGenWarps), 128, (size_t)kGenWarps * a.gen_warp_doubles * sizeof(double),
-      a);
-  const int rho = rho_mode(a);
+static void launch_vertices(const DevArgs &a, Emit &e) {
+  const int rho = rho_mode(a), per = 128 / a.gen_lanes;
+  int gb = (int)nblocks(a.ngen, per);
+  size_t gen_smem = gb ? (size_t)per * a.gen_doubles * sizeof(double) : 0;
+  if (a.gen_apart) {
+    e(a.jac_ff ? generic_vertex_kernel<true> : generic_vertex_kernel<false>, gb, 128, gen_smem, a);
+    gb = 0;
+    gen_smem = 0;
+  }
   if (a.jac_ff) {
-    const size_t smem = (size_t)pair_shared_rows(rho) * (kPairThreads / 2) * sizeof(double);
-    const int pb = (int)nblocks(a.vc1 - a.vc0, kPairThreads / 2), gb = gen_warp ? 0 : (int)nblocks(a.ngen, kPairThreads);
+    static_assert(kPairThreads == 128, "blocks of the other vertices");
+    const int pb = (int)nblocks(a.vc1 - a.vc0, kPairThreads / 2);
+    const size_t smem = pb ? (size_t)pair_shared_rows(rho) * (kPairThreads / 2) * sizeof(double) : 0;
     auto k = rho == RHO_CONST ? vertex_pair_kernel<RHO_CONST>
              : rho == RHO_NODERIV ? vertex_pair_kernel<RHO_NODERIV>
                                   : vertex_pair_kernel<RHO_EXP>;
-    e(k, pb + gb, kPairThreads, smem, a, gb);
+    e(k, pb + gb, kPairThreads, std::max(smem, gen_smem), a, gb);
     return;
   }
-  const size_t smem = 36 * 128 * sizeof(double);
-  const int cb = (int)nblocks(a.vc1 - a.vc0, 128), gb = gen_warp ? 0 : (int)nblocks(a.ngen, 128);
+  const int cb = (int)nblocks(a.vc1 - a.vc0, 128);
+  const size_t smem = cb ? 36 * 128 * sizeof(double) : 0;
   auto k = rho == RHO_CONST ? vertex_kernel<RHO_CONST, false>
            : rho == RHO_NODERIV ? vertex_kernel<RHO_NODERIV, false>
                                 : vertex_kernel<RHO_EXP, false>;
-  e(k, cb + gb, 128, smem, a, gb);
+  e(k, cb + gb, 128, std::max(smem, gen_smem), a, gb);
 }
 
 // Cell stage over the cells a names (sc_cells/nS, gc_cells/ngc); gen_warp:
@@ -1864,7 +1877,6 @@ static void launch_cells(const DevArgs &a, bool gen_warp, Emit &e) {
       (size_t)2 * kCellWarps * (size_t)a.max_row_nnz * sizeof(double), a);
 }
 
-static bool vertex_warp_form(const DevArgs &a) { return a.ngen > a.nC; }
 static bool cell_warp_form(const DevArgs &a) { return a.ngc > a.nS; }
 
 // The stages of one evaluation; events[] (4 entries, or null) bracket them
@@ -1874,7 +1886,7 @@ static int launch_eval(const DevArgs &a, cudaStream_t st, cudaEvent_t *events) {
   if (events) CUDA_TRY(cudaEventRecord(events[0], st));
   launch_state(a, e);
   if (events) CUDA_TRY(cudaEventRecord(events[1], st));
-  launch_vertices(a, vertex_warp_form(a), e);
+  launch_vertices(a, e);
   if (events) CUDA_TRY(cudaEventRecord(events[2], st));
   launch_cells(a, cell_warp_form(a), e);
   if (events) CUDA_TRY(cudaEventRecord(events[3], st));
@@ -2075,7 +2087,7 @@ int device_eval_dae_host(_p_TDy *t, double time, const double *U2, const double 
 // The arguments of slab k: the vertices and cells of slab k only.
 static DevArgs slab_args(const DevArgs &a, const DeviceState::Slab &sl) {
   DevArgs b = a;
-  b.gen_vertex = a.gen_vertex + sl.g0;
+  b.gen = a.gen + sl.g0;
   b.ngen = sl.g1 - sl.g0;
   b.vc0 = sl.vc0;
   b.vc1 = sl.vc1;
@@ -2124,7 +2136,7 @@ static int build_slab_graph(_p_TDy *t, DeviceState *d, const DevArgs &a, const d
   e.g = g;
   e.last = join;
   if (err == cudaSuccess) {
-    const bool vw = vertex_warp_form(a), cw = cell_warp_form(a);
+    const bool cw = cell_warp_form(a);
     const size_t K = d->slabs.size();
     launch_state_range(a, a.nc, a.nc + a.nb, e);  // boundary faces
     cudaGraphNode_t sprev = e.last, vprev = nullptr;
@@ -2139,7 +2151,7 @@ static int build_slab_graph(_p_TDy *t, DeviceState *d, const DevArgs &a, const d
       e.last = sjoin;
       launch_state_range(a, sl.e0, sl.e1, e);
       sprev = e.last;
-      launch_vertices(b, vw, e);
+      launch_vertices(b, e);
       vprev = e.last;
       launch_cells(b, cw, e);
       if (e.err != cudaSuccess) break;
@@ -2201,14 +2213,14 @@ int device_eval_host(_p_TDy *t, int form, double time, const double *U, const do
       for (cudaEvent_t &e : d->slab_ev)
         if ((ierr = pool_event(&e))) return ierr;
     }
-    const bool vw = vertex_warp_form(a), cw = cell_warp_form(a);
+    const bool cw = cell_warp_form(a);
     Emit e(d->stream);
     launch_state_range(a, a.nc, a.nc + a.nb, e);  // boundary faces
     for (size_t k = 0; k < d->slabs.size(); k++) {
       const DeviceState::Slab &sl = d->slabs[k];
       const DevArgs b = slab_args(a, sl);
       launch_state_range(a, sl.e0, sl.e1, e);
-      launch_vertices(b, vw, e);
+      launch_vertices(b, e);
       launch_cells(b, cw, e);
       CUDA_TRY(cudaEventRecord(d->slab_ev[k], d->stream));
       CUDA_TRY(cudaStreamWaitEvent(d->copy_stream, d->slab_ev[k], 0));
@@ -2306,8 +2318,8 @@ int device_eval_noalloc(_p_TDy *t, const double *dU, double *dR, double *dJ, voi
 
 int device_launches_per_eval(_p_TDy *t) {
   const DevArgs &a = t->dev->a;
-  const bool vw = a.ngen > a.nC, cw = a.ngc > a.nS;
-  const int nvert = vw ? (a.ngen > 0) + (a.nC > 0) : ((a.nC + a.ngen) > 0 ? 1 : 0);
+  const bool cw = a.ngc > a.nS;
+  const int nvert = a.gen_apart ? 1 + (a.nC > 0) : (a.nC + a.ngen) > 0;
   const int ncell = cw ? (a.ngc > 0) + (a.nS > 0) : ((a.nS + a.ngc) > 0 ? 1 : 0);
   return 1 + nvert + ncell;
 }
