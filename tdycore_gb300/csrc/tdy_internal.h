@@ -155,15 +155,20 @@ struct MPFAOSetup {
   // then generic per-vertex blocks J_v[nint][nint], R_v[nint].
   std::vector<long long> v_jv_off; // nv: generic block offset, or canonical column index
   long long scratch_size = 0;
-  // cell -> (vertex) gather program
-  std::vector<int> cv_off;         // nc+1
-  std::vector<long long> cv_jbase; // offset of J_v[a][0] in scratch
-  std::vector<long long> cv_rbase; // offset of R_v[a]
-  std::vector<int> cv_stride;      // distance between J_v[a][b] and J_v[a][b+1]
-  std::vector<int> cv_nint;        // columns of the vertex
-  std::vector<int> cv_local;       // a: local index of the cell at the vertex
-  std::vector<int> cv_slot_off;    // offset into cv_slots for this (cell, vertex)
-  std::vector<uint8_t> cv_slots;   // CSR slot (within the row) of each vertex column
+  // Gather program of the other cells gc_cells[g]: their vertices' partials
+  // (gv_*, from gv_off[g], in corner order: offsets of J_v[a][0] and R_v[a] in
+  // scratch, a the cell, and position | columns << 16), and per CSR entry (from
+  // ge_off[g], entries with many contributions first) its slot in the row and,
+  // in corner order, its contributions: positions in the cell's rows J_v[a]
+  // set one behind the other, in a byte each (0xff: none), or in 16 bits each
+  // (0xffff) where some cell has more than 255 of them.  One or two 64-bit
+  // words per entry (ge_words).
+  std::vector<int> gv_off, ge_off;          // ngc + 1
+  std::vector<long long> gv_j, gv_r;
+  std::vector<uint32_t> gv_n;
+  std::vector<uint64_t> ge_code;
+  std::vector<uint8_t> ge_slot, gc_diag;    // gc_diag: the row's diagonal slot
+  int ge_words = 1, gc_max_vals = 0;        // gc_max_vals: positions of a cell
   // Structured interior cells: all 8 vertices canonical, 27-entry row in
   // (dz, dy, dx) order, vertices in corner order (see kCornerOffset).  Their
   // gather needs only the 8 canonical vertex indices (SoA, stride nSpad).

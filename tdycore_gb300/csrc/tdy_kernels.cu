@@ -21,11 +21,10 @@
 //        blocks, a few lanes each, in the first blocks of the same launch.
 //   3. cells: sum, in a fixed order, the partials of the cell's vertices into
 //        R[cell] and into the cell's row of the fixed CSR pattern, then add
-//        the accumulation terms (cell_kernel: structured cells, and the
-//        others one thread each when structured cells dominate; else the
-//        others one warp each in generic_cell_kernel).  No atomics, and the
-//        thread and warp forms sum in the same order: results are bitwise
-//        reproducible run to run and independent of the form.
+//        the accumulation terms (cell_kernel: structured cells, one thread
+//        each; generic_cell_kernel: the others, a few lanes each).  No
+//        atomics, and both sum in the same order: results are bitwise
+//        reproducible run to run.
 //
 // Per row the flux is evaluated as -w*(T.P + rho_avg*G) with w = rho_avg*kr/mu
 // and the Jacobian entry as -(w*T + E) with E the derivative terms of the
@@ -52,8 +51,7 @@ namespace tdy {
 
 #define TDY_MAX_ROWS 64
 #define TDY_MAX_NINT 64
-// Jacobian row length: the gather program stores slots in 8 bits (the
-// generic cell kernel stages one row per warp in shared memory)
+// Jacobian row length: the gather program stores slots in 8 bits
 #define TDY_MAX_ROW_NNZ 255
 
 // An other (not canonical) vertex: its rows, columns and internal cells in the
@@ -62,6 +60,13 @@ struct __align__(16) GenVertex {
   long long trans, jv;
   int row0, col0, cell0;
   unsigned char nrow, ncol, nint, pad;
+};
+
+// An other (not structured) cell: where its vertices and entries start in gv_*
+// and ge_*, their numbers, the diagonal's slot.
+struct __align__(16) GenCellHead {
+  int cell, k0, e0;
+  unsigned char n, rn, diag, pad;
 };
 
 struct DevArgs {
@@ -105,15 +110,19 @@ struct DevArgs {
   const double *trans;
   double *scratch;
   // cell gather
-  const int *rowptr, *cv_off, *cv_stride, *cv_nint, *cv_local, *cv_slot_off;
-  const long long *cv_jbase, *cv_rbase;
-  const unsigned char *cv_slots;
+  const int *rowptr;
+  const GenCellHead *gc;
+  const long long *gv_j, *gv_r;
+  const unsigned long long *ge_code;
+  const unsigned *gv_n;
+  const unsigned char *ge_slot;
+  int ge_words, gc_max_vals;
   int max_row_nnz;
   // instances: of each cell, and (a call on some instances only, else null)
   // which are evaluated; the others' entities are skipped
   const int *cell_inst, *inst_on;
   int nS, nSpad, ngc;
-  const int *sc_cells, *sc_vc, *gc_cells;
+  const int *sc_cells, *sc_vc;
   // outputs
   double *R, *J;
 };
@@ -588,6 +597,14 @@ __host__ __device__ constexpr int d_struct_octant(int j) { return 7 ^ corner_off
 __host__ __device__ constexpr int d_struct_slot(int j, int b) {
   return ((((corner_offset(j) >> 2) & 1) - 1 + ((b >> 2) & 1)) + 1) * 9 +
          ((((corner_offset(j) >> 1) & 1) - 1 + ((b >> 1) & 1)) + 1) * 3 + (((corner_offset(j) & 1) - 1 + (b & 1)) + 1);
+}
+// whether corner j is the first of a structured cell's corners whose vertex
+// touches octant b's slot
+__host__ __device__ constexpr bool first_touch(int j, int b) {
+  for (int i = 0; i < j; i++)
+    for (int o = 0; o < 8; o++)
+      if (d_struct_slot(i, o) == d_struct_slot(j, b)) return false;
+  return true;
 }
 static_assert(corner_offset(2) == kCornerOffset[2] && corner_offset(7) == kCornerOffset[7] &&
                   d_struct_slot(0, 7) == struct_slot(0, 7) && d_struct_slot(6, 0) == struct_slot(6, 0) &&
@@ -1142,10 +1159,9 @@ __global__ void __launch_bounds__(128) generic_vertex_kernel(DevArgs a) {
 // 4. per-cell deterministic gather into R and the CSR row.
 //
 // Structured interior cells (all vertices canonical, 27-point row) read their
-// eight vertices' partials at compile-time slots.  Other cells follow their
-// gather program; each warp stages its rows in shared memory and writes them
-// with coalesced stores.  Both sum the vertices in the cell's corner order, so
-// a cell gets the same bits on either path.
+// eight vertices' partials at compile-time slots, one thread each; the others
+// follow their gather program.  Both sum the vertices in the cell's corner
+// order.
 
 // structured cell sc_cells[sidx]; the 32 lanes of a warp call it together
 // with consecutive sidx (those at or past s_end do nothing)
@@ -1165,28 +1181,24 @@ __device__ __forceinline__ void struct_cell_at(const DevArgs &a, int sidx, int s
 #pragma unroll
     for (int j = 0; j < 8; j++) vc[j] = a.sc_vc[j * Q + sidx];
     if (a.needR) {
-      double s = 0.0;
+      double s = S[64 * P + d_struct_octant(0) * P + vc[0]];
 #pragma unroll
-      for (int j = 0; j < 8; j++) s += S[64 * P + d_struct_octant(j) * P + vc[j]];
+      for (int j = 1; j < 8; j++) s += S[64 * P + d_struct_octant(j) * P + vc[j]];
       s += a.acc_a[i];
       s -= a.acc_b[i];
       a.R[i] = s;
     }
     if (a.needJ) {
 #pragma unroll
-      for (int k = 0; k < 27; k++) row[k] = 0.0;
-#pragma unroll
       for (int j = 0; j < 8; j++) {
-        const double2 *blk = reinterpret_cast<const double2 *>(S + ((long long)d_struct_octant(j) * P + vc[j]) * 8);
-        const double2 v0 = blk[0], v1 = blk[1], v2 = blk[2], v3 = blk[3];
-        row[d_struct_slot(j, 0)] += v0.x;
-        row[d_struct_slot(j, 1)] += v0.y;
-        row[d_struct_slot(j, 2)] += v1.x;
-        row[d_struct_slot(j, 3)] += v1.y;
-        row[d_struct_slot(j, 4)] += v2.x;
-        row[d_struct_slot(j, 5)] += v2.y;
-        row[d_struct_slot(j, 6)] += v3.x;
-        row[d_struct_slot(j, 7)] += v3.y;
+        // 32-byte loads: with 16-byte ones half of a sector waits in L1 for the
+        // next request, and more resident warps made the kernel slower
+        const double *blk = S + ((long long)d_struct_octant(j) * P + vc[j]) * 8;
+        double v[8];
+        asm volatile("ld.global.v4.f64 {%0, %1, %2, %3}, [%4];" : "=d"(v[0]), "=d"(v[1]), "=d"(v[2]), "=d"(v[3]) : "l"(blk));
+        asm volatile("ld.global.v4.f64 {%0, %1, %2, %3}, [%4];" : "=d"(v[4]), "=d"(v[5]), "=d"(v[6]), "=d"(v[7]) : "l"(blk + 4));
+#pragma unroll
+        for (int b = 0; b < 8; b++) row[d_struct_slot(j, b)] = first_touch(j, b) ? v[b] : row[d_struct_slot(j, b)] + v[b];
       }
       row[13] += a.jdiag[i];
     }
@@ -1198,12 +1210,22 @@ __device__ __forceinline__ void struct_cell_at(const DevArgs &a, int sidx, int s
   const int rp0 = __shfl_sync(0xffffffffu, rp, 0);
   const bool contig = __all_sync(0xffffffffu, active && rp == rp0 + 27 * lane);
   if (contig) {
-    double *buf = rowbuf + (size_t)warp * 32 * 27;
+    // nine slots at a time: shared memory for whole rows (13.8 KB a block)
+    // would leave L1 little
+    double *buf = rowbuf + warp * 32 * 9;
 #pragma unroll
-    for (int k = 0; k < 27; k++) buf[lane * 27 + k] = row[k];
-    __syncwarp();
-    double *out = a.J + rp0;
-    for (int j = lane; j < 32 * 27; j += 32) out[j] = buf[j];
+    for (int c = 0; c < 3; c++) {
+#pragma unroll
+      for (int k = 0; k < 9; k++) buf[lane * 9 + k] = row[9 * c + k];
+      __syncwarp();
+      double *out = a.J + rp0 + 9 * c;
+#pragma unroll
+      for (int t = 0; t < 9; t++) {
+        const int e = lane + 32 * t;
+        out[27 * (e / 9) + e % 9] = buf[e];
+      }
+      __syncwarp();
+    }
   } else if (active) {
     double *out = a.J + rp;
 #pragma unroll
@@ -1211,101 +1233,124 @@ __device__ __forceinline__ void struct_cell_at(const DevArgs &a, int sidx, int s
   }
 }
 
-// Other cells, thread form (meshes with structured cells).
-// other cell gc_cells[gidx], one thread
-__device__ __forceinline__ void generic_cell_at(const DevArgs &a, int gidx, int g_end) {
-  extern __shared__ double rowbuf[];  // [warps][32 * max_row_nnz]
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  const int g0 = gidx - lane;
-  if (g0 >= g_end) return;  // whole warp out of range
-  bool active = gidx < g_end;
-  const int i = active ? a.gc_cells[gidx] : -1;
-  active = active && !inst_skipped(a, i);
-  if (a.needR && active) {
-    const int k0 = a.cv_off[i], k1 = a.cv_off[i + 1];
-    double s = 0.0;
-    for (int k = k0; k < k1; k++) s += a.scratch[a.cv_rbase[k]];
-    s += a.acc_a[i];
-    s -= a.acc_b[i];
-    a.R[i] = s;
-  }
-  if (!a.needJ) return;
-  double *row = rowbuf + ((size_t)warp * 32 + lane) * a.max_row_nnz;
-  int p0 = 0, rn = 0;
-  if (active) {
-    p0 = a.rowptr[i];
-    rn = a.rowptr[i + 1] - p0;
-    for (int j = 0; j < rn; j++) row[j] = 0.0;
-    const int k0 = a.cv_off[i], k1 = a.cv_off[i + 1];
-    int diag = -1;
-    for (int k = k0; k < k1; k++) {
-      const int nint = a.cv_nint[k], stride = a.cv_stride[k];
-      const long long jb = a.cv_jbase[k];
-      const unsigned char *sl = a.cv_slots + a.cv_slot_off[k];
-      for (int b = 0; b < nint; b++) row[sl[b]] += a.scratch[jb + (long long)b * stride];
-      diag = sl[a.cv_local[k]];
+// Other cells: kCellLanes lanes each.  The cell's rows J_v[a] of its vertices
+// are copied into shared memory (whole sectors, all in flight together, while
+// the entries' words load), then every CSR entry is summed by one lane: its
+// contributions come packed in a word or two (MPFAOSetup::ge_code), in the
+// cell's corner order, and the entries are sorted by the number of
+// contributions, so a pass of the lanes makes few additions (a warp's FP64
+// addition costs 57 cycles whatever its active lanes).  The row is stored in
+// order.  The residuals, ten additions in a chain, take one lane per cell in
+// the block's first warp.  204 k prisms: 0.098 ms (0.174 ms adding vertex
+// blocks to the row one by one, a half-warp per cell); 387 k boundary cells of
+// 512 columns: 0.13 ms (0.416 ms).
+constexpr int kCellLanes = 8;
+constexpr int kCellThreads = 128;
+constexpr int kCellWords = 8;  // words held per lane: rows of up to 64 entries
+
+__global__ void __launch_bounds__(kCellThreads) generic_cell_kernel(DevArgs a) {
+  extern __shared__ double rowbuf[];  // per cell: the row, then the vertices' rows
+  constexpr int NC = kCellThreads / kCellLanes, L = kCellLanes;
+  const int tid = threadIdx.x, grp = tid / L, lane = tid % L, block = blockIdx.x;
+  const double *S = a.scratch;
+  const int per = a.needJ ? NC : kCellThreads;  // cells of the block
+  if (a.needR && tid < per && block * per + tid < a.ngc) {
+    const GenCellHead h = a.gc[block * per + tid];
+    if (!inst_skipped(a, h.cell)) {
+      double v[8];
+#pragma unroll
+      for (int k = 0; k < 8; k++) v[k] = k < h.n ? S[a.gv_r[h.k0 + k]] : 0.0;
+      double s = v[0];
+#pragma unroll
+      for (int k = 1; k < 8; k++)
+        if (k < h.n) s += v[k];
+      s += a.acc_a[h.cell];
+      s -= a.acc_b[h.cell];
+      a.R[h.cell] = s;
     }
-    if (diag >= 0) row[diag] += a.jdiag[i];
-    double *out = a.J + p0;
-    for (int j = 0; j < rn; j++) out[j] = row[j];
-  }
-}
-
-// Other cells, warp form (meshes without structured cells): one half-warp
-// per cell (vertex blocks of such meshes have about 12 columns, so 16 lanes
-// keep the FP64 adds, this kernel's bound, mostly full).  The row is staged
-// in shared memory; the lanes take the columns of each vertex block (distinct
-// columns land in distinct slots) and the vertices are added in the cell's
-// corner order, as in the thread form.
-constexpr int kCellWarps = 4;  // warps per generic-cell block (two cells each)
-
-__device__ __forceinline__ void generic_cell_warp(const DevArgs &a, int block) {
-  extern __shared__ double rowbuf[];  // [2 * kCellWarps][max_row_nnz]
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int half = lane >> 4, hl = lane & 15;
-  const int pair = block * kCellWarps + warp;
-  if (2 * pair >= a.ngc) return;  // whole warp
-  const int gidx = 2 * pair + half;
-  if (gidx >= a.ngc) return;  // the second half of the last warp
-  const unsigned mask = 0xffffu << (16 * half);
-  const int i = a.gc_cells[gidx];
-  if (inst_skipped(a, i)) return;  // whole half-warp
-  const int k0 = a.cv_off[i], k1 = a.cv_off[i + 1];
-  if (a.needR && hl == 0) {
-    double s = 0.0;
-    for (int k = k0; k < k1; k++) s += a.scratch[a.cv_rbase[k]];
-    s += a.acc_a[i];
-    s -= a.acc_b[i];
-    a.R[i] = s;
   }
   if (!a.needJ) return;
-  double *row = rowbuf + (size_t)(2 * warp + half) * a.max_row_nnz;
-  const int p0 = a.rowptr[i], rn = a.rowptr[i + 1] - p0;
-  for (int j = hl; j < rn; j += 16) row[j] = 0.0;
-  __syncwarp(mask);
-  int diag = -1;
-  for (int k = k0; k < k1; k++) {
-    const int nint = a.cv_nint[k], stride = a.cv_stride[k];
-    const long long jb = a.cv_jbase[k];
-    const unsigned char *sl = a.cv_slots + a.cv_slot_off[k];
-    for (int b = hl; b < nint; b += 16) row[sl[b]] += a.scratch[jb + (long long)b * stride];
-    diag = sl[a.cv_local[k]];
-    __syncwarp(mask);
+  const int g = block * NC + grp;
+  GenCellHead h = {0, 0, 0, 0, 0, 0, 0};
+  if (g < a.ngc) h = a.gc[g];
+  if (g >= a.ngc || inst_skipped(a, h.cell)) h.n = h.rn = 0;  // (the warp stays together)
+  long long src = 0;
+  unsigned pos = 0;
+  if (lane < h.n) {
+    src = a.gv_j[h.k0 + lane];
+    pos = a.gv_n[h.k0 + lane];
   }
-  if (hl == 0 && diag >= 0) row[diag] += a.jdiag[i];
-  __syncwarp(mask);
+  const bool bytes = a.ge_words == 1;
+  unsigned long long w[kCellWords];
+  unsigned char slot[kCellWords];
+  if (bytes) {
+#pragma unroll
+    for (int t = 0; t < kCellWords; t++)
+      if (lane + L * t < h.rn) {
+        w[t] = a.ge_code[h.e0 + lane + L * t];
+        slot[t] = a.ge_slot[h.e0 + lane + L * t];
+      }
+  }
+  const double jd = h.rn ? a.jdiag[h.cell] : 0.0;
+  const int p0 = h.rn ? a.rowptr[h.cell] : 0;
+  double *row = rowbuf + (size_t)grp * (a.max_row_nnz + a.gc_max_vals), *val = row + a.max_row_nnz;
+#pragma unroll
+  for (int k = 0; k < 8; k++) {
+    const double *from = S + __shfl_sync(0xffffffffu, src, k, L);
+    const unsigned pk = __shfl_sync(0xffffffffu, pos, k, L);
+    const unsigned to = (unsigned)__cvta_generic_to_shared(val + (pk & 0xffffu));
+    for (int b = lane; b < (int)(pk >> 16); b += L)  // (no columns beyond the last vertex)
+      asm volatile("cp.async.ca.shared.global [%0], [%1], 8;" ::"r"(to + 8 * b), "l"(from + b));
+  }
+  asm volatile("cp.async.wait_all;" ::: "memory");
+  __syncwarp();
+  // (the whole warp together; `on`: the lane has an entry.  An addition whose
+  // predicate is off in every lane would still take its 57 cycles: branch)
+  auto entry = [&](bool on, unsigned long long w0, unsigned long long w1, int sl) {
+    double v[8];
+    int cnt = 0;
+#pragma unroll
+    for (int k = 0; k < 8; k++) {
+      const unsigned c = bytes ? (unsigned)(w0 >> (8 * k)) & 0xffu : (unsigned)((k < 4 ? w0 : w1) >> (16 * (k % 4))) & 0xffffu;
+      v[k] = 0.0;
+      if (on && c != (bytes ? 0xffu : 0xffffu)) {
+        v[k] = val[c];
+        cnt = k + 1;
+      }
+    }
+    double s = v[0];
+#pragma unroll
+    for (int k = 1; k < 8; k++) {
+      if (!__any_sync(0xffffffffu, k < cnt)) break;
+      s = k < cnt ? __dadd_rn(s, v[k]) : s;
+    }
+    if (__any_sync(0xffffffffu, on && sl == h.diag)) s = sl == h.diag ? __dadd_rn(s, jd) : s;
+    if (on) row[sl] = s;
+  };
+  const int most = __reduce_max_sync(0xffffffffu, (int)h.rn);
+  if (bytes) {
+#pragma unroll
+    for (int t = 0; t < kCellWords; t++)
+      if (L * t < most) entry(lane + L * t < h.rn, w[t], 0, slot[t]);
+  }
+  for (int e0 = bytes ? L * kCellWords : 0; e0 < most; e0 += L) {
+    const int e = e0 + lane;
+    const bool on = e < h.rn;
+    const size_t q = (size_t)a.ge_words * (h.e0 + e);
+    entry(on, on ? a.ge_code[q] : 0, on && !bytes ? a.ge_code[q + 1] : 0, on ? a.ge_slot[h.e0 + e] : 0);
+  }
+  __syncwarp();
   double *out = a.J + p0;
-  for (int j = hl; j < rn; j += 16) out[j] = row[j];
+  for (int e = lane; e < h.rn; e += L) out[e] = row[e];
 }
 
-__global__ void __launch_bounds__(64) cell_kernel(DevArgs a, int struct_blocks) {
-  if ((int)blockIdx.x < struct_blocks)
-    struct_cell_at(a, blockIdx.x * blockDim.x + threadIdx.x, a.nS);
-  else
-    generic_cell_at(a, ((int)blockIdx.x - struct_blocks) * blockDim.x + threadIdx.x, a.ngc);
+// At 60 x 220 x 85, this launch and the other cells': 0.208 ms, 4.3 TB/s of
+// partials, rows and lists; 0.234 ms with 16-byte loads and whole rows in
+// shared memory, 0.22 ms with 80 registers and 24 warps, 0.31 ms with the
+// other cells in the same launch (69 registers).
+__global__ void __launch_bounds__(64, 8) cell_kernel(DevArgs a) {
+  struct_cell_at(a, blockIdx.x * blockDim.x + threadIdx.x, a.nS);
 }
-
-__global__ void __launch_bounds__(32 * kCellWarps) generic_cell_kernel(DevArgs a) { generic_cell_warp(a, blockIdx.x); }
 
 // ---------------------------------------------------------------------------
 // Host side
@@ -1454,18 +1499,17 @@ static void build_slabs(_p_TDy *t, DeviceState *d) {
 }
 
 static int noalloc_resolve(int dev);
-static size_t cell_smem_bytes(const DevArgs &a, bool gen_warp);
-static bool cell_warp_form(const DevArgs &a);
 
 // Dynamic shared memory above 48 KB is an opt-in per kernel and device; it
 // is made at set-up with the device current (and only ever raised).
 static size_t g_cell_smem_granted[kMaxDevices] = {};
+static size_t gen_cell_smem(const DevArgs &a);
 static int cell_smem_optin(int dev, size_t bytes) {
   if (bytes <= 48 * 1024) return 0;
   if (dev < 0 || dev >= kMaxDevices) return set_error(TDY_ERR_SUP, "device ordinal %d not supported", dev);
   std::lock_guard<std::mutex> lk(g_dev_mutex);
   if (bytes > g_cell_smem_granted[dev]) {
-    CUDA_TRY(cudaFuncSetAttribute(cell_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes));
+    CUDA_TRY(cudaFuncSetAttribute(generic_cell_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes));
     g_cell_smem_granted[dev] = bytes;
   }
   return 0;
@@ -1671,21 +1715,26 @@ int device_setup(_p_TDy *t) {
   ar.up(&a.g_cell, g_cell);
   ar.up(&a.trans, s.trans);
   ar.up(&a.rowptr, s.rowptr);
-  ar.up(&a.cv_off, s.cv_off);
-  ar.up(&a.cv_jbase, s.cv_jbase);
-  ar.up(&a.cv_rbase, s.cv_rbase);
-  ar.up(&a.cv_stride, s.cv_stride);
-  ar.up(&a.cv_nint, s.cv_nint);
-  ar.up(&a.cv_local, s.cv_local);
-  ar.up(&a.cv_slot_off, s.cv_slot_off);
-  ar.up(&a.cv_slots, s.cv_slots);
+  std::vector<GenCellHead> gc(s.gc_cells.size());
+  for (size_t g = 0; g < gc.size(); g++) {
+    const int c = s.gc_cells[g];
+    gc[g] = GenCellHead{c, s.gv_off[g], s.ge_off[g], (unsigned char)(s.gv_off[g + 1] - s.gv_off[g]),
+                        (unsigned char)(s.rowptr[c + 1] - s.rowptr[c]), s.gc_diag[g], 0};
+  }
+  ar.up(&a.gc, gc);
+  ar.up(&a.gv_j, s.gv_j);
+  ar.up(&a.gv_r, s.gv_r);
+  ar.up(&a.gv_n, s.gv_n);
+  ar.up(&a.ge_code, s.ge_code);
+  ar.up(&a.ge_slot, s.ge_slot);
+  a.ge_words = s.ge_words;
+  a.gc_max_vals = s.gc_max_vals;
   a.max_row_nnz = s.max_row_nnz;
   a.nS = s.nS;
   a.nSpad = s.nSpad;
   a.ngc = (int)s.gc_cells.size();
   ar.up(&a.sc_cells, s.sc_cells);
   ar.up(&a.sc_vc, s.sc_vc);
-  ar.up(&a.gc_cells, s.gc_cells);
   ar.work(&a.P, next);
   ar.work(&a.hr, next);
   ar.work(&a.hdr, next);
@@ -1728,7 +1777,7 @@ int device_setup(_p_TDy *t) {
     return ierr;
   if (t->opt.setup_on_device && (ierr = device_gen_trans(t, const_cast<double *>(a.trans), d->stream))) return ierr;
   build_slabs(t, d);  // their copy stream and events are taken on first use
-  if ((ierr = cell_smem_optin(d->device, cell_smem_bytes(a, cell_warp_form(a))))) return ierr;
+  if ((ierr = cell_smem_optin(d->device, gen_cell_smem(a)))) return ierr;
   if ((ierr = noalloc_resolve(d->device))) return ierr;
   if ((ierr = pool_event(&d->noalloc_ev))) return ierr;
   // the uploads (and the device-built Trans) are complete before any other
@@ -1861,23 +1910,16 @@ static void launch_vertices(const DevArgs &a, Emit &e) {
   e(k, cb + gb, 128, std::max(smem, gen_smem), a, gb);
 }
 
-// Cell stage over the cells a names (sc_cells/nS, gc_cells/ngc); gen_warp:
-// mostly other cells take the warp form.
-static size_t cell_smem_bytes(const DevArgs &a, bool gen_warp) {
-  return 64 * (size_t)(gen_warp || a.max_row_nnz < 27 ? 27 : a.max_row_nnz) * sizeof(double);
+// Cell stage over the cells a names (sc_cells/nS, gc/ngc).
+static size_t gen_cell_smem(const DevArgs &a) {
+  return (size_t)(kCellThreads / kCellLanes) * (a.max_row_nnz + a.gc_max_vals) * sizeof(double);
 }
 
-// (rows longer than 96 entries need more than 48 KB of dynamic shared
-// memory: device_setup opts in for the handle's device)
-static void launch_cells(const DevArgs &a, bool gen_warp, Emit &e) {
-  const int sb = (int)nblocks(a.nS, 64), gcb = gen_warp ? 0 : (int)nblocks(a.ngc, 64);
-  e(cell_kernel, sb + gcb, 64, cell_smem_bytes(a, gen_warp), a, sb);
-  if (gen_warp && a.ngc > 0)
-    e(generic_cell_kernel, nblocks(a.ngc, 2 * kCellWarps), 32 * kCellWarps,
-      (size_t)2 * kCellWarps * (size_t)a.max_row_nnz * sizeof(double), a);
+static void launch_cells(const DevArgs &a, Emit &e) {
+  e(cell_kernel, nblocks(a.nS, 64), 64, 64 * 9 * sizeof(double), a);
+  e(generic_cell_kernel, nblocks(a.ngc, a.needJ ? kCellThreads / kCellLanes : kCellThreads), kCellThreads,
+    a.needJ ? gen_cell_smem(a) : 0, a);
 }
-
-static bool cell_warp_form(const DevArgs &a) { return a.ngc > a.nS; }
 
 // The stages of one evaluation; events[] (4 entries, or null) bracket them
 // for the per-kernel timers.
@@ -1888,7 +1930,7 @@ static int launch_eval(const DevArgs &a, cudaStream_t st, cudaEvent_t *events) {
   if (events) CUDA_TRY(cudaEventRecord(events[1], st));
   launch_vertices(a, e);
   if (events) CUDA_TRY(cudaEventRecord(events[2], st));
-  launch_cells(a, cell_warp_form(a), e);
+  launch_cells(a, e);
   if (events) CUDA_TRY(cudaEventRecord(events[3], st));
   CUDA_TRY(cudaGetLastError());
   return 0;
@@ -2094,7 +2136,7 @@ static DevArgs slab_args(const DevArgs &a, const DeviceState::Slab &sl) {
   b.sc_cells = a.sc_cells + sl.s0;
   b.sc_vc = a.sc_vc + sl.s0;  // structure of arrays, stride nSpad: the offset carries over
   b.nS = sl.s1 - sl.s0;
-  b.gc_cells = a.gc_cells + sl.gc0;
+  b.gc = a.gc + sl.gc0;
   b.ngc = sl.gc1 - sl.gc0;
   return b;
 }
@@ -2136,7 +2178,6 @@ static int build_slab_graph(_p_TDy *t, DeviceState *d, const DevArgs &a, const d
   e.g = g;
   e.last = join;
   if (err == cudaSuccess) {
-    const bool cw = cell_warp_form(a);
     const size_t K = d->slabs.size();
     launch_state_range(a, a.nc, a.nc + a.nb, e);  // boundary faces
     cudaGraphNode_t sprev = e.last, vprev = nullptr;
@@ -2153,7 +2194,7 @@ static int build_slab_graph(_p_TDy *t, DeviceState *d, const DevArgs &a, const d
       sprev = e.last;
       launch_vertices(b, e);
       vprev = e.last;
-      launch_cells(b, cw, e);
+      launch_cells(b, e);
       if (e.err != cudaSuccess) break;
       cudaGraphNode_t deps[2] = {e.last, copy_last}, nj = nullptr;
       err = cudaGraphAddMemcpyNode1D(&nj, g, deps, copy_last ? 2 : 1, J + sl.j0, d->dJ + sl.j0,
@@ -2213,7 +2254,6 @@ int device_eval_host(_p_TDy *t, int form, double time, const double *U, const do
       for (cudaEvent_t &e : d->slab_ev)
         if ((ierr = pool_event(&e))) return ierr;
     }
-    const bool cw = cell_warp_form(a);
     Emit e(d->stream);
     launch_state_range(a, a.nc, a.nc + a.nb, e);  // boundary faces
     for (size_t k = 0; k < d->slabs.size(); k++) {
@@ -2221,7 +2261,7 @@ int device_eval_host(_p_TDy *t, int form, double time, const double *U, const do
       const DevArgs b = slab_args(a, sl);
       launch_state_range(a, sl.e0, sl.e1, e);
       launch_vertices(b, e);
-      launch_cells(b, cw, e);
+      launch_cells(b, e);
       CUDA_TRY(cudaEventRecord(d->slab_ev[k], d->stream));
       CUDA_TRY(cudaStreamWaitEvent(d->copy_stream, d->slab_ev[k], 0));
       CUDA_TRY(cudaMemcpyAsync(J + sl.j0, d->dJ + sl.j0, sizeof(double) * (size_t)(sl.j1 - sl.j0),
@@ -2318,9 +2358,8 @@ int device_eval_noalloc(_p_TDy *t, const double *dU, double *dR, double *dJ, voi
 
 int device_launches_per_eval(_p_TDy *t) {
   const DevArgs &a = t->dev->a;
-  const bool cw = a.ngc > a.nS;
   const int nvert = a.gen_apart ? 1 + (a.nC > 0) : (a.nC + a.ngen) > 0;
-  const int ncell = cw ? (a.ngc > 0) + (a.nS > 0) : ((a.nS + a.ngc) > 0 ? 1 : 0);
+  const int ncell = (a.ngc > 0) + (a.nS > 0);
   return 1 + nvert + ncell;
 }
 

@@ -572,66 +572,86 @@ int mpfao_setup(const Options &opt, const Mesh &m, const Materials &mat, const B
   }
   s.scratch_size = off;
 
-  // ---- cell gather program ----
-  s.cv_off.assign(nc + 1, 0);
+  // ---- structured interior cells, and the gather program of the others ----
+  std::vector<std::array<int, 8>> svc;
+  for (int c = 0; c < nc; c++) {
+    int vals = 0;
+    for (int j = m.cell_vert_off[c]; j < m.cell_vert_off[c + 1]; j++) vals += s.v_nint[m.cell_verts[j]];
+    s.gc_max_vals = std::max(s.gc_max_vals, vals);
+  }
+  s.ge_words = s.gc_max_vals > 255 ? 2 : 1;
+  s.gv_off.assign(1, 0);
+  s.ge_off.assign(1, 0);
+  std::vector<int> count, order;
+  std::vector<std::array<uint16_t, 8>> from;  // per slot: positions
   for (int c = 0; c < nc; c++) {
     const int *row = &s.colidx[s.rowptr[c]];
     const int rn = s.rowptr[c + 1] - s.rowptr[c];
-    for (int j = m.cell_vert_off[c]; j < m.cell_vert_off[c + 1]; j++) {
-      int v = m.cell_verts[j];
-      const int c0 = s.v_col_off[v], nint = s.v_nint[v];
-      std::vector<int> cols(nint);
-      if (canon_idx[v] >= 0) {
-        for (int o = 0; o < 8; o++) cols[o] = s.col_ext[c0 + octant_col[canon_idx[v]][o]];
-      } else {
-        for (int k = 0; k < nint; k++) cols[k] = s.col_ext[c0 + k];
-      }
-      int a = -1;
-      for (int k = 0; k < nint; k++)
-        if (cols[k] == c) a = k;
-      if (a < 0) return set_error(TDY_ERR_LIB, "cell %d missing at its vertex %d", c, v);
-      if (canon_idx[v] >= 0) {
-        s.cv_jbase.push_back(((long long)a * P + canon_idx[v]) * 8);
-        s.cv_rbase.push_back(64 * P + (long long)a * P + canon_idx[v]);
-        s.cv_stride.push_back(1);
-      } else {
-        s.cv_jbase.push_back(s.v_jv_off[v] + (long long)a * nint);
-        s.cv_rbase.push_back(s.v_jv_off[v] + (long long)nint * nint + a);
-        s.cv_stride.push_back(1);
-      }
-      s.cv_nint.push_back(nint);
-      s.cv_local.push_back(a);
-      s.cv_slot_off.push_back((int)s.cv_slots.size());
-      for (int k = 0; k < nint; k++) {
-        int pos = (int)(std::lower_bound(row, row + rn, cols[k]) - row);
-        s.cv_slots.push_back((uint8_t)pos);
-      }
-    }
-    s.cv_off[c + 1] = (int)s.cv_jbase.size();
-  }
-
-  // ---- structured interior cells ----
-  std::vector<std::array<int, 8>> svc;
-  for (int c = 0; c < nc; c++) {
-    bool ok = (s.rowptr[c + 1] - s.rowptr[c] == 27) && (s.cv_off[c + 1] - s.cv_off[c] == 8);
+    const int *cv = &m.cell_verts[m.cell_vert_off[c]];
+    const int ncv = m.cell_vert_off[c + 1] - m.cell_vert_off[c];
+    if (ncv > 8) return set_error(TDY_ERR_SUP, "cell %d has %d vertices (max 8)", c, ncv);
+    // columns of corner j's vertex: in octant order where it is canonical
+    auto column = [&](int j, int k) {
+      const int v = cv[j];
+      return s.col_ext[s.v_col_off[v] + (canon_idx[v] >= 0 ? octant_col[canon_idx[v]][k] : k)];
+    };
+    bool ok = rn == 27 && ncv == 8;
     std::array<int, 8> vcs;
     for (int j = 0; ok && j < 8; j++) {
-      const int k = s.cv_off[c] + j;
-      const int v = m.cell_verts[m.cell_vert_off[c] + j];
-      if (canon_idx[v] < 0 || s.cv_local[k] != struct_octant(j)) {
-        ok = false;
-        break;
-      }
-      for (int b = 0; b < 8; b++)
-        if (s.cv_slots[s.cv_slot_off[k] + b] != struct_slot(j, b)) ok = false;
+      const int v = cv[j];
+      ok = canon_idx[v] >= 0 && column(j, struct_octant(j)) == c;
+      for (int b = 0; ok && b < 8; b++) ok = row[struct_slot(j, b)] == column(j, b);
       vcs[j] = canon_idx[v];
     }
     if (ok) {
       s.sc_cells.push_back(c);
       svc.push_back(vcs);
-    } else {
-      s.gc_cells.push_back(c);
+      continue;
     }
+    s.gc_cells.push_back(c);
+    count.assign(rn, 0);
+    from.resize(std::max<size_t>(from.size(), rn));
+    int pos = 0;
+    for (int j = 0; j < ncv; j++) {
+      const int v = cv[j], nint = s.v_nint[v];
+      int a = -1;
+      for (int k = 0; k < nint; k++) {
+        const int col = column(j, k);
+        if (col == c) a = k;
+        const int slot = (int)(std::lower_bound(row, row + rn, col) - row);
+        from[slot][count[slot]++] = (uint16_t)(pos + k);
+      }
+      s.gv_n.push_back((uint32_t)pos | (uint32_t)nint << 16);
+      pos += nint;
+      if (a < 0) return set_error(TDY_ERR_LIB, "cell %d missing at its vertex %d", c, v);
+      if (canon_idx[v] >= 0) {
+        s.gv_j.push_back(((long long)a * P + canon_idx[v]) * 8);
+        s.gv_r.push_back(64 * P + (long long)a * P + canon_idx[v]);
+      } else {
+        s.gv_j.push_back(s.v_jv_off[v] + (long long)a * nint);
+        s.gv_r.push_back(s.v_jv_off[v] + (long long)nint * nint + a);
+      }
+    }
+    order.clear();
+    for (int n = ncv; n > 0; n--)
+      for (int k = 0; k < rn; k++)
+        if (count[k] == n) order.push_back(k);
+    for (int slot : order) {
+      uint64_t w[2] = {~0ull, ~0ull};
+      for (int k = 0; k < count[slot]; k++) {
+        const uint64_t b = from[slot][k];
+        if (s.ge_words == 1)
+          w[0] = (w[0] & ~(0xffull << (8 * k))) | b << (8 * k);
+        else
+          w[k / 4] = (w[k / 4] & ~(0xffffull << (16 * (k % 4)))) | b << (16 * (k % 4));
+      }
+      s.ge_code.insert(s.ge_code.end(), w, w + s.ge_words);
+      s.ge_slot.push_back((uint8_t)slot);
+    }
+    if ((int)order.size() != rn) return set_error(TDY_ERR_LIB, "cell %d: a matrix entry without a vertex", c);
+    s.gc_diag.push_back((uint8_t)(std::lower_bound(row, row + rn, c) - row));
+    s.gv_off.push_back((int)s.gv_j.size());
+    s.ge_off.push_back((int)s.ge_slot.size());
   }
   s.nS = (int)s.sc_cells.size();
   s.nSpad = ((s.nS + 31) / 32) * 32;
