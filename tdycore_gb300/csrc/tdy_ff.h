@@ -83,8 +83,31 @@ __device__ __forceinline__ double ff_f2d(float f, int s) {
   return __hiloint2double((int)(sign | ((unsigned)de << 20) | ((u & 0x7fffffu) >> 3)), (int)(u << 29));
 }
 
-// (hi + lo) * 2^s rounded once to double
-__device__ __forceinline__ double ff_to_d(ff a, int s) { return __dadd_rn(ff_f2d(a.h, s), ff_f2d(a.l, s)); }
+// (hi + lo) * 2^s rounded once to double, without the FP64 pipe (a warp's
+// addition occupies it for 57 cycles): the pair renormalised by TwoSum, lo
+// rounded to a whole number of the double's last places (ties to even: hi's 24
+// bits leave 29 zeros below them, so the parity is lo's) and added to the
+// mantissa.  The same bits as adding the two in FP64, which is left for zeros
+// with a remainder, for results near the ends of the exponent range, and for
+// sums below hi's power of two.
+__device__ __forceinline__ double ff_to_d(ff a, int s) {
+  const float h = __fadd_rn(a.h, a.l);
+  const float bp = __fadd_rn(h, -a.h);
+  const float l = __fadd_rn(__fadd_rn(a.h, -__fadd_rn(h, -bp)), __fadd_rn(a.l, -bp));
+  const unsigned u = __float_as_uint(h);
+  const int e = (int)((u >> 23) & 0xffu), de = e + 896 + s;
+  const float places = __uint_as_float((unsigned)(306 - e) << 23);  // 2^52 / 2^(e - 127); e >= 60 below
+  int li = __float2int_rn(__fmul_rn(l, places));
+  li = (int)u < 0 ? -li : li;
+  // (a power of two with a remainder of the other sign: the sum lies below it)
+  if (e < 60 || de <= 1 || de >= 2046 ||
+      ((u & 0x7fffffu) == 0 && l != 0.0f && (int)(u ^ __float_as_uint(l)) < 0)) {
+    if ((u & 0x7fffffffu) == 0 && l == 0.0f) return 0.0;
+    return __dadd_rn(ff_f2d(a.h, s), ff_f2d(a.l, s));
+  }
+  const long long m = __double_as_longlong(__hiloint2double((int)(((unsigned)de << 20) | ((u & 0x7fffffu) >> 3)), (int)(u << 29))) + li;
+  return __longlong_as_double(m | ((long long)(u & 0x80000000u) << 32));
+}
 
 __device__ __forceinline__ ff ff_neg(ff a) {
   ff r;

@@ -87,6 +87,7 @@ struct DevArgs {
   const double *bnd_val, *bnd_rho, *bnd_vis;
   // extended state (cells then boundary faces): P, rho/2, (drho/dP)/2, kr/mu,
   // d(kr/mu)/dP, seepage flag
+  // (constant density: lam holds rho kr/mu, every row's w)
   double *P, *hr, *hdr, *lam, *dlam;
   unsigned char *seep;
   double *acc_a, *acc_b, *jdiag;
@@ -456,7 +457,7 @@ __device__ __forceinline__ void state_entity(const DevArgs &a, int i) {
       a.hr[i] = 0.5 * rho;
       a.hdr[i] = 0.5 * drho;
     }
-    a.lam[i] = lam;
+    a.lam[i] = a.rho_type == WATER_DENSITY_CONSTANT ? __dmul_rn(kRhoConst, lam) : lam;
     a.dlam[i] = dlam;
     const double poro = a.poro[i], vol = a.vol[i];
     // d(rho phi S)/dP (the porosity does not depend on pressure)
@@ -499,7 +500,7 @@ __device__ __forceinline__ void state_entity(const DevArgs &a, int i) {
     a.P[i] = p;
     a.hr[i] = 0.5 * a.bnd_rho[b];
     a.hdr[i] = 0.0;
-    a.lam[i] = lam;
+    a.lam[i] = a.rho_type == WATER_DENSITY_CONSTANT ? __dmul_rn(kRhoConst, lam) : lam;
     a.dlam[i] = 0.0;
     a.seep[i] = (a.bnd_type[b] == SEEPAGE_BC && p <= a.Pref) ? 1 : 0;
   }
@@ -670,7 +671,7 @@ __device__ __forceinline__ void canon_vertex_at(const DevArgs &a, int vc, int ti
     const double q = __fma_rn(den, G, TP);
     const bool fdn = dneg(q);
     const double lm = fdn ? lam[u] : lam[d];
-    const double w = __dmul_rn(den, lm);
+    const double w = RHO == RHO_CONST ? lm : __dmul_rn(den, lm);
     const double flux = -__dmul_rn(w, q);
     // an octant's partial residual starts from its first row's flux
     if (r == canon_first_row(u))
@@ -831,12 +832,15 @@ __device__ __forceinline__ void canon_vertex_pair(const DevArgs &a, int vc, int 
   }
   __syncwarp(pm);
   double fx[2], fy[2], fz[2];
+  // octant of the up side of the lane's row t (canon_up)
+  auto up_octant = [&](int axis, int i) { return h ? (axis == 0 ? 4 + 2 * i : axis == 1 ? 4 + i : 2 + i) : (axis == 0 ? 2 * i : i); };
+  unsigned down = 0;  // constant density: bit t, the row's upwind cell is its up cell
+  long long any_e = 0;
 #pragma unroll
   for (int t = 0; t < 6; t++) {
     const int axis = t >> 1, i = t & 1;
     const int r = 4 * axis + 2 * h + i;
-    // octants of row r (canon_up, canon_dn) for this lane
-    const int u = h ? (axis == 0 ? 4 + 2 * i : axis == 1 ? 4 + i : 2 + i) : (axis == 0 ? 2 * i : i);
+    const int u = up_octant(axis, i);
     const int d = u + (1 << axis);
     const double *T = a.Tc + (long long)(r * 8) * P + vc;
     double TP = __dmul_rn(T[0], p[0]);
@@ -848,13 +852,20 @@ __device__ __forceinline__ void canon_vertex_pair(const DevArgs &a, int vc, int 
     const bool fdn = dneg(q);
     const int uw = fdn ? u : d;  // upwind octant
     const double lm = s_lam[uw * ns + slot];
-    const double w = __dmul_rn(den, lm);
+    const double w = RHO == RHO_CONST ? lm : __dmul_rn(den, lm);
     const double flux = -__dmul_rn(w, q);
     (axis == 0 ? fx : axis == 1 ? fy : fz)[i] = flux;
     if (a.needJ) {
       const double dl = s_dlam[uw * ns + slot];
       double eu, ed;
-      if (CONST_RHO) {
+      if (RHO == RHO_CONST) {
+        // E below, for the warps that have any (dl = 0 in saturated cells)
+        eu = q;
+        ed = 0.0;
+        down |= (unsigned)fdn << t;
+        any_e |= __double_as_longlong(dl) << 1;
+        any_e |= d_bexp(q) == 0x7ff;
+      } else if (CONST_RHO) {
         const double e = __dmul_rn(__dmul_rn(den, q), dl);
         eu = fdn ? e : 0.0;
         ed = fdn ? 0.0 : e;
@@ -883,11 +894,26 @@ __device__ __forceinline__ void canon_vertex_pair(const DevArgs &a, int vc, int 
       const double f3 = ((ol >> 1) == h) ? fz[ol & 1] : pz[ol & 1];
       double Rv = (ol & 1) ? -f1 : f1;
       Rv = (ol & 2) ? Rv - f2 : Rv + f2;
-      Rv = h ? Rv - f3 : Rv + f3;
+      // (one addition: a predicated one of the other sign takes the pipe as long)
+      Rv += __longlong_as_double(__double_as_longlong(f3) ^ ((long long)h << 63));
       S[64 * P + (4 * h + ol) * P + vc] = Rv;
     }
   }
   if (!a.needJ) return;
+  // whether any row of this warp's vertices has an E term
+  const bool with_e = RHO != RHO_CONST || __any_sync(__activemask(), any_e != 0);
+  if (RHO == RHO_CONST && with_e) {
+#pragma unroll 1
+    for (int t = 0; t < 6; t++) {
+      const int axis = t >> 1, i = t & 1, r = 4 * axis + 2 * h + i;
+      const bool fdn = down >> t & 1;
+      const int u = up_octant(axis, i);
+      const double dl = s_dlam[(fdn ? u : u + (1 << axis)) * ns + slot];
+      const double e = __dmul_rn(__dmul_rn(kRhoConst, sh[(12 + r) * ns + slot]), dl);
+      sh[(12 + r) * ns + slot] = fdn ? e : 0.0;
+      sh[(24 + r) * ns + slot] = fdn ? 0.0 : e;
+    }
+  }
   __syncwarp(pm);
 #pragma unroll 1
   for (int c = 0; c < 8; c++) {
@@ -902,15 +928,18 @@ __device__ __forceinline__ void canon_vertex_pair(const DevArgs &a, int vc, int 
       const bool up = canon_is_up(c, k);
       wk[k] = sh[r * ns + slot];
       bw[k] = d_bexp(wk[k]);
-      const double eu = sh[(12 + r) * ns + slot], ed = sh[(24 + r) * ns + slot];
-      es[k] = up ? eu : ed;  // E term of c itself (entry 0)
-      en[k] = up ? ed : eu;  // E term of the neighbour c ^ (1 << k) (entry 1 << k)
+      if (with_e) {
+        const double eu = sh[(12 + r) * ns + slot], ed = sh[(24 + r) * ns + slot];
+        es[k] = up ? eu : ed;  // E term of c itself (entry 0)
+        en[k] = up ? ed : eu;  // E term of the neighbour c ^ (1 << k) (entry 1 << k)
+      }
       const double *T = a.Tc + (long long)(r * 8) * P + vc;
 #pragma unroll
       for (int jj = 0; jj < 4; jj++) {
         Tk[k][jj] = T[((4 * h + jj) ^ c) * P];
         mb[jj] = max(mb[jj], bw[k] + d_bexp(Tk[k][jj]) - 1023);
       }
+      if (!with_e) continue;
       if (k < 2) {
         if (h == 0) {
           mb[0] = max(mb[0], d_bexp(es[k]));
@@ -927,17 +956,18 @@ __device__ __forceinline__ void canon_vertex_pair(const DevArgs &a, int vc, int 
     for (int k = 0; k < 3; k++) {
       const bool up = canon_is_up(c, k);
       ff wf = ff_split_scaled(wk[k], bw[k], 1023 - bw[k]);
+      if (up) wf = ff_neg(wf);
+#pragma unroll
+      for (int jj = 0; jj < 4; jj++)
+        ff_acc(acc[jj], ff_mul(wf, ff_split_scaled(Tk[k][jj], d_bexp(Tk[k][jj]), bw[k] - mb[jj])));
+      if (!with_e) continue;
       const double e0 = h ? en[k] : es[k];
       ff ef = ff_split_scaled(e0, d_bexp(e0), 1023 - mb[0]);
       ff nf = k < 2 ? ff_split_scaled(en[k], d_bexp(en[k]), 1023 - mb[(1 << k) & 3]) : ff{0.0f, 0.0f};
       if (up) {
-        wf = ff_neg(wf);
         ef = ff_neg(ef);
         nf = ff_neg(nf);
       }
-#pragma unroll
-      for (int jj = 0; jj < 4; jj++)
-        ff_acc(acc[jj], ff_mul(wf, ff_split_scaled(Tk[k][jj], d_bexp(Tk[k][jj]), bw[k] - mb[jj])));
       if (h == 0 || k == 2) ff_acc(acc[0], ef);
       if (k < 2 && h == 0) ff_acc(acc[(1 << k) & 3], nf);
     }
@@ -1024,7 +1054,7 @@ __device__ __forceinline__ void generic_vertex_group(const DevArgs &a, int block
     const int u = flowdn ? up : dn;
     const double lm = sl[u];
     const bool zero = sp[u] != 0;
-    const double wr = zero ? 0.0 : __dmul_rn(den, lm);
+    const double wr = zero ? 0.0 : vary ? __dmul_rn(den, lm) : lm;
     fl[r] = -__dmul_rn(wr, q);
     if (a.needJ) {
       double eu = 0.0, ed = 0.0;
@@ -1576,6 +1606,9 @@ static int pack_generic(const _p_TDy *t, std::vector<GenVertex> &gen, std::vecto
   const MPFAOSetup &s = t->setup;
   int max_row = 1, max_col = 1;
   long long trans = 0;
+  gen.reserve(s.gen_vertex.size());
+  g_rowG.reserve(s.nrows);
+  g_rowc.reserve(s.nrows);
   for (int v : s.gen_vertex) {
     GenVertex d;
     const int r0 = s.v_row_off[v], nrow = s.v_row_off[v + 1] - r0;
@@ -1594,7 +1627,7 @@ static int pack_generic(const _p_TDy *t, std::vector<GenVertex> &gen, std::vecto
     g_col.insert(g_col.end(), s.col_ext.begin() + c0, s.col_ext.begin() + c0 + ncol);
     g_cell.insert(g_cell.end(), nint, make_uint2(0x00ffffffu, 0x00ffffffu));
     uint2 *cells = g_cell.data() + d.cell0;
-    std::vector<int> count(nint, 0);
+    int count[TDY_MAX_NINT] = {0};
     auto add = [&](int c, int r, bool up, int other) {
       if (c < 0) return true;
       const int k = count[c]++;

@@ -574,7 +574,7 @@ int mpfao_setup(const Options &opt, const Mesh &m, const Materials &mat, const B
 
   // ---- structured interior cells, and the gather program of the others ----
   std::vector<std::array<int, 8>> svc;
-  for (int c = 0; c < nc; c++) {
+  for (int c = 0; c < nc; c++) {  // (over every cell: a bound)
     int vals = 0;
     for (int j = m.cell_vert_off[c]; j < m.cell_vert_off[c + 1]; j++) vals += s.v_nint[m.cell_verts[j]];
     s.gc_max_vals = std::max(s.gc_max_vals, vals);
@@ -582,8 +582,20 @@ int mpfao_setup(const Options &opt, const Mesh &m, const Materials &mat, const B
   s.ge_words = s.gc_max_vals > 255 ? 2 : 1;
   s.gv_off.assign(1, 0);
   s.ge_off.assign(1, 0);
-  std::vector<int> count, order;
-  std::vector<std::array<uint16_t, 8>> from;  // per slot: positions
+  // (rows of cells with a vertex outside the canonical ones, at most)
+  {
+    size_t nnz = 0;
+    for (int c = 0; c < nc; c++) {
+      bool inner = s.rowptr[c + 1] - s.rowptr[c] == 27;
+      for (int j = m.cell_vert_off[c]; inner && j < m.cell_vert_off[c + 1]; j++) inner = canon_idx[m.cell_verts[j]] >= 0;
+      if (!inner) nnz += s.rowptr[c + 1] - s.rowptr[c];
+    }
+    s.ge_slot.reserve(nnz);
+    s.ge_code.reserve(s.ge_words * nnz);
+  }
+  uint8_t count[256];      // per slot: its contributions so far,
+  uint64_t word[256][2];   // and their positions
+  size_t other_nnz = 0;
   for (int c = 0; c < nc; c++) {
     const int *row = &s.colidx[s.rowptr[c]];
     const int rn = s.rowptr[c + 1] - s.rowptr[c];
@@ -609,22 +621,26 @@ int mpfao_setup(const Options &opt, const Mesh &m, const Materials &mat, const B
       continue;
     }
     s.gc_cells.push_back(c);
-    count.assign(rn, 0);
-    from.resize(std::max<size_t>(from.size(), rn));
+    std::memset(count, 0, rn);
+    std::memset(word, 0xff, sizeof(word[0]) * rn);
     int pos = 0;
     for (int j = 0; j < ncv; j++) {
       const int v = cv[j], nint = s.v_nint[v];
-      int a = -1;
-      for (int k = 0; k < nint; k++) {
+      const bool canon = canon_idx[v] >= 0;  // (else the columns ascend)
+      int a = -1, slot = 0;
+      for (int k = 0; k < nint; k++, pos++) {
         const int col = column(j, k);
         if (col == c) a = k;
-        const int slot = (int)(std::lower_bound(row, row + rn, col) - row);
-        from[slot][count[slot]++] = (uint16_t)(pos + k);
+        slot = (int)(std::lower_bound(row + (canon ? 0 : slot), row + rn, col) - row);
+        const int n = count[slot]++;
+        if (s.ge_words == 1)
+          word[slot][0] ^= (uint64_t)(0xff ^ pos) << (8 * n);
+        else
+          word[slot][n / 4] ^= (uint64_t)(0xffff ^ pos) << (16 * (n % 4));
       }
-      s.gv_n.push_back((uint32_t)pos | (uint32_t)nint << 16);
-      pos += nint;
       if (a < 0) return set_error(TDY_ERR_LIB, "cell %d missing at its vertex %d", c, v);
-      if (canon_idx[v] >= 0) {
+      s.gv_n.push_back((uint32_t)(pos - nint) | (uint32_t)nint << 16);
+      if (canon) {
         s.gv_j.push_back(((long long)a * P + canon_idx[v]) * 8);
         s.gv_r.push_back(64 * P + (long long)a * P + canon_idx[v]);
       } else {
@@ -632,26 +648,27 @@ int mpfao_setup(const Options &opt, const Mesh &m, const Materials &mat, const B
         s.gv_r.push_back(s.v_jv_off[v] + (long long)nint * nint + a);
       }
     }
-    order.clear();
-    for (int n = ncv; n > 0; n--)
-      for (int k = 0; k < rn; k++)
-        if (count[k] == n) order.push_back(k);
-    for (int slot : order) {
-      uint64_t w[2] = {~0ull, ~0ull};
-      for (int k = 0; k < count[slot]; k++) {
-        const uint64_t b = from[slot][k];
-        if (s.ge_words == 1)
-          w[0] = (w[0] & ~(0xffull << (8 * k))) | b << (8 * k);
-        else
-          w[k / 4] = (w[k / 4] & ~(0xffffull << (16 * (k % 4)))) | b << (16 * (k % 4));
-      }
-      s.ge_code.insert(s.ge_code.end(), w, w + s.ge_words);
-      s.ge_slot.push_back((uint8_t)slot);
+    // entries by their number of contributions, the most first
+    int start[10] = {0};
+    for (int k = 0; k < rn; k++) start[count[k]]++;
+    if (start[0]) return set_error(TDY_ERR_LIB, "cell %d: a matrix entry without a vertex", c);
+    for (int n = 8, at = 0; n > 0; n--) {
+      const int here = start[n];
+      start[n] = at;
+      at += here;
     }
-    if ((int)order.size() != rn) return set_error(TDY_ERR_LIB, "cell %d: a matrix entry without a vertex", c);
+    const size_t e0 = other_nnz;
+    s.ge_slot.resize(e0 + rn);
+    s.ge_code.resize(s.ge_words * (e0 + rn));
+    for (int k = 0; k < rn; k++) {
+      const size_t e = e0 + start[count[k]]++;
+      s.ge_slot[e] = (uint8_t)k;
+      for (int w = 0; w < s.ge_words; w++) s.ge_code[s.ge_words * e + w] = word[k][w];
+    }
+    other_nnz += rn;
     s.gc_diag.push_back((uint8_t)(std::lower_bound(row, row + rn, c) - row));
     s.gv_off.push_back((int)s.gv_j.size());
-    s.ge_off.push_back((int)s.ge_slot.size());
+    s.ge_off.push_back((int)other_nnz);
   }
   s.nS = (int)s.sc_cells.size();
   s.nSpad = ((s.nS + 31) / 32) * 32;
