@@ -351,8 +351,6 @@ __device__ __forceinline__ bool vg_mualem(const double *par, const double *p, do
   const double Se = exp2_fx(fx_neg(mw)), oms = __dadd_rn(1.0, -Sr);
   c->S = __fma_rn(oms, Se, Sr);
   if (!want_kr && !want_d) return true;
-  // (the exponent m (n log2 x - log2 w): 1 - t cancels in dry soil)
-  const double t = exp2_fx(fx_scale(m, fx_add(tn, fx_neg(lw))));
   double g = 0.0, u = 0.0, xi = 0.0, us = 0.0;  // us: x^(n-1) Se
   if (want_d) {
     const double wi = exp2_fx(fx_neg(lw)), mn = __dmul_rn(m, n);
@@ -373,7 +371,22 @@ __device__ __forceinline__ bool vg_mualem(const double *par, const double *p, do
     if (want_d) c->dkr = __dmul_rn((p[6] + xt * (2.0 * p[7] + xt * 3.0 * p[8])) / dx, __dmul_rn(g, us));
     return true;
   }
-  const double f = __dadd_rn(1.0, -t), sq = exp2_fx(fx_neg(fx_half(mw)));
+  // f = 1 - t cancels in dry soil, where s = 1/w is small: there by the
+  // binomial series of 1 - (1 - s)^m (its sixth term is below 2^-47), else
+  // before any rounding.  kr is then within 1e-12 of 300-bit arithmetic (x up
+  // to 1e6); the plain formulas lose 7 digits at x = 100, all by 1e6.
+  double f;
+  if (lw.k >= 9) {
+    const double so = exp2_fx(fx_neg(lw));
+    f = __fma_rn(__dmul_rn(__dadd_rn(4.0, -m), 0.2), so, 1.0);
+    f = __fma_rn(__dmul_rn(__dmul_rn(__dadd_rn(3.0, -m), 0.25), so), f, 1.0);
+    f = __fma_rn(__dmul_rn(__dmul_rn(__dadd_rn(2.0, -m), 1.0 / 3.0), so), f, 1.0);
+    f = __fma_rn(__dmul_rn(__dmul_rn(__dadd_rn(1.0, -m), 0.5), so), f, 1.0);
+    f = __dmul_rn(__dmul_rn(m, so), f);
+  } else {
+    f = one_minus_exp2_fx(fx_scale(m, fx_add(tn, fx_neg(lw))));
+  }
+  const double sq = exp2_fx(fx_neg(fx_half(mw)));
   c->kr = __dmul_rn(sq, __dmul_rn(f, f));
   if (want_d)
     c->dkr = __dmul_rn(g, __fma_rn(__dmul_rn(0.5, c->kr), u, __dmul_rn(__dmul_rn(2.0, __dmul_rn(sq, xi)), __dmul_rn(f, us))));

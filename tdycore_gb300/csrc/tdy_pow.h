@@ -145,9 +145,9 @@ __device__ __forceinline__ fx fx_scale(double y, fx a) {
   return t;
 }
 
-// 2^a, |a| < 1000
-__device__ __forceinline__ double exp2_fx(fx a) {
-  const int k = a.k + (int)(a.f >> 62);
+// 2^(fraction of a) with 63 fraction bits, in [1, 2); *k: the integer part
+__device__ __forceinline__ unsigned long long exp2_fraction(fx a, int *k) {
+  *k = a.k + (int)(a.f >> 62);
   const unsigned long long f = (unsigned long long)a.f & 0x3fffffffffffffffULL;
   const unsigned long long T = kExpTable[(int)(f >> 55)];
   const unsigned long long s = fx_umulhi((f & 0x7fffffffffffffULL) << 2, 0xb17217f7d1cf79acULL);  // 64 fraction bits
@@ -157,9 +157,27 @@ __device__ __forceinline__ double exp2_fx(fx a) {
   const unsigned long long g3 = 0x2aaaaaaaaaaaaaabULL + (((unsigned long long)s39 * q) >> 7);
   const unsigned long long g2 = 0x8000000000000000ULL + fx_umulhi(s, g3);
   const unsigned long long p = s + fx_umulhi(s, fx_umulhi(s, g2));
-  const unsigned long long v = T + fx_umulhi(T, p);  // [1, 2), 63 fraction bits
+  return T + fx_umulhi(T, p);
+}
+
+// 2^a, |a| < 1000
+__device__ __forceinline__ double exp2_fx(fx a) {
+  int k;
+  const unsigned long long v = exp2_fraction(a, &k);
   // round to 53 bits; a carry moves into the exponent
   return __longlong_as_double(((long long)(k + 1022) << 52) + (long long)((v >> 11) + ((v >> 10) & 1)));
+}
+
+// 1 - 2^a, -1000 < a < -2^-50, to 2^-62: the difference is formed before the
+// rounding to 53 bits
+__device__ __forceinline__ double one_minus_exp2_fx(fx a) {
+  int k;
+  const unsigned long long v = exp2_fraction(a, &k);
+  if (k < -60) return 1.0;
+  const unsigned long long u = 0ULL - (v >> (-1 - k));  // 64 fraction bits
+  const int lz = __clzll((long long)u);
+  const unsigned long long m = u << lz;
+  return __longlong_as_double(((long long)(1021 - lz) << 52) + (long long)((m >> 11) + ((m >> 10) & 1)));
 }
 
 }  // namespace tdy

@@ -73,3 +73,54 @@ def test_residual_and_jacobian(same_m):
              o.ts_ijacobian(U, Ut, 0.01, with_mag=True))):
         assert np.all(np.abs(R - Ro) <= 1e-12 * Rm)
         assert np.all(np.abs(J - Jo) <= 1e-10 * Jm)
+
+
+# wet to very dry: the plain formula of kr loses 7 digits at x = 100
+@pytest.mark.parametrize("log_x", [(-1.5, 0), (0, 2), (2, 6)])
+def test_relative_permeability(log_x):
+    """kr of dry soil in extended precision, from the flux between two cells
+    (accumulation suppressed by a huge time step).  Tolerance 1e-12: kr itself
+    is within 1e-13 of 300-bit arithmetic, the flux adds a few roundings."""
+    r = np.random.default_rng(9)
+    n = 256
+    T.options_clear()
+    t = T.create_richards_mpfao()
+    xy, quads = W.structured_surface(1, 1, 1.0, 1.0)
+    blocks = []
+    for b in range(n):
+        s = xy.copy()
+        s[:, 0] += 2.0 * b
+        blocks.append((s, quads, W.layered_z(4, 2, 1.0)))
+    t.set_extruded_meshes(blocks)
+    t.set_from_options()
+    m, alpha = np.repeat(r.uniform(0.2, 0.6, n), 2), np.repeat(10.0 ** r.uniform(-5, -3, n), 2)
+    t.set_vangenuchten_values(m, alpha)
+    t.set_mualem_values(m)
+    t.set_constant_isotropic_permeability(1e-12)
+    t.set_boundary_pressure_type_function(lambda x, y, z: np.full(np.shape(x), T.NEUMANN_BC))
+    t.set_water_density_type(T.WATER_DENSITY_CONSTANT)
+    t.setup()
+    x = 10.0 ** r.uniform(*log_x, 2 * n)
+    x[1::2] = 3.0 * x[::2]
+    U = 101325.0 - x / alpha
+    t.set_dtime(1e60)
+    t.presolve(U)
+    R = t.snes_function(U)[::2]
+    v = t.setup_view()
+    L = np.longdouble
+    # every vertex of a block has one row, its face's up cell first: sum the four
+    q = np.zeros(n, dtype=L)
+    for k in range(v["nverts"]):
+        r0, r1, c0 = v["v_row_off"][k], v["v_row_off"][k + 1], v["v_col_off"][k]
+        if r1 > r0:
+            Tr = v["trans"][v["v_trans_off"][k]:v["v_trans_off"][k] + 2].astype(L)
+            cols = v["col_ext"][c0:c0 + 2]
+            q[cols[0] // 2] += Tr @ U[cols].astype(L) + L(998.0) * L(v["gravdis"][v["row_face"][r0]])
+    up = np.where(q < 0, np.arange(n) * 2, np.arange(n) * 2 + 1)
+    ml = m[up].astype(L)
+    w = 1 + ((101325.0 - U[up]) * alpha[up]).astype(L) ** (1.0 / (1.0 - m[up])).astype(L)
+    kr = w ** (-ml / 2) * np.expm1(ml * np.log1p(-1 / w)) ** 2
+    flux = -q * L(998.0) * kr / L(9.94e-4)
+    dry = w ** (-ml) < 0.99
+    assert dry.sum() > n // 2
+    assert np.all(np.abs(R - flux)[dry] <= 1e-12 * np.abs(flux)[dry])
