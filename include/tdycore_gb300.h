@@ -239,9 +239,8 @@ typedef struct {
                           on the process's first solve; 1, 2, 4 or 8.  Every choice gives the same
                           bits (each row is summed in 8 phases added by a fixed tree) */
 } TDyNewtonOptions;
-/* Inner-solve schedules.  TILE: every kernel of a BiCGStab iteration runs over
- * all cells of the batch, instances masked as they converge (one iteration is
- * a CUDA graph).  BLOCK: one to eight CTAs per instance (a cluster) run the
+/* Inner-solve schedules.  TILE: one cooperative grid runs the BiCGStab loop over
+ * all cells of the batch, instances masked as they converge.  BLOCK: one to eight CTAs per instance (a cluster) run the
  * instance's whole BiCGStab loop (clusters take instances from a counter,
  * largest first); an instance of more than 65536 cells stays on the tile
  * schedule.  AUTO: an autotuner times the tile, block and split schedules (instances up to

@@ -13,9 +13,9 @@
 //     coupling of each column of an extruded block, Thomas algorithm, one
 //     thread per column), which carries the stiff vertical coupling of thin
 //     layers;
-//   * one BiCGStab iteration is built once as a CUDA graph with the explicit
-//     graph API (kernel nodes in a chain, no stream capture, so device calls
-//     that other threads make meanwhile cannot invalidate it) and replayed;
+//   * a solve is one launch: a cluster of CTAs per instance, or one
+//     cooperative grid for all cells (bicgstab_block_kernel,
+//     bicgstab_grid_kernel), whose loop ends with its last instance;
 //   * the sparse matrix-vector product's threads per row (1, 2, 4 or 8) are
 //     picked by timing the candidates on the first solve that uses them.
 // No reference counterpart: the reference hands F and J to PETSc's SNES/KSP.
@@ -35,7 +35,6 @@
 
 #include "tdy_arena.h"
 #include "tdy_device.h"
-#include "tdy_emit.h"
 
 namespace tdy {
 
@@ -51,7 +50,7 @@ namespace {
 inline unsigned nblk(long long n, int bs) { return (unsigned)((n + bs - 1) / bs); }
 
 // per-instance scalars, [slot][nseg]
-enum { S_RHO = 0, S_ALPHA, S_OMEGA, S_BETA, S_BNORM2, S_T1, S_T2, S_HALF, S_NSCAL };
+enum { S_RHO = 0, S_ALPHA, S_OMEGA, S_BETA, S_BNORM2, S_XNORM2, S_HALF, S_NSCAL };
 
 struct Krylov {
   bool ready = false;
@@ -63,9 +62,6 @@ struct Krylov {
   void *sell = nullptr;                                // matrix values of the block schedule's instances (T)
   void *clu = nullptr;                                 // clusters: LU factors (T), grown on demand
   size_t clu_cap = 0;                                  // elements of clu
-  cudaGraphExec_t graph = nullptr;
-  int graph_precond = -1;  // preconditioner the graph was built with
-  int graph_tpr = 0;       // spmv threads per row the graph was built with
   int tpr = 0;  // spmv threads per row (autotuned)
 };
 
@@ -81,14 +77,16 @@ struct SolverState {
   int *newt_active = nullptr, *lin_active = nullptr, *lin_its = nullptr;
   int nchunks = 0;
   int *chunk_off = nullptr, *seg_chunk = nullptr;  // chunks of the per-instance reductions
-  double *part = nullptr, *part2 = nullptr;
-  double linear_rtol = -1.0;
+  double *part = nullptr;
+  // the tile schedule's sums (accumulators and chunk sums) and counters, on its first use
+  double *grid_acc = nullptr, *grid_part = nullptr;
+  unsigned *grid_sync = nullptr;
   int *dpos = nullptr;  // position of each row's diagonal in the CSR values
   // strong-coupling clusters, rebuilt for every linear solve that uses them:
   // label per cell, a change flag, local index in its cluster (-1: the cell
   // takes its diagonal), the members of the 2..64-cell clusters (cluster by
-  // cluster, ascending cell index), their offsets and LU offsets, pivots
-  int *clab = nullptr, *cflag = nullptr, *cloc = nullptr, *cmem = nullptr, *coff = nullptr, *cpiv = nullptr;
+  // cluster, ascending cell index), their offsets and LU offsets, row orders
+  int *clab = nullptr, *cflag = nullptr, *cloc = nullptr, *cmem = nullptr, *coff = nullptr, *cperm = nullptr;
   long long *cluoff = nullptr;
   int ncl = 0;  // clusters of 2..64 cells in the current solve
   int ncl_cells = 0, ncl_big_cells = 0;  // cells in them; cells of clusters over 64 cells
@@ -96,8 +94,8 @@ struct SolverState {
   std::vector<int> h_lab, h_cnt, h_id, h_fill, h_loc, h_mem, h_off;
   std::vector<long long> h_luoff;
   Krylov k32, k64;
-  // schedules of the line-preconditioned inner solve (block: one CTA per
-  // instance; tile: the batch-wide graph): instances with at most
+  // schedules of the line-preconditioned inner solve (block: a cluster per
+  // instance; tile: one grid for all cells): instances with at most
   // block_max_cells cells take the block schedule (-2: not chosen yet)
   int *inst_line_off = nullptr, *block_inst = nullptr, *block_mask = nullptr, *ticket = nullptr;
   std::vector<int> h_inst_line_off, h_order;  // h_order: instances by size, largest first
@@ -133,10 +131,8 @@ struct SolverState {
     // (joined into the solve's stream, which every solve synchronises)
     device_pool_release(device, nullptr, fork);
     for (int i = 0; i < 3; i++) device_pool_release(device, side[i], joined[i]);
-    for (Krylov *k : {&k32, &k64}) {
-      if (k->graph) cudaGraphExecDestroy(k->graph);
+    for (Krylov *k : {&k32, &k64})
       if (k->clu) dmem_free(k->clu, st);
-    }
     for (void *p : allocs) dmem_free(p, st);
   }
 };
@@ -164,10 +160,10 @@ int sup(SolverState *s, T **p, const std::vector<T> &h) {
 // ---------------------------------------------------------------------------
 // kernels
 //
-// Two schedules run the BiCGStab iterations: "tile" (every kernel over all
-// cells of the batch, instances masked as they converge; one iteration is a
-// graph) and "block" (one CTA per instance runs its whole Krylov loop, see
-// bicgstab_block_kernel).  Both perform every floating-point operation of an
+// Two schedules run the BiCGStab iterations: "tile" (one grid works through
+// all cells of the batch, instances masked as they converge, see
+// bicgstab_grid_kernel) and "block" (a cluster per instance runs its whole
+// Krylov loop, see bicgstab_block_kernel).  Both perform every floating-point operation of an
 // instance in the same order with explicit roundings (the element operations
 // below, the chunked reductions, the per-row lane split of the product), so
 // an instance gets the same bits from either schedule.
@@ -218,43 +214,27 @@ __global__ void cast_masked_kernel(int n, const int *cell_seg, const int *flag, 
 constexpr int kChunk = 4096;
 
 template <class TA, class TB>
-__global__ void __launch_bounds__(256) chunk_dot_kernel(const int *chunk_off, const TA *a, const TB *b, const TA *c,
-                                                        const TB *d, double *part, double *part2) {
-  __shared__ double sh[2][256];
+__global__ void __launch_bounds__(256) chunk_dot_kernel(const int *chunk_off, const TA *a, const TB *b, double *part) {
+  __shared__ double sh[256];
   const int ch = blockIdx.x;
   const int i0 = chunk_off[ch], i1 = chunk_off[ch + 1];
-  double acc = 0.0, acc2 = 0.0;
-  for (int i = i0 + threadIdx.x; i < i1; i += blockDim.x) {
-    acc = op_dot(acc, a[i], b[i]);
-    if (c) acc2 = op_dot(acc2, c[i], d[i]);
-  }
-  sh[0][threadIdx.x] = acc;
-  sh[1][threadIdx.x] = acc2;
+  double acc = 0.0;
+  for (int i = i0 + threadIdx.x; i < i1; i += blockDim.x) acc = op_dot(acc, a[i], b[i]);
+  sh[threadIdx.x] = acc;
   __syncthreads();
   for (int w = blockDim.x / 2; w > 0; w >>= 1) {
-    if ((int)threadIdx.x < w) {
-      sh[0][threadIdx.x] += sh[0][threadIdx.x + w];
-      sh[1][threadIdx.x] += sh[1][threadIdx.x + w];
-    }
+    if ((int)threadIdx.x < w) sh[threadIdx.x] += sh[threadIdx.x + w];
     __syncthreads();
   }
-  if (threadIdx.x == 0) {
-    part[ch] = sh[0][0];
-    if (c) part2[ch] = sh[1][0];
-  }
+  if (threadIdx.x == 0) part[ch] = sh[0];
 }
 
-__global__ void chunk_sum_kernel(int nseg, const int *seg_chunk, const double *part, const double *part2, double *out,
-                                 double *out2) {
+__global__ void chunk_sum_kernel(int nseg, const int *seg_chunk, const double *part, double *out) {
   const int s = blockIdx.x * blockDim.x + threadIdx.x;
   if (s >= nseg) return;
-  double acc = 0.0, acc2 = 0.0;
-  for (int k = seg_chunk[s]; k < seg_chunk[s + 1]; k++) {
-    acc += part[k];
-    if (out2) acc2 += part2[k];
-  }
+  double acc = 0.0;
+  for (int k = seg_chunk[s]; k < seg_chunk[s + 1]; k++) acc += part[k];
   out[s] = acc;
-  if (out2) out2[s] = acc2;
 }
 
 // y = A x over the CSR pattern with TPR threads per row
@@ -315,140 +295,6 @@ __global__ void line_factor_kernel(int nlines, const int *line_off, const int *l
     lcp[i] = (T)cp;
     linv[i] = (T)inv;
   }
-}
-
-// out = (line-tridiagonal)^-1 in, line l
-template <class T>
-__device__ __forceinline__ void line_solve_one(int l, const int *line_off, const int *line_cells, const T *la,
-                                               const T *lcp, const T *linv, const T *in, T *out) {
-  const int k0 = line_off[l], k1 = line_off[l + 1];
-  T prev = 0;
-  for (int k = k0; k < k1; k++) {
-    const int i = line_cells[k];
-    prev = e_mul(e_fma(-la[i], prev, in[i]), linv[i]);
-    out[i] = prev;
-  }
-  T next = 0;
-  for (int k = k1 - 1; k >= k0; k--) {
-    const int i = line_cells[k];
-    next = e_fma(-lcp[i], next, out[i]);
-    out[i] = next;
-  }
-}
-template <class T>
-__global__ void line_solve_kernel(int nlines, const int *line_off, const int *line_cells, const T *la, const T *lcp,
-                                  const T *linv, const T *in, T *out) {
-  const int l = blockIdx.x * blockDim.x + threadIdx.x;
-  if (l >= nlines) return;
-  line_solve_one(l, line_off, line_cells, la, lcp, linv, in, out);
-}
-
-template <class T>
-__global__ void init_kernel(int n, const int *cell_seg, const int *active, const double *F, T *b, T *r, T *r0, T *p,
-                            T *v, T *y) {
-  const int i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= n) return;
-  const T f = active[cell_seg[i]] ? (T)F[i] : (T)0;
-  b[i] = f;
-  r[i] = f;
-  r0[i] = f;
-  p[i] = 0;
-  v[i] = 0;
-  y[i] = 0;
-}
-
-// (instances on the block schedule stay inactive in the tile iterations)
-__global__ void init_scalars_kernel(int nseg, const int *newt_active, const int *block_mask, int *lin_active,
-                                    int *lin_its, double *scal) {
-  const int s = blockIdx.x * blockDim.x + threadIdx.x;
-  if (s >= nseg) return;
-  scal[S_RHO * nseg + s] = 1.0;
-  scal[S_ALPHA * nseg + s] = 1.0;
-  scal[S_OMEGA * nseg + s] = 1.0;
-  scal[S_HALF * nseg + s] = 0.0;
-  lin_active[s] = newt_active[s] && scal[S_BNORM2 * nseg + s] > 0.0 && !block_mask[s];
-}
-
-// after rho_new = (r0, r) in T1
-__global__ void scal_beta_kernel(int nseg, int *act, double *sc) {
-  const int s = blockIdx.x * blockDim.x + threadIdx.x;
-  if (s >= nseg || !act[s]) return;
-  const double rn = sc[S_T1 * nseg + s];
-  if (rn == 0.0) {
-    act[s] = 0;
-    return;
-  }
-  sc[S_BETA * nseg + s] = (rn / sc[S_RHO * nseg + s]) * (sc[S_ALPHA * nseg + s] / sc[S_OMEGA * nseg + s]);
-  sc[S_RHO * nseg + s] = rn;
-}
-// after (r0, v) in T1
-__global__ void scal_alpha_kernel(int nseg, int *act, double *sc) {
-  const int s = blockIdx.x * blockDim.x + threadIdx.x;
-  if (s >= nseg || !act[s]) return;
-  const double d = sc[S_T1 * nseg + s];
-  if (d == 0.0) {
-    act[s] = 0;
-    return;
-  }
-  sc[S_ALPHA * nseg + s] = sc[S_RHO * nseg + s] / d;
-}
-// after (s, s) in T1: converged already at the half step?
-__global__ void scal_half_kernel(int nseg, const int *act, double *sc, double tol2) {
-  const int s = blockIdx.x * blockDim.x + threadIdx.x;
-  if (s >= nseg || !act[s]) return;
-  sc[S_HALF * nseg + s] = (sc[S_T1 * nseg + s] <= tol2 * sc[S_BNORM2 * nseg + s]) ? 1.0 : 0.0;
-}
-// after (t, t) in T1 and (t, s) in T2
-__global__ void scal_omega_kernel(int nseg, const int *act, double *sc) {
-  const int s = blockIdx.x * blockDim.x + threadIdx.x;
-  if (s >= nseg || !act[s]) return;
-  const double tt = sc[S_T1 * nseg + s];
-  sc[S_OMEGA * nseg + s] = tt > 0.0 ? sc[S_T2 * nseg + s] / tt : 0.0;
-}
-// after (r, r) in T1
-__global__ void scal_check_kernel(int nseg, int *act, int *its, double *sc, double tol2) {
-  const int s = blockIdx.x * blockDim.x + threadIdx.x;
-  if (s >= nseg || !act[s]) return;
-  its[s] += 1;
-  if (sc[S_HALF * nseg + s] != 0.0 || sc[S_T1 * nseg + s] <= tol2 * sc[S_BNORM2 * nseg + s] ||
-      sc[S_OMEGA * nseg + s] == 0.0)
-    act[s] = 0;
-}
-
-template <class T>
-__global__ void p_update_kernel(int n, const int *cs, const int *act, const double *sc, int nseg, const T *r, const T *v,
-                                T *p) {
-  const int i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= n) return;
-  const int s = cs[i];
-  if (!act[s]) return;
-  const T beta = (T)sc[S_BETA * nseg + s], omega = (T)sc[S_OMEGA * nseg + s];
-  p[i] = op_p(r[i], p[i], v[i], beta, omega);
-}
-template <class T>
-__global__ void s_update_kernel(int n, const int *cs, const int *act, const double *sc, int nseg, const T *r, const T *v,
-                                T *sv) {
-  const int i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= n) return;
-  const int s = cs[i];
-  if (!act[s]) return;
-  sv[i] = e_fma(-(T)sc[S_ALPHA * nseg + s], v[i], r[i]);
-}
-template <class T>
-__global__ void xr_update_kernel(int n, const int *cs, const int *act, const double *sc, int nseg, const T *ph,
-                                 const T *sh, const T *sv, const T *tv, T *y, T *r) {
-  const int i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= n) return;
-  const int s = cs[i];
-  if (!act[s]) return;
-  const T alpha = (T)sc[S_ALPHA * nseg + s];
-  if (sc[S_HALF * nseg + s] != 0.0) {
-    y[i] = op_y(y[i], ph[i], alpha);
-    return;
-  }
-  const T omega = (T)sc[S_OMEGA * nseg + s];
-  y[i] = op_y2(y[i], ph[i], sh[i], alpha, omega);
-  r[i] = e_fma(-omega, tv[i], sv[i]);
 }
 
 // ---------------------------------------------------------------------------
@@ -1120,13 +966,15 @@ constexpr int kClusterLd = kClusterMax + 1;  // padded row of the staged block
 
 // One warp per cluster: stage the cluster's block of J (every coupling
 // between its cells) in shared memory, factor it by LU with partial pivoting
-// (ties to the smaller row; a zero pivot becomes 1), store the factors.
+// (ties to the smaller row; a zero pivot becomes 1), store the factors column
+// by column (the solves read a column at a time) and the order of the rows.
 template <class T>
 __global__ void __launch_bounds__(32) cl_factor_kernel(int ncl, const int *coff, const long long *luoff,
                                                        const int *cmem, const int *loc, const int *lab,
                                                        const int *rowptr, const int *colidx, const double *J, T *lu,
-                                                       int *piv) {
+                                                       int *perm) {
   extern __shared__ unsigned char cl_smem[];
+  __shared__ int order[kClusterMax];
   T *B = reinterpret_cast<T *>(cl_smem);  // [kClusterMax][kClusterLd]
   const int cl = blockIdx.x, lane = threadIdx.x;
   if (cl >= ncl) return;
@@ -1134,6 +982,7 @@ __global__ void __launch_bounds__(32) cl_factor_kernel(int ncl, const int *coff,
   for (int e = lane; e < sz * kClusterLd; e += 32) B[e] = (T)0;
   __syncwarp();
   for (int r = lane; r < sz; r += 32) {
+    order[r] = r;
     const int m = cmem[c0 + r], L = lab[m];
     for (int k = rowptr[m]; k < rowptr[m + 1]; k++) {
       const int col = colidx[k];
@@ -1161,7 +1010,11 @@ __global__ void __launch_bounds__(32) cl_factor_kernel(int ncl, const int *coff,
       }
     }
     bi = __shfl_sync(0xffffffffu, bi, 0);
-    if (lane == 0) piv[c0 + kk] = bi;
+    if (lane == 0 && bi != kk) {
+      const int t = order[kk];
+      order[kk] = order[bi];
+      order[bi] = t;
+    }
     if (bi != kk)
       for (int j = lane; j < sz; j += 32) {
         const T t = B[kk * kClusterLd + j];
@@ -1181,139 +1034,448 @@ __global__ void __launch_bounds__(32) cl_factor_kernel(int ncl, const int *coff,
     __syncwarp();
   }
   T *out = lu + luoff[cl];
-  for (int e = lane; e < sz * sz; e += 32) out[e] = B[(e / sz) * kClusterLd + e % sz];
+  for (int e = lane; e < sz * sz; e += 32) out[e] = B[(e % sz) * kClusterLd + e / sz];
+  for (int r = lane; r < sz; r += 32) perm[c0 + r] = order[r];
 }
 
-template <class T>
-__global__ void cl_apply_diag_kernel(int n, const int *loc, const T *inv, const T *in, T *out) {
-  const int i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i < n && loc[i] < 0) out[i] = inv[i] * in[i];
-}
+// ---------------------------------------------------------------------------
+// Tile schedule: one cooperative grid runs the whole BiCGStab loop of every
+// instance that is not on the block schedule, in seven phases an iteration
+// with a grid barrier after each: update of p and preconditioner, product,
+// (r0, v); update of s and preconditioner, product, (t, t), (t, s), (s, s);
+// update of y and r, (r, r), (r0, r).  The vector updates run in the phase
+// that first reads them, by the thread that owns the cell there.
+//
+// What bounds it up to some 100 k cells is latency: a barrier and a round trip
+// to L2 per phase, the columns of a cluster's triangular solves, the chains of
+// the FP64 sums.  Hence the accumulators of a chunk (256 chains over its
+// cells) are spread warp by warp over the SMs; the warp that comes last in a
+// chunk adds the tree, the last of an instance the chunks and forms the
+// scalars, so that a sum costs one phase; loads go in groups ahead of the
+// stores that the compiler cannot move them past; and the loop leaves with
+// the last instance.  Four Newton iterations' inner solves in
+// FP32, as some twenty kernels an iteration in a graph replayed eight times
+// between looks at the flags, and now: 20,960 prisms with clusters 2.96 ms and
+// 0.60 (8 iterations), 264,000 hexahedra with lines 16.5 and 11.2 (89),
+// 1,122,000 of them 48.5 and 30.5 (78), 192 columns 77.7 and 38.9.
+constexpr int kGridThreads = 512, kGridWarps = kGridThreads / 32;
+enum { GS_BAR = 0, GS_ACTIVE, GS_ERR, GS_COUNT };  // then a counter per chunk and per instance
+constexpr int kGridSums = 3;    // sums of one phase at most
+constexpr int kChainGroup = 4;  // cells of a chain whose loads go ahead of its stores
 
-// out = (cluster block)^-1 in, one warp per cluster: the row swaps, then the
-// unit-lower and upper triangular solves
 template <class T>
-__global__ void __launch_bounds__(32) cl_apply_kernel(int ncl, const int *coff, const long long *luoff,
-                                                      const int *cmem, const T *lu, const int *piv, const T *in,
-                                                      T *out) {
-  __shared__ T x[kClusterMax];
-  const int cl = blockIdx.x, lane = threadIdx.x;
-  if (cl >= ncl) return;
-  const int c0 = coff[cl], sz = coff[cl + 1] - c0;
-  for (int r = lane; r < sz; r += 32) x[r] = in[cmem[c0 + r]];
-  __syncwarp();
-  if (lane == 0)
-    for (int kk = 0; kk < sz; kk++) {
-      const int p = piv[c0 + kk];
-      if (p != kk) {
-        const T t = x[kk];
-        x[kk] = x[p];
-        x[p] = t;
+struct GridSolve {
+  int n, ns, nchunks, nlines, ncl;
+  int clusters;  // preconditioner: clusters, else lines
+  const int *cell_seg, *newt_active, *block_mask;
+  const int *chunk_off, *seg_chunk;
+  const int *rowptr, *colidx;
+  const T *A;
+  const int *line_off, *line_cells;
+  const T *la, *lcp, *linv;
+  const int *cloc, *coff, *cmem, *cperm;
+  const long long *cluoff;
+  const T *cinv, *clu;
+  const double *F;
+  T *r, *r0, *p, *v, *sv, *tv, *ph, *sh, *y;
+  int *act, *its;
+  double *sc;         // [S_NSCAL][ns]
+  double *acc;        // [nchunks][kGridSums][256]
+  double *part;       // [kGridSums][nchunks]
+  unsigned *sync;
+  double tol2;
+  int max_it;
+};
+
+// Every CTA of the launch is past its phase; false if that took longer than
+// seconds (a CTA that gives up flags the error for the others and the host).
+__device__ __forceinline__ bool grid_barrier(unsigned *sync, unsigned &target, int *ok) {
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    target += gridDim.x;
+    __threadfence();
+    atomicAdd(&sync[GS_BAR], 1u);
+    int good = 1;
+    for (unsigned spin = 0;; spin++) {
+      unsigned now;
+      asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(now) : "l"(&sync[GS_BAR]) : "memory");
+      if ((int)(now - target) >= 0) break;
+      if (spin > (1u << 23) || ((spin & 1023u) == 1023u && *(volatile unsigned *)&sync[GS_ERR])) {
+        atomicExch(&sync[GS_ERR], 1u);
+        good = 0;
+        break;
       }
     }
+    *ok = good;
+  }
+  __syncthreads();
+  return *ok != 0;
+}
+
+// whether this warp is the last of `of` to arrive; then it sees what the
+// others wrote, and the counter is zero again
+__device__ __forceinline__ bool last_arrival(unsigned *count, int of, int lane) {
+  if (of == 1) {
+    __syncwarp();
+    return true;
+  }
+  __threadfence();
   __syncwarp();
-  const T *L = lu + luoff[cl];
-  for (int kk = 0; kk < sz; kk++) {
-    const T xk = x[kk];
-    __syncwarp();
-    for (int i = kk + 1 + lane; i < sz; i += 32) x[i] -= L[i * sz + kk] * xk;
-    __syncwarp();
+  unsigned old = 0;
+  if (lane == 0) old = atomicAdd(count, 1u);
+  old = __shfl_sync(0xffffffffu, old, 0);
+  if (old != (unsigned)of - 1) return false;
+  if (lane == 0) *count = 0;
+  __threadfence();
+  return true;
+}
+
+// The accumulators 32 w + lane of chunk ch (of `cells` cells, instance g) are
+// in a.  True in the warp that holds the instance's sums, in every lane: the
+// tree of chunk_dot_kernel (levels 128, 64, 32 across the 8 values of a lane,
+// the others by shuffles), then the chunks in order.
+template <int ND, class T>
+__device__ __forceinline__ bool chunk_sums(const GridSolve<T> &G, int ch, int w, int cells, int g, int lane,
+                                           double (&a)[ND]) {
+  const int parts = min(8, (cells + 31) / 32);
+  double *acc = G.acc + (size_t)ch * kGridSums * 256;
+  if (parts > 1) {
+#pragma unroll
+    for (int d = 0; d < ND; d++) __stcg(&acc[d * 256 + 32 * w + lane], a[d]);
+    if (!last_arrival(&G.sync[GS_COUNT + ch], parts, lane)) return false;
   }
-  for (int kk = sz - 1; kk >= 0; kk--) {
-    if (lane == 0) x[kk] /= L[kk * sz + kk];
-    __syncwarp();
-    const T xk = x[kk];
-    for (int i = lane; i < kk; i += 32) x[i] -= L[i * sz + kk] * xk;
-    __syncwarp();
+  const int c0 = G.seg_chunk[g], nch = G.seg_chunk[g + 1] - c0;
+#pragma unroll
+  for (int d = 0; d < ND; d++) {
+    double x = a[d];
+    if (parts > 1) {
+      double e[8];
+#pragma unroll
+      for (int j = 0; j < 8; j++) e[j] = j < parts ? __ldcg(&acc[d * 256 + 32 * j + lane]) : 0.0;
+#pragma unroll
+      for (int o = 4; o > 0; o >>= 1)
+#pragma unroll
+        for (int j = 0; j < o; j++) e[j] = __dadd_rn(e[j], e[j + o]);
+      x = e[0];
+    }
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) x = __dadd_rn(x, __shfl_down_sync(0xffffffffu, x, o));
+    a[d] = __shfl_sync(0xffffffffu, x, 0);
+    if (nch > 1 && lane == 0) __stcg(&G.part[(size_t)d * G.nchunks + ch], x);
   }
-  for (int r = lane; r < sz; r += 32) out[cmem[c0 + r]] = x[r];
+  if (nch == 1) return true;
+  if (!last_arrival(&G.sync[GS_COUNT + G.nchunks + g], nch, lane)) return false;
+#pragma unroll
+  for (int d = 0; d < ND; d++) a[d] = 0.0;
+  for (int k = 0; k < nch; k += 32) {
+    double x[ND];
+#pragma unroll
+    for (int d = 0; d < ND; d++) x[d] = k + lane < nch ? __ldcg(&G.part[(size_t)d * G.nchunks + c0 + k + lane]) : 0.0;
+    for (int j = 0; j < min(32, nch - k); j++)
+#pragma unroll
+      for (int d = 0; d < ND; d++) a[d] = __dadd_rn(a[d], __shfl_sync(0xffffffffu, x[d], j));
+  }
+  return true;
+}
+
+// y = A x for the rows of the active instances
+template <class T, int TPR>
+__device__ __forceinline__ void grid_spmv(const GridSolve<T> &G, const T *x, T *y) {
+  constexpr int kRows = kGridThreads / TPR;
+  const int lane = threadIdx.x % TPR;
+  for (long long b = (long long)blockIdx.x * kRows; b < G.n; b += (long long)gridDim.x * kRows) {
+    const long long row = b + threadIdx.x / TPR;
+    const bool valid = row < G.n && G.act[G.cell_seg[row]];
+    const T d = row_dot<T, TPR>(valid, valid ? G.rowptr[row] : 0, valid ? G.rowptr[row + 1] : 0, lane, G.colidx, G.A, x);
+    if (valid && lane == 0) y[row] = d;
+  }
+}
+
+// out = M^-1 in for the active instances; in(g) gives the entries of instance
+// g's cells: value(i) reads, keep(i, value) stores what the update of the
+// vector is.  Lines: a thread each, kLineGroup layers' loads ahead of their
+// steps.  Clusters: a warp each, rows lane and lane + 32 in its registers (the
+// rows' order, then the unit-lower and upper triangular solves, whose columns
+// do not wait for the values); the other cells by their diagonal.
+constexpr int kLineGroup = 4;
+
+template <class T, class In>
+__device__ __forceinline__ void grid_precondition(const GridSolve<T> &G, const In &in, T *out) {
+  // neighbouring warps' work on different SMs
+  const int warp = (threadIdx.x / 32) * gridDim.x + blockIdx.x, nwarps = gridDim.x * kGridWarps;
+  const int lane = threadIdx.x % 32;
+  if (!G.clusters) {
+    for (int l = warp * 32 + lane; l < G.nlines; l += nwarps * 32) {
+      const int k0 = G.line_off[l], len = G.line_off[l + 1] - k0;
+      // a column's cells lie one layer apart
+      const int first = G.line_cells[k0], step = len > 1 ? G.line_cells[k0 + 1] - first : 0;
+      const int g = G.cell_seg[first];
+      if (!G.act[g]) continue;
+      const auto f = in(g);
+      T prev = 0;
+      for (int k = 0; k < len; k += kLineGroup) {
+        T a[kLineGroup], d[kLineGroup], x[kLineGroup];
+#pragma unroll
+        for (int j = 0; j < kLineGroup; j++) {
+          const int i = first + min(k + j, len - 1) * step;
+          a[j] = G.la[i];
+          d[j] = G.linv[i];
+          x[j] = f.value(i);
+        }
+#pragma unroll
+        for (int j = 0; j < kLineGroup; j++)
+          if (k + j < len) {
+            const int i = first + (k + j) * step;
+            f.keep(i, x[j]);
+            prev = e_mul(e_fma(-a[j], prev, x[j]), d[j]);
+            out[i] = prev;
+          }
+      }
+      T next = 0;
+      for (int k = len - 1; k >= 0; k -= kLineGroup) {
+        T c[kLineGroup], x[kLineGroup];
+#pragma unroll
+        for (int j = 0; j < kLineGroup; j++) {
+          const int i = first + max(k - j, 0) * step;
+          c[j] = G.lcp[i];
+          x[j] = out[i];
+        }
+#pragma unroll
+        for (int j = 0; j < kLineGroup; j++)
+          if (k - j >= 0) {
+            next = e_fma(-c[j], next, x[j]);
+            out[first + (k - j) * step] = next;
+          }
+      }
+    }
+    return;
+  }
+  for (int cl = warp; cl < G.ncl; cl += nwarps) {
+    const int c0 = G.coff[cl], sz = G.coff[cl + 1] - c0;
+    const int g = G.cell_seg[G.cmem[c0]];
+    if (!G.act[g]) continue;
+    const auto f = in(g);
+    const bool on0 = lane < sz, on1 = lane + 32 < sz;
+    const int m0 = on0 ? G.cmem[c0 + lane] : 0, m1 = on1 ? G.cmem[c0 + lane + 32] : 0;
+    const int s0 = on0 ? G.cperm[c0 + lane] : 0, s1 = on1 ? G.cperm[c0 + lane + 32] : 0;
+    const T v0 = on0 ? f.value(m0) : (T)0, v1 = on1 ? f.value(m1) : (T)0;
+    if (on0) f.keep(m0, v0);
+    if (on1) f.keep(m1, v1);
+    auto from = [&](int r) {  // row r's value (r differs by lane)
+      const T a = __shfl_sync(0xffffffffu, v0, r & 31), b = __shfl_sync(0xffffffffu, v1, r & 31);
+      return r < 32 ? a : b;
+    };
+    T x0 = from(s0), x1 = from(s1);
+    const T *L = G.clu + G.cluoff[cl];
+#pragma unroll 4
+    for (int k = 0; k < sz; k++) {
+      const T l0 = on0 ? L[k * sz + lane] : (T)0, l1 = on1 ? L[k * sz + lane + 32] : (T)0;
+      const T xk = __shfl_sync(0xffffffffu, k < 32 ? x0 : x1, k & 31);
+      if (lane > k) x0 -= l0 * xk;
+      if (lane + 32 > k) x1 -= l1 * xk;
+    }
+#pragma unroll 4
+    for (int k = sz - 1; k >= 0; k--) {
+      const T l0 = on0 ? L[k * sz + lane] : (T)0, l1 = on1 ? L[k * sz + lane + 32] : (T)0;
+      const T xk = __shfl_sync(0xffffffffu, k < 32 ? x0 : x1, k & 31) / L[k * sz + k];
+      x0 = lane == k ? xk : lane < k ? x0 - l0 * xk : x0;
+      x1 = lane + 32 == k ? xk : lane + 32 < k ? x1 - l1 * xk : x1;
+    }
+    if (on0) out[m0] = x0;
+    if (on1) out[m1] = x1;
+  }
+  for (int i = blockIdx.x * kGridThreads + threadIdx.x; i < G.n; i += gridDim.x * kGridThreads) {
+    if (G.cloc[i] >= 0) continue;
+    const int g = G.cell_seg[i];
+    if (!G.act[g]) continue;
+    const auto f = in(g);
+    const T x = f.value(i);
+    f.keep(i, x);
+    out[i] = G.cinv[i] * x;
+  }
+}
+
+// p = r + beta (p - omega v)
+template <class T>
+struct UpdateP {
+  const GridSolve<T> &G;
+  T beta, omega;
+  __device__ T value(int i) const { return op_p(G.r[i], G.p[i], G.v[i], beta, omega); }
+  __device__ void keep(int i, T p) const { G.p[i] = p; }
+};
+// s = r - alpha v
+template <class T>
+struct UpdateS {
+  const GridSolve<T> &G;
+  T alpha;
+  __device__ T value(int i) const { return e_fma(-alpha, G.v[i], G.r[i]); }
+  __device__ void keep(int i, T s) const { G.sv[i] = s; }
+};
+
+// f(ch, w, i0, i1, g) for the accumulators 32 w .. 32 w + 31 of every chunk
+template <class T, class Fn>
+__device__ __forceinline__ void grid_chunks(const GridSolve<T> &G, const Fn &f) {
+  for (int e = (threadIdx.x / 32) * gridDim.x + blockIdx.x; e < 8 * G.nchunks; e += gridDim.x * kGridWarps) {
+    const int ch = e / 8, w = e % 8;
+    const int i0 = G.chunk_off[ch], i1 = G.chunk_off[ch + 1];
+    if (i0 + 32 * w < i1) f(ch, w, i0, i1, G.cell_seg[i0]);
+  }
+}
+
+template <class T, int TPR>
+__global__ void __launch_bounds__(kGridThreads, sizeof(T) == 4 ? 2 : 1) bicgstab_grid_kernel(const GridSolve<T> G) {
+  __shared__ int ok;
+  const int lane = threadIdx.x % 32, ns = G.ns;
+  unsigned target = 0;
+  auto S = [&](int slot, int g) -> double & { return G.sc[(size_t)slot * ns + g]; };
+  auto retire = [&](int g) {
+    G.act[g] = 0;
+    atomicSub(&G.sync[GS_ACTIVE], 1u);
+  };
+  // rho = (r0, r) and the next beta
+  auto beta = [&](int g, double rn, double rho, double alpha, double omega) {
+    if (rn == 0.0) {
+      retire(g);
+      return;
+    }
+    S(S_BETA, g) = (rn / rho) * (alpha / omega);
+    S(S_RHO, g) = rn;
+  };
+  // r = r0 = F, and ||F||^2
+  grid_chunks(G, [&](int ch, int w, int i0, int i1, int g) {
+    const bool on = G.newt_active[g];
+    const bool mine = !G.block_mask[g];
+    if (!on || !mine) {
+      if (lane == 0 && w == 0 && ch == G.seg_chunk[g]) G.act[g] = 0;
+      if (mine)
+        for (int i = i0 + 32 * w + lane; i < i1; i += 256) G.y[i] = 0;
+      return;
+    }
+    double a[1] = {0.0};
+    for (int i = i0 + 32 * w + lane; i < i1; i += 256) {
+      const T f = (T)G.F[i];
+      G.r[i] = f;
+      G.r0[i] = f;
+      G.p[i] = 0;
+      G.v[i] = 0;
+      G.y[i] = 0;
+      a[0] = op_dot(a[0], f, f);
+    }
+    if (chunk_sums(G, ch, w, i1 - i0, g, lane, a) && lane == 0) {
+      S(S_BNORM2, g) = a[0];
+      S(S_OMEGA, g) = S(S_ALPHA, g) = 1.0;
+      const bool solve = a[0] > 0.0;
+      G.act[g] = solve;
+      if (solve) {
+        atomicAdd(&G.sync[GS_ACTIVE], 1u);
+        beta(g, a[0], 1.0, 1.0, 1.0);
+      }
+    }
+  });
+  if (!grid_barrier(G.sync, target, &ok)) return;
+  for (int it = 0; it < G.max_it && __ldcg(&G.sync[GS_ACTIVE]) != 0; it++) {
+    grid_precondition(
+        G, [&](int g) { return UpdateP<T>{G, (T)S(S_BETA, g), (T)S(S_OMEGA, g)}; }, G.ph);
+    if (!grid_barrier(G.sync, target, &ok)) return;
+    grid_spmv<T, TPR>(G, G.ph, G.v);
+    if (!grid_barrier(G.sync, target, &ok)) return;
+    grid_chunks(G, [&](int ch, int w, int i0, int i1, int g) {
+      if (!G.act[g]) return;
+      double a[1] = {0.0};
+#pragma unroll 8
+      for (int i = i0 + 32 * w + lane; i < i1; i += 256) a[0] = op_dot(a[0], G.r0[i], G.v[i]);
+      if (chunk_sums(G, ch, w, i1 - i0, g, lane, a) && lane == 0) {
+        if (a[0] == 0.0)
+          retire(g);
+        else
+          S(S_ALPHA, g) = S(S_RHO, g) / a[0];
+      }
+    });
+    if (!grid_barrier(G.sync, target, &ok)) return;
+    grid_precondition(
+        G, [&](int g) { return UpdateS<T>{G, (T)S(S_ALPHA, g)}; }, G.sh);
+    if (!grid_barrier(G.sync, target, &ok)) return;
+    grid_spmv<T, TPR>(G, G.sh, G.tv);
+    if (!grid_barrier(G.sync, target, &ok)) return;
+    grid_chunks(G, [&](int ch, int w, int i0, int i1, int g) {
+      if (!G.act[g]) return;
+      double a[3] = {0.0, 0.0, 0.0};
+#pragma unroll 8
+      for (int i = i0 + 32 * w + lane; i < i1; i += 256) {
+        const T t = G.tv[i], s = G.sv[i];
+        a[0] = op_dot(a[0], t, t);
+        a[1] = op_dot(a[1], t, s);
+        a[2] = op_dot(a[2], s, s);
+      }
+      if (chunk_sums(G, ch, w, i1 - i0, g, lane, a) && lane == 0) {
+        S(S_OMEGA, g) = a[0] > 0.0 ? a[1] / a[0] : 0.0;
+        S(S_HALF, g) = a[2] <= G.tol2 * S(S_BNORM2, g) ? 1.0 : 0.0;  // converged at the half step
+      }
+    });
+    if (!grid_barrier(G.sync, target, &ok)) return;
+    grid_chunks(G, [&](int ch, int w, int i0, int i1, int g) {
+      if (!G.act[g]) return;
+      const T alpha = (T)S(S_ALPHA, g), omega = (T)S(S_OMEGA, g);
+      const bool half = S(S_HALF, g) != 0.0;
+      double a[2] = {0.0, 0.0};
+      // kChainGroup cells' loads ahead of their stores
+      for (int b = i0 + 32 * w + lane; b < i1; b += 256 * kChainGroup) {
+        T y[kChainGroup], ph[kChainGroup], sh[kChainGroup], t[kChainGroup], sv[kChainGroup], r0[kChainGroup];
+#pragma unroll
+        for (int j = 0; j < kChainGroup; j++) {
+          const int i = min(b + 256 * j, i1 - 1);
+          y[j] = G.y[i];
+          ph[j] = G.ph[i];
+          sh[j] = G.sh[i];
+          t[j] = G.tv[i];
+          sv[j] = G.sv[i];
+          r0[j] = G.r0[i];
+        }
+#pragma unroll
+        for (int j = 0; j < kChainGroup; j++) {
+          const int i = b + 256 * j;
+          if (i >= i1) break;
+          if (half) {
+            G.y[i] = op_y(y[j], ph[j], alpha);
+          } else {
+            G.y[i] = op_y2(y[j], ph[j], sh[j], alpha, omega);
+            const T r = e_fma(-omega, t[j], sv[j]);
+            G.r[i] = r;
+            a[0] = op_dot(a[0], r, r);
+            a[1] = op_dot(a[1], r0[j], r);
+          }
+        }
+      }
+      if (chunk_sums(G, ch, w, i1 - i0, g, lane, a) && lane == 0) {
+        G.its[g] += 1;
+        const double om = S(S_OMEGA, g);
+        if (half || a[0] <= G.tol2 * S(S_BNORM2, g) || om == 0.0)
+          retire(g);
+        else
+          beta(g, a[1], S(S_RHO, g), S(S_ALPHA, g), om);
+      }
+    });
+    if (!grid_barrier(G.sync, target, &ok)) return;
+  }
 }
 
 // ---------------------------------------------------------------------------
 template <class T>
-int spmv(SolverState *s, const Krylov &k, const T *x, T *y, Emit &e) {
+void spmv(SolverState *s, const Krylov &k, const T *x, T *y, cudaStream_t st) {
   const T *A = (const T *)k.Jv;
   const unsigned g = nblk((long long)s->n * k.tpr, 256);
   switch (k.tpr) {
-    case 1:
-      e(spmv_kernel<T, 1>, g, 256, 0, s->n, (const int *)s->rowptr, (const int *)s->colidx, A, x, y);
-      break;
-    case 2:
-      e(spmv_kernel<T, 2>, g, 256, 0, s->n, (const int *)s->rowptr, (const int *)s->colidx, A, x, y);
-      break;
-    case 4:
-      e(spmv_kernel<T, 4>, g, 256, 0, s->n, (const int *)s->rowptr, (const int *)s->colidx, A, x, y);
-      break;
-    default:
-      e(spmv_kernel<T, 8>, g, 256, 0, s->n, (const int *)s->rowptr, (const int *)s->colidx, A, x, y);
-      break;
-  }
-  return 0;
-}
-
-template <class TA, class TB>
-void seg_dot(SolverState *s, const TA *a, const TB *b, const TA *c, const TB *d, double *out, double *out2, Emit &e) {
-  e(chunk_dot_kernel<TA, TB>, (unsigned)s->nchunks, 256, 0, (const int *)s->chunk_off, a, b, c, d, s->part,
-    s->part2);
-  e(chunk_sum_kernel, nblk(s->nseg, 128), 128, 0, s->nseg, (const int *)s->seg_chunk, (const double *)s->part,
-    (const double *)s->part2, out, c ? out2 : (double *)nullptr);
-}
-template <class TA, class TB>
-void seg_dot(SolverState *s, const TA *a, const TB *b, const TA *c, const TB *d, double *out, double *out2,
-             cudaStream_t st) {
-  Emit e(st);
-  seg_dot<TA, TB>(s, a, b, c, d, out, out2, e);
-}
-
-template <class T>
-int dot(SolverState *s, const T *a, const T *b, const T *c, const T *d, int slot1, int slot2, Emit &e) {
-  seg_dot<T, T>(s, a, b, c, d, s->scal + (size_t)slot1 * s->nseg, c ? s->scal + (size_t)slot2 * s->nseg : nullptr, e);
-  return 0;
-}
-
-// out = M^-1 in with the preconditioner of the current solve
-template <class T>
-void precondition(SolverState *s, Krylov &k, const T *in, T *out, Emit &e) {
-  if (s->precond_used == TDY_PRECOND_CLUSTERS) {
-    e(cl_apply_diag_kernel<T>, nblk(s->n, 256), 256, 0, s->n, (const int *)s->cloc, (const T *)k.cinv, in, out);
-    e(cl_apply_kernel<T>, (unsigned)s->ncl, 32, 0, s->ncl, (const int *)s->coff, (const long long *)s->cluoff,
-      (const int *)s->cmem, (const T *)k.clu, (const int *)s->cpiv, in, out);
-  } else {
-    e(line_solve_kernel<T>, nblk(s->nlines, 128), 128, 0, s->nlines, (const int *)s->line_off,
-      (const int *)s->line_cells, (const T *)k.la, (const T *)k.lcp, (const T *)k.linv, in, out);
+    case 1: spmv_kernel<T, 1><<<g, 256, 0, st>>>(s->n, s->rowptr, s->colidx, A, x, y); break;
+    case 2: spmv_kernel<T, 2><<<g, 256, 0, st>>>(s->n, s->rowptr, s->colidx, A, x, y); break;
+    case 4: spmv_kernel<T, 4><<<g, 256, 0, st>>>(s->n, s->rowptr, s->colidx, A, x, y); break;
+    default: spmv_kernel<T, 8><<<g, 256, 0, st>>>(s->n, s->rowptr, s->colidx, A, x, y);
   }
 }
 
-// one BiCGStab iteration for every active instance (the graph body)
-template <class T>
-void bicgstab_iteration(SolverState *s, Krylov &k, double tol2, Emit &e) {
-  const int n = s->n, ns = s->nseg;
-  const unsigned gb = nblk(n, 256), sb = nblk(ns, 128);
-  T *r = (T *)k.r, *r0 = (T *)k.r0, *p = (T *)k.p, *v = (T *)k.v, *sv = (T *)k.s, *tv = (T *)k.t;
-  T *ph = (T *)k.ph, *sh = (T *)k.sh, *y = (T *)k.y;
-  const int *cs = s->cell_seg;
-  int *act = s->lin_active;
-  const int *cact = s->lin_active;
-  double *sc = s->scal;
-  const double *csc = s->scal;
-  dot<T>(s, r0, r, nullptr, nullptr, S_T1, 0, e);
-  e(scal_beta_kernel, sb, 128, 0, ns, act, sc);
-  e(p_update_kernel<T>, gb, 256, 0, n, cs, cact, csc, ns, (const T *)r, (const T *)v, p);
-  precondition<T>(s, k, p, ph, e);
-  spmv<T>(s, k, ph, v, e);
-  dot<T>(s, r0, v, nullptr, nullptr, S_T1, 0, e);
-  e(scal_alpha_kernel, sb, 128, 0, ns, act, sc);
-  e(s_update_kernel<T>, gb, 256, 0, n, cs, cact, csc, ns, (const T *)r, (const T *)v, sv);
-  dot<T>(s, sv, sv, nullptr, nullptr, S_T1, 0, e);
-  e(scal_half_kernel, sb, 128, 0, ns, cact, sc, tol2);
-  precondition<T>(s, k, sv, sh, e);
-  spmv<T>(s, k, sh, tv, e);
-  dot<T>(s, tv, tv, tv, sv, S_T1, S_T2, e);
-  e(scal_omega_kernel, sb, 128, 0, ns, cact, sc);
-  e(xr_update_kernel<T>, gb, 256, 0, n, cs, cact, csc, ns, (const T *)ph, (const T *)sh, (const T *)sv,
-    (const T *)tv, y, r);
-  dot<T>(s, r, r, nullptr, nullptr, S_T1, 0, e);
-  e(scal_check_kernel, sb, 128, 0, ns, act, s->lin_its, sc, tol2);
+template <class TA, class TB>
+void seg_dot(SolverState *s, const TA *a, const TB *b, double *out, cudaStream_t st) {
+  chunk_dot_kernel<TA, TB><<<s->nchunks, 256, 0, st>>>(s->chunk_off, a, b, s->part);
+  chunk_sum_kernel<<<nblk(s->nseg, 128), 128, 0, st>>>(s->nseg, s->seg_chunk, s->part, out);
 }
 
 // (one allocation for every vector; ordered on the solve's stream, which uses
@@ -1349,12 +1511,11 @@ int autotune_spmv(SolverState *s, Krylov &k, int forced, cudaStream_t st) {
   SCUDA(cudaEventCreate(&e1));
   float best = 1e30f;
   int best_tpr = 1;
-  Emit em(st);
   for (int tpr : {1, 2, 4, 8}) {
     k.tpr = tpr;
-    spmv<T>(s, k, (const T *)k.b, (T *)k.v, em);  // warm-up
+    spmv<T>(s, k, (const T *)k.b, (T *)k.v, st);  // warm-up
     cudaEventRecord(e0, st);
-    for (int it = 0; it < 5; it++) spmv<T>(s, k, (const T *)k.b, (T *)k.v, em);
+    for (int it = 0; it < 5; it++) spmv<T>(s, k, (const T *)k.b, (T *)k.v, st);
     cudaEventRecord(e1, st);
     SCUDA(cudaEventSynchronize(e1));
     float ms = 0.f;
@@ -1388,7 +1549,7 @@ int cluster_setup(SolverState *s, Krylov &k, double tau, cudaStream_t st) {
     if ((ierr = salloc(s, &s->cmem, n))) return ierr;
     if ((ierr = salloc(s, &s->coff, n + 1))) return ierr;
     if ((ierr = salloc(s, &s->cluoff, n + 1))) return ierr;
-    if ((ierr = salloc(s, &s->cpiv, n))) return ierr;
+    if ((ierr = salloc(s, &s->cperm, n))) return ierr;
   }
   if (!k.cinv) {
     T *p;
@@ -1464,7 +1625,7 @@ int cluster_setup(SolverState *s, Krylov &k, double tau, cudaStream_t st) {
   cl_diag_kernel<T><<<nblk(n, 256), 256, 0, st>>>(n, s->cloc, s->dpos, s->J, (T *)k.cinv);
   if (ncl > 0)
     cl_factor_kernel<T><<<ncl, 32, kClusterMax * kClusterLd * sizeof(T), st>>>(
-        ncl, s->coff, s->cluoff, s->cmem, s->cloc, s->clab, s->rowptr, s->colidx, s->J, (T *)k.clu, s->cpiv);
+        ncl, s->coff, s->cluoff, s->cmem, s->cloc, s->clab, s->rowptr, s->colidx, s->J, (T *)k.clu, s->cperm);
   SCUDA(cudaGetLastError());
   // the host vectors above stay alive until the copies complete
   SCUDA(cudaStreamSynchronize(st));
@@ -1696,41 +1857,115 @@ int launch_block(SolverState *s, Krylov &k, const TDyNewtonOptions &o, double to
   return 0;
 }
 
+// The active instances of the tile schedule.  As many CTAs as the product has
+// rows for, up to what the GPU holds at once: a cooperative launch, whose CTAs
+// are all resident, so that its barriers end.
+template <class T, int TPR>
+int launch_grid_tpr(const GridSolve<T> &G, int nsm, cudaStream_t st) {
+  auto kern = bicgstab_grid_kernel<T, TPR>;
+  int per_sm = 0;
+  SCUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, kGridThreads, 0));
+  const long long want = ((long long)G.n * TPR + kGridThreads - 1) / kGridThreads;
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3((unsigned)std::max(1LL, std::min(want, (long long)nsm * per_sm)));
+  cfg.blockDim = dim3(kGridThreads);
+  cfg.stream = st;
+  cudaLaunchAttribute at[1];
+  at[0].id = cudaLaunchAttributeCooperative;
+  at[0].val.cooperative = 1;
+  cfg.attrs = at;
+  cfg.numAttrs = 1;
+  SCUDA(cudaLaunchKernelEx(&cfg, kern, G));
+  return 0;
+}
+
+template <class T>
+int launch_grid(SolverState *s, Krylov &k, const TDyNewtonOptions &o, double tol2, cudaStream_t st) {
+  int ierr, dev = 0, nsm = 0;
+  SCUDA(cudaGetDevice(&dev));
+  SCUDA(cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev));
+  const size_t nsync = GS_COUNT + (size_t)s->nchunks + s->nseg;
+  if (!s->grid_sync) {
+    Arena ar;
+    ar.work(&s->grid_acc, (size_t)s->nchunks * kGridSums * 256);
+    ar.work(&s->grid_part, (size_t)s->nchunks * kGridSums);
+    ar.work(&s->grid_sync, nsync);
+    if ((ierr = ar.commit(st))) return ierr;
+    s->allocs.push_back(ar.base);
+  }
+  SCUDA(cudaMemsetAsync(s->grid_sync, 0, nsync * sizeof(unsigned), st));
+  GridSolve<T> G;
+  G.n = s->n;
+  G.ns = s->nseg;
+  G.nchunks = s->nchunks;
+  G.nlines = s->nlines;
+  G.clusters = s->precond_used == TDY_PRECOND_CLUSTERS;
+  G.ncl = G.clusters ? s->ncl : 0;
+  G.cell_seg = s->cell_seg;
+  G.newt_active = s->newt_active;
+  G.block_mask = s->block_mask;
+  G.chunk_off = s->chunk_off;
+  G.seg_chunk = s->seg_chunk;
+  G.rowptr = s->rowptr;
+  G.colidx = s->colidx;
+  G.A = (const T *)k.Jv;
+  G.line_off = s->line_off;
+  G.line_cells = s->line_cells;
+  G.la = (const T *)k.la;
+  G.lcp = (const T *)k.lcp;
+  G.linv = (const T *)k.linv;
+  G.cloc = s->cloc;
+  G.coff = s->coff;
+  G.cmem = s->cmem;
+  G.cperm = s->cperm;
+  G.cluoff = s->cluoff;
+  G.cinv = (const T *)k.cinv;
+  G.clu = (const T *)k.clu;
+  G.F = s->F;
+  G.r = (T *)k.r;
+  G.r0 = (T *)k.r0;
+  G.p = (T *)k.p;
+  G.v = (T *)k.v;
+  G.sv = (T *)k.s;
+  G.tv = (T *)k.t;
+  G.ph = (T *)k.ph;
+  G.sh = (T *)k.sh;
+  G.y = (T *)k.y;
+  G.act = s->lin_active;
+  G.its = s->lin_its;
+  G.sc = s->scal;
+  G.acc = s->grid_acc;
+  G.part = s->grid_part;
+  G.sync = s->grid_sync;
+  G.tol2 = tol2;
+  G.max_it = o.linear_max_it;
+  switch (k.tpr) {
+    case 1: return launch_grid_tpr<T, 1>(G, nsm, st);
+    case 2: return launch_grid_tpr<T, 2>(G, nsm, st);
+    case 4: return launch_grid_tpr<T, 4>(G, nsm, st);
+    default: return launch_grid_tpr<T, 8>(G, nsm, st);
+  }
+}
+
 // One linear solve with instances of at most `thr` cells on the block
 // schedule and the others on the tile schedule; its = inner iterations.
 template <class T>
 int solve_scheduled(SolverState *s, Krylov &k, const TDyNewtonOptions &o, double tol2, long long thr,
                     const std::vector<int> &newt_act, cudaStream_t st, std::vector<int> &its) {
   int ierr;
-  const int n = s->n, ns = s->nseg;
+  const int ns = s->nseg;
   if ((ierr = set_block_split(s, thr, st))) return ierr;
   SCUDA(cudaMemsetAsync(s->lin_its, 0, sizeof(int) * ns, st));
-  if (s->n_tile > 0) {
-    init_kernel<T><<<nblk(n, 256), 256, 0, st>>>(n, s->cell_seg, s->newt_active, s->F, (T *)k.b, (T *)k.r, (T *)k.r0,
-                                                 (T *)k.p, (T *)k.v, (T *)k.y);
-    SCUDA(cudaGetLastError());
-  }
   if (s->n_block > 0 && (ierr = launch_block<T>(s, k, o, tol2, thr, newt_act, st))) return ierr;
+  unsigned err = 0;
   if (s->n_tile > 0) {
-    Emit em(st);
-    dot<T>(s, (T *)k.b, (T *)k.b, nullptr, nullptr, S_BNORM2, 0, em);
-    init_scalars_kernel<<<nblk(ns, 128), 128, 0, st>>>(ns, s->newt_active, s->block_mask, s->lin_active, s->lin_its,
-                                                       s->scal);
-    SCUDA(cudaGetLastError());
-    std::vector<int> act(ns);
-    const int check_every = 8;
-    for (int it = 0; it < o.linear_max_it; it += check_every) {
-      for (int j = 0; j < check_every && it + j < o.linear_max_it; j++) SCUDA(cudaGraphLaunch(k.graph, st));
-      SCUDA(cudaMemcpyAsync(act.data(), s->lin_active, sizeof(int) * ns, cudaMemcpyDeviceToHost, st));
-      SCUDA(cudaStreamSynchronize(st));
-      bool any = false;
-      for (int a : act) any |= (a != 0);
-      if (!any) break;
-    }
+    if ((ierr = launch_grid<T>(s, k, o, tol2, st))) return ierr;
+    SCUDA(cudaMemcpyAsync(&err, s->grid_sync + GS_ERR, sizeof(err), cudaMemcpyDeviceToHost, st));
   }
   its.resize(ns);
   SCUDA(cudaMemcpyAsync(its.data(), s->lin_its, sizeof(int) * ns, cudaMemcpyDeviceToHost, st));
   SCUDA(cudaStreamSynchronize(st));
+  if (err) return set_error(TDY_ERR_GPU, "solver: a wait of the tile schedule ran out");
   return 0;
 }
 
@@ -1802,38 +2037,6 @@ int tune_schedule(SolverState *s, Krylov &k, const TDyNewtonOptions &o, double t
   return 0;
 }
 
-// What the tile schedule needs for the current Jacobian: the CSR copy of its
-// values in the inner precision, the threads per row of its products and the
-// graph of one iteration.  The graph is built with the explicit graph API, not
-// by stream capture: a capture is invalidated by device-wide operations that
-// other threads issue meanwhile (a cudaFree, a device synchronisation), which
-// a server running many handles at once cannot rule out.  The cluster launches
-// depend on this solve's cluster count: rebuild for every solve.
-template <class T>
-int tile_setup(SolverState *s, Krylov &k, const TDyNewtonOptions &o, double tol2, cudaStream_t st) {
-  if ((!k.graph || s->linear_rtol != o.linear_rtol || k.graph_precond != s->precond_used || k.graph_tpr != k.tpr ||
-       s->precond_used == TDY_PRECOND_CLUSTERS)) {
-    if (k.graph) cudaGraphExecDestroy(k.graph);
-    k.graph = nullptr;
-    cudaGraph_t g = nullptr;
-    SCUDA(cudaGraphCreate(&g, 0));
-    Emit em(st);
-    em.g = g;
-    bicgstab_iteration<T>(s, k, tol2, em);
-    cudaError_t e = em.err;
-    if (e == cudaSuccess) e = cudaGraphInstantiate(&k.graph, g, 0);
-    cudaGraphDestroy(g);
-    if (e != cudaSuccess) {
-      k.graph = nullptr;
-      return set_error(TDY_ERR_GPU, "BiCGStab iteration graph: %s", cudaGetErrorString(e));
-    }
-    k.graph_precond = s->precond_used;
-    k.graph_tpr = k.tpr;
-    s->linear_rtol = o.linear_rtol;
-  }
-  return 0;
-}
-
 // act: the instances to solve (the host's copy of newt_active)
 template <class T>
 int linear_solve(SolverState *s, Krylov &k, const TDyNewtonOptions &o, const std::vector<int> &act, cudaStream_t st,
@@ -1882,7 +2085,6 @@ int linear_solve(SolverState *s, Krylov &k, const TDyNewtonOptions &o, const std
                                                                  (T *)k.linv);
   SCUDA(cudaEventRecord(s->tev[3], st));
   const double tol2 = o.linear_rtol * o.linear_rtol;
-  if (tile && (ierr = tile_setup<T>(s, k, o, tol2, st))) return ierr;
   std::vector<int> its(ns);
   if (tune && (ierr = tune_schedule<T>(s, k, o, tol2, act, st, &thr))) return ierr;
   if ((ierr = solve_scheduled<T>(s, k, o, tol2, thr, act, st, its))) return ierr;
@@ -1970,7 +2172,6 @@ int solver_init(_p_TDy *t) {
   ar.up(&s->chunk_off, chunk_off);
   ar.up(&s->seg_chunk, seg_chunk);
   ar.work(&s->part, s->nchunks);
-  ar.work(&s->part2, s->nchunks);
   ar.up(&s->cell_seg, cell_seg);
   ar.up(&s->line_off, line_off);
   ar.up(&s->line_cells, line_cells);
@@ -2067,7 +2268,7 @@ int device_be_solve(_p_TDy *t, double dt, double *dU, const TDyNewtonOptions &o,
       e = device_eval(t, FORM_SNES, 0.0, s->x, nullptr, 0.0, s->F, s->J, st, true);
     if (e) return e;
     SCUDA(cudaEventRecord(s->tev[1], st));
-    seg_dot<double, double>(s, s->F, s->F, nullptr, nullptr, s->fn2, nullptr, st);
+    seg_dot<double, double>(s, s->F, s->F, s->fn2, st);
     SCUDA(cudaGetLastError());
     SCUDA(cudaMemcpyAsync(g2.data(), s->fn2, sizeof(double) * ns, cudaMemcpyDeviceToHost, st));
     SCUDA(cudaStreamSynchronize(st));
@@ -2148,13 +2349,13 @@ int device_be_solve(_p_TDy *t, double dt, double *dU, const TDyNewtonOptions &o,
     // full step fails and ||y|| < stol ||x||
     {
       if (fp32)
-        seg_dot<float, float>(s, (const float *)y, (const float *)y, nullptr, nullptr, s->fn2, nullptr, st);
+        seg_dot<float, float>(s, (const float *)y, (const float *)y, s->fn2, st);
       else
-        seg_dot<double, double>(s, (const double *)y, (const double *)y, nullptr, nullptr, s->fn2, nullptr, st);
-      seg_dot<double, double>(s, s->xb, s->xb, nullptr, nullptr, s->scal + (size_t)S_T2 * ns, nullptr, st);
+        seg_dot<double, double>(s, (const double *)y, (const double *)y, s->fn2, st);
+      seg_dot<double, double>(s, s->xb, s->xb, s->scal + (size_t)S_XNORM2 * ns, st);
       SCUDA(cudaGetLastError());
       SCUDA(cudaMemcpyAsync(y2.data(), s->fn2, sizeof(double) * ns, cudaMemcpyDeviceToHost, st));
-      SCUDA(cudaMemcpyAsync(x2.data(), s->scal + (size_t)S_T2 * ns, sizeof(double) * ns, cudaMemcpyDeviceToHost, st));
+      SCUDA(cudaMemcpyAsync(x2.data(), s->scal + (size_t)S_XNORM2 * ns, sizeof(double) * ns, cudaMemcpyDeviceToHost, st));
       SCUDA(cudaStreamSynchronize(st));
     }
     // backtracking per instance: accept when ||F(x - lam y)||^2 <= (1 - 2 alpha lam) ||F(x)||^2
@@ -2228,13 +2429,13 @@ int device_be_solve(_p_TDy *t, double dt, double *dU, const TDyNewtonOptions &o,
     // line search does not count as convergence.
     if (o.stol > 0.0) {
       if (fp32)
-        seg_dot<float, float>(s, (const float *)y, (const float *)y, nullptr, nullptr, s->fn2, nullptr, st);
+        seg_dot<float, float>(s, (const float *)y, (const float *)y, s->fn2, st);
       else
-        seg_dot<double, double>(s, (const double *)y, (const double *)y, nullptr, nullptr, s->fn2, nullptr, st);
-      seg_dot<double, double>(s, s->xb, s->xb, nullptr, nullptr, s->scal + (size_t)S_T2 * ns, nullptr, st);
+        seg_dot<double, double>(s, (const double *)y, (const double *)y, s->fn2, st);
+      seg_dot<double, double>(s, s->xb, s->xb, s->scal + (size_t)S_XNORM2 * ns, st);
       SCUDA(cudaGetLastError());
       SCUDA(cudaMemcpyAsync(y2.data(), s->fn2, sizeof(double) * ns, cudaMemcpyDeviceToHost, st));
-      SCUDA(cudaMemcpyAsync(x2.data(), s->scal + (size_t)S_T2 * ns, sizeof(double) * ns, cudaMemcpyDeviceToHost, st));
+      SCUDA(cudaMemcpyAsync(x2.data(), s->scal + (size_t)S_XNORM2 * ns, sizeof(double) * ns, cudaMemcpyDeviceToHost, st));
       SCUDA(cudaStreamSynchronize(st));
       for (int g = 0; g < ns; g++)
         if (act[g] && std::sqrt(y2[g]) < o.stol * std::sqrt(x2[g])) {
