@@ -52,6 +52,14 @@ inline unsigned nblk(long long n, int bs) { return (unsigned)((n + bs - 1) / bs)
 // per-instance scalars, [slot][nseg]
 enum { S_RHO = 0, S_ALPHA, S_OMEGA, S_BETA, S_BNORM2, S_XNORM2, S_HALF, S_NSCAL };
 
+// what the host reads of a set-up of clusters
+struct ClusterCounts {
+  unsigned long long both;  // clusters of 2..64 cells << 32 | cells in them
+  unsigned long long lu;    // elements of their factors
+  unsigned long long big;   // cells of larger clusters
+  int settled;              // 0: the labels still changed in the last round
+};
+
 struct Krylov {
   bool ready = false;
   void *Jv = nullptr;                                  // matrix values (T)
@@ -83,16 +91,20 @@ struct SolverState {
   unsigned *grid_sync = nullptr;
   int *dpos = nullptr;  // position of each row's diagonal in the CSR values
   // strong-coupling clusters, rebuilt for every linear solve that uses them:
-  // label per cell, a change flag, local index in its cluster (-1: the cell
+  // scratch of the set-up (cl_setup_kernel), label per cell, local index in
+  // its cluster (-1: the cell
   // takes its diagonal), the members of the 2..64-cell clusters (cluster by
   // cluster, ascending cell index), their offsets and LU offsets, row orders
-  int *clab = nullptr, *cflag = nullptr, *cloc = nullptr, *cmem = nullptr, *coff = nullptr, *cperm = nullptr;
+  unsigned char *cstrong = nullptr;
+  int *ccnt = nullptr, *cid = nullptr;
+  unsigned long long *ctotal = nullptr;
+  unsigned *csync = nullptr;
+  ClusterCounts *ccounts = nullptr;
+  int *clab = nullptr, *cloc = nullptr, *cmem = nullptr, *coff = nullptr, *cperm = nullptr;
   long long *cluoff = nullptr;
   int ncl = 0;  // clusters of 2..64 cells in the current solve
   int ncl_cells = 0, ncl_big_cells = 0;  // cells in them; cells of clusters over 64 cells
   int precond_used = 0;
-  std::vector<int> h_lab, h_cnt, h_id, h_fill, h_loc, h_mem, h_off;
-  std::vector<long long> h_luoff;
   Krylov k32, k64;
   // schedules of the line-preconditioned inner solve (block: a cluster per
   // instance; tile: one grid for all cells): instances with at most
@@ -910,80 +922,260 @@ __global__ void commit_kernel(int n, const int *cs, const int *commit, const dou
 }
 
 // ---------------------------------------------------------------------------
+// Cooperative grids: words of their state (zeroed before the launch), then
+// what each kernel counts in it.
+enum { GS_BAR = 0, GS_ACTIVE, GS_ERR, GS_COUNT };
+
+// Every CTA of the launch is past its phase; false if that took longer than
+// seconds (a CTA that gives up flags the error for the others and the host).
+__device__ __forceinline__ bool grid_barrier(unsigned *sync, unsigned &target, int *ok) {
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    target += gridDim.x;
+    __threadfence();
+    atomicAdd(&sync[GS_BAR], 1u);
+    int good = 1;
+    for (unsigned spin = 0;; spin++) {
+      unsigned now;
+      asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(now) : "l"(&sync[GS_BAR]) : "memory");
+      if ((int)(now - target) >= 0) break;
+      if (spin > (1u << 23) || ((spin & 1023u) == 1023u && *(volatile unsigned *)&sync[GS_ERR])) {
+        atomicExch(&sync[GS_ERR], 1u);
+        good = 0;
+        break;
+      }
+    }
+    *ok = good;
+  }
+  __syncthreads();
+  return *ok != 0;
+}
+
+// ---------------------------------------------------------------------------
 // Strong-coupling clusters.  A coupling with |a_ij| >= tau sqrt(|a_ii a_jj|)
 // joins cells i and j; the connected clusters are found by label
 // propagation (every strong coupling hooks the labels of both cells to the
-// smaller one, then labels jump to their label's label).  The labels
+// smaller one, then every cell follows the labels to their root).  The labels
 // converge to each cluster's smallest cell index whatever the order of the
 // atomic updates, so the clusters are deterministic.
 
-__global__ void cl_init_kernel(int n, int *lab) {
-  const int i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i < n) lab[i] = i;
+constexpr int kClusterMax = 64;
+constexpr int kClusterLd = kClusterMax + 1;  // padded row of the staged block
+constexpr int kClusterRounds = 64;           // of hooks, at most
+constexpr int kClusterThreads = 512;
+constexpr int kClusterRowLanes = 8;  // lanes of a row in the hooks
+
+template <class T>
+struct ClusterSetup {
+  int n;
+  double tau;
+  const int *rowptr, *colidx, *dpos;
+  const double *J;
+  unsigned char *strong;      // by entry
+  int *lab, *cnt, *id, *loc;  // by cell; cnt and id at a cluster's smallest cell
+  int *coff, *cmem;
+  long long *cluoff;
+  T *inv;  // 1 / diagonal of the cells outside the clusters
+  unsigned long long *total;  // [3][grid]
+  ClusterCounts *out;
+  unsigned *sync;  // the barrier's words, then a changed flag per round
+};
+
+// exclusive prefix sums of a and b over the block's threads; ta, tb the totals
+__device__ __forceinline__ void block_scan(unsigned long long &a, unsigned long long &b, unsigned long long &ta,
+                                           unsigned long long &tb, unsigned long long (*sh)[2]) {
+  const int lane = threadIdx.x % 32, warp = threadIdx.x / 32;
+  unsigned long long xa = a, xb = b;
+#pragma unroll
+  for (int o = 1; o < 32; o <<= 1) {
+    const unsigned long long ua = __shfl_up_sync(0xffffffffu, xa, o), ub = __shfl_up_sync(0xffffffffu, xb, o);
+    if (lane >= o) {
+      xa += ua;
+      xb += ub;
+    }
+  }
+  __syncthreads();
+  if (lane == 31) {
+    sh[warp][0] = xa;
+    sh[warp][1] = xb;
+  }
+  __syncthreads();
+  a = xa - a;
+  b = xb - b;
+  ta = tb = 0;
+  for (int w = 0; w < kClusterThreads / 32; w++) {
+    if (w == warp) {
+      a += ta;
+      b += tb;
+    }
+    ta += sh[w][0];
+    tb += sh[w][1];
+  }
 }
 
-__global__ void cl_hook_kernel(int n, const int *rowptr, const int *colidx, const int *dpos, const double *J,
-                               double tau, int *lab, int *flag) {
-  const int i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= n) return;
-  const double di = fabs(J[dpos[i]]);
-  for (int k = rowptr[i]; k < rowptr[i + 1]; k++) {
-    const int j = colidx[k];
-    if (j == i) continue;
-    const double aij = fabs(J[k]);
-    if (!(aij > 0.0) || !(aij >= tau * sqrt(di * fabs(J[dpos[j]])))) continue;
-    const int li = lab[i], lj = lab[j];
-    if (li != lj) {
-      const int m = li < lj ? li : lj;
-      atomicMin(&lab[li], m);
-      atomicMin(&lab[lj], m);
-      *flag = 1;
+// Labels, numbering of the clusters of 2..kClusterMax cells in order of their
+// smallest cell, members (in any order: cl_factor_kernel sorts them) and the
+// other cells' diagonals, in one cooperative grid.  What bounds it is latency:
+// two barriers a round and a few for the numbering.  Set-ups and factors of
+// four Newton iterations, with a launch per step, a look at the flag per round
+// and the numbering on the host, and now: 20,960 prisms 1.27 ms and 0.53,
+// 82,400 prisms 3.41 and 1.00.
+template <class T>
+__global__ void __launch_bounds__(kClusterThreads, 2) cl_setup_kernel(const ClusterSetup<T> C) {
+  __shared__ int ok;
+  __shared__ unsigned long long sh[kClusterThreads / 32][2];
+  unsigned target = 0;
+  const int n = C.n, stride = gridDim.x * kClusterThreads, t0 = blockIdx.x * kClusterThreads + threadIdx.x;
+  for (int i = t0; i < n; i += stride) {
+    C.lab[i] = i;
+    C.cnt[i] = 0;
+  }
+  if (!grid_barrier(C.sync, target, &ok)) return;
+  unsigned *changed = C.sync + GS_COUNT;
+  bool settled = false;
+  for (int round = 0; round < kClusterRounds && !settled; round++) {
+    bool any = false;
+    for (long long e = t0; e < (long long)n * kClusterRowLanes; e += stride) {
+      const int i = (int)(e / kClusterRowLanes);
+      const double di = round ? 0.0 : fabs(C.J[C.dpos[i]]);
+      for (int k = C.rowptr[i] + (int)(e % kClusterRowLanes); k < C.rowptr[i + 1]; k += kClusterRowLanes) {
+        const int j = C.colidx[k];
+        bool s;
+        if (round) {
+          s = C.strong[k];
+        } else {
+          const double aij = fabs(C.J[k]);
+          s = j != i && aij > 0.0 && aij >= C.tau * sqrt(di * fabs(C.J[C.dpos[j]]));
+          C.strong[k] = s;
+        }
+        if (!s) continue;
+        const int li = __ldcg(&C.lab[i]), lj = __ldcg(&C.lab[j]);
+        if (li == lj) continue;
+        atomicMin(&C.lab[max(li, lj)], min(li, lj));
+        any = true;
+      }
+    }
+    if (any) changed[round] = 1;
+    if (!grid_barrier(C.sync, target, &ok)) return;
+    settled = __ldcg(&changed[round]) == 0;
+    if (settled) break;
+    for (int i = t0; i < n; i += stride) {
+      int l = __ldcg(&C.lab[i]);
+      for (int up = __ldcg(&C.lab[l]); up != l; up = __ldcg(&C.lab[l])) l = up;  // (labels only fall towards the root)
+      C.lab[i] = l;
+    }
+    if (!grid_barrier(C.sync, target, &ok)) return;
+  }
+  if (!settled) {
+    if (t0 == 0) C.out->settled = 0;
+    return;
+  }
+  for (int i = t0; i < n; i += stride) atomicAdd(&C.cnt[C.lab[i]], 1);
+  if (!grid_barrier(C.sync, target, &ok)) return;
+  // numbering: this CTA's cells [b0, b1), the sums before them from every CTA's totals
+  const long long per = (n + (long long)gridDim.x - 1) / gridDim.x;
+  const long long b0 = min((long long)n, blockIdx.x * per), b1 = min((long long)n, b0 + per);
+  auto value = [&](long long r, unsigned long long &a, unsigned long long &lu, unsigned long long &big) {
+    const int c = r < b1 ? __ldcg(&C.cnt[r]) : 0;
+    const bool in = c >= 2 && c <= kClusterMax;
+    a = in ? (1ull << 32) | (unsigned)c : 0;
+    lu = in ? (unsigned long long)c * c : 0;
+    big = c > kClusterMax ? c : 0;
+  };
+  unsigned long long sa = 0, sl = 0, sb = 0, zero = 0, ta, tl, tb, none;
+  for (long long r = b0 + threadIdx.x; r < b1; r += kClusterThreads) {
+    unsigned long long a, lu, big;
+    value(r, a, lu, big);
+    sa += a;
+    sl += lu;
+    sb += big;
+  }
+  block_scan(sa, sl, ta, tl, sh);
+  block_scan(sb, zero, tb, none, sh);
+  if (threadIdx.x == 0) {
+    C.total[blockIdx.x] = ta;
+    C.total[gridDim.x + blockIdx.x] = tl;
+    C.total[2 * gridDim.x + blockIdx.x] = tb;
+  }
+  if (!grid_barrier(C.sync, target, &ok)) return;
+  sa = sl = sb = 0;
+  for (int b = threadIdx.x; b < (int)blockIdx.x; b += kClusterThreads) {
+    sa += __ldcg(&C.total[b]);
+    sl += __ldcg(&C.total[gridDim.x + b]);
+  }
+  if (blockIdx.x == gridDim.x - 1)
+    for (int b = threadIdx.x; b < (int)gridDim.x; b += kClusterThreads) sb += __ldcg(&C.total[2 * gridDim.x + b]);
+  unsigned long long ca, cl;  // before this tile
+  block_scan(sa, sl, ca, cl, sh);
+  block_scan(sb, zero, tb, none, sh);
+  for (long long r0 = b0; r0 < b1; r0 += kClusterThreads) {
+    const long long r = r0 + threadIdx.x;
+    unsigned long long a, lu, big;
+    value(r, a, lu, big);
+    const bool in = a != 0;
+    block_scan(a, lu, ta, tl, sh);
+    if (r < b1) {
+      const int c = (int)((ca + a) >> 32);
+      C.id[r] = in ? c : -1;
+      C.cnt[r] = in ? (int)(unsigned)(ca + a) : 0;  // from here on: where the next member goes
+      if (in) {
+        C.coff[c] = (int)(unsigned)(ca + a);
+        C.cluoff[c] = (long long)(cl + lu);
+      }
+    }
+    ca += ta;
+    cl += tl;
+  }
+  if (blockIdx.x == gridDim.x - 1 && threadIdx.x == 0) {
+    C.coff[ca >> 32] = (int)(unsigned)ca;
+    C.cluoff[ca >> 32] = (long long)cl;
+    *C.out = {ca, cl, tb, 1};
+  }
+  if (!grid_barrier(C.sync, target, &ok)) return;
+  for (int i = t0; i < n; i += stride) {
+    const int l = C.lab[i], c = C.id[l];
+    C.loc[i] = c < 0 ? -1 : 0;
+    if (c >= 0) {
+      C.cmem[atomicAdd(&C.cnt[l], 1)] = i;
+    } else {
+      const double d = C.J[C.dpos[i]];
+      C.inv[i] = d != 0.0 ? (T)(1.0 / d) : (T)1;
     }
   }
 }
 
-__global__ void cl_jump_kernel(int n, int *lab, int *flag) {
-  const int i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= n) return;
-  const int l = lab[i], ll = lab[l];
-  if (ll != l) {
-    lab[i] = ll;
-    *flag = 1;
-  }
-}
-
-// cells outside the 2..64-cell clusters precondition with their diagonal
-template <class T>
-__global__ void cl_diag_kernel(int n, const int *loc, const int *dpos, const double *J, T *inv) {
-  const int i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= n || loc[i] >= 0) return;
-  const double d = J[dpos[i]];
-  inv[i] = d != 0.0 ? (T)(1.0 / d) : (T)1;
-}
-
-constexpr int kClusterMax = 64;
-constexpr int kClusterLd = kClusterMax + 1;  // padded row of the staged block
-
-// One warp per cluster: stage the cluster's block of J (every coupling
-// between its cells) in shared memory, factor it by LU with partial pivoting
-// (ties to the smaller row; a zero pivot becomes 1), store the factors column
-// by column (the solves read a column at a time) and the order of the rows.
+// One warp per cluster: sort its members, stage the cluster's block of J
+// (every coupling between its cells) in shared memory, factor it by LU with
+// partial pivoting (ties to the smaller row; a zero pivot becomes 1), store
+// the factors column by column (the solves read a column at a time) and the
+// order of the rows.
 template <class T>
 __global__ void __launch_bounds__(32) cl_factor_kernel(int ncl, const int *coff, const long long *luoff,
-                                                       const int *cmem, const int *loc, const int *lab,
+                                                       int *cmem, int *loc, const int *lab,
                                                        const int *rowptr, const int *colidx, const double *J, T *lu,
                                                        int *perm) {
   extern __shared__ unsigned char cl_smem[];
-  __shared__ int order[kClusterMax];
+  __shared__ int order[kClusterMax], member[kClusterMax];
   T *B = reinterpret_cast<T *>(cl_smem);  // [kClusterMax][kClusterLd]
   const int cl = blockIdx.x, lane = threadIdx.x;
   if (cl >= ncl) return;
   const int c0 = coff[cl], sz = coff[cl + 1] - c0;
   for (int e = lane; e < sz * kClusterLd; e += 32) B[e] = (T)0;
   __syncwarp();
+  for (int r = lane; r < sz; r += 32) order[r] = cmem[c0 + r];
+  __syncwarp();
+  for (int r = lane; r < sz; r += 32) {  // ascending cells
+    const int m = order[r];
+    int rank = 0;
+    for (int q = 0; q < sz; q++) rank += order[q] < m;
+    member[rank] = m;
+    cmem[c0 + rank] = m;
+    loc[m] = rank;
+  }
+  __syncwarp();
   for (int r = lane; r < sz; r += 32) {
     order[r] = r;
-    const int m = cmem[c0 + r], L = lab[m];
+    const int m = member[r], L = lab[m];
     for (int k = rowptr[m]; k < rowptr[m + 1]; k++) {
       const int col = colidx[k];
       if (lab[col] == L) B[r * kClusterLd + loc[col]] = (T)J[k];
@@ -1059,7 +1251,6 @@ __global__ void __launch_bounds__(32) cl_factor_kernel(int ncl, const int *coff,
 // 0.60 (8 iterations), 264,000 hexahedra with lines 16.5 and 11.2 (89),
 // 1,122,000 of them 48.5 and 30.5 (78), 192 columns 77.7 and 38.9.
 constexpr int kGridThreads = 512, kGridWarps = kGridThreads / 32;
-enum { GS_BAR = 0, GS_ACTIVE, GS_ERR, GS_COUNT };  // then a counter per chunk and per instance
 constexpr int kGridSums = 3;    // sums of one phase at most
 constexpr int kChainGroup = 4;  // cells of a chain whose loads go ahead of its stores
 
@@ -1082,35 +1273,10 @@ struct GridSolve {
   double *sc;         // [S_NSCAL][ns]
   double *acc;        // [nchunks][kGridSums][256]
   double *part;       // [kGridSums][nchunks]
-  unsigned *sync;
+  unsigned *sync;     // GS_*, then a counter per chunk and per instance
   double tol2;
   int max_it;
 };
-
-// Every CTA of the launch is past its phase; false if that took longer than
-// seconds (a CTA that gives up flags the error for the others and the host).
-__device__ __forceinline__ bool grid_barrier(unsigned *sync, unsigned &target, int *ok) {
-  __syncthreads();
-  if (threadIdx.x == 0) {
-    target += gridDim.x;
-    __threadfence();
-    atomicAdd(&sync[GS_BAR], 1u);
-    int good = 1;
-    for (unsigned spin = 0;; spin++) {
-      unsigned now;
-      asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(now) : "l"(&sync[GS_BAR]) : "memory");
-      if ((int)(now - target) >= 0) break;
-      if (spin > (1u << 23) || ((spin & 1023u) == 1023u && *(volatile unsigned *)&sync[GS_ERR])) {
-        atomicExch(&sync[GS_ERR], 1u);
-        good = 0;
-        break;
-      }
-    }
-    *ok = good;
-  }
-  __syncthreads();
-  return *ok != 0;
-}
 
 // whether this warp is the last of `of` to arrive; then it sees what the
 // others wrote, and the counter is zero again
@@ -1531,89 +1697,93 @@ int autotune_spmv(SolverState *s, Krylov &k, int forced, cudaStream_t st) {
   return 0;
 }
 
-// Clusters for the current Jacobian: label propagation on the device (at
-// most kClusterRounds rounds of one hook pass and four jump passes, until a
-// round changes nothing), compaction on the host in cell order, then the
-// factors.  Returns 0 with precond_used = TDY_PRECOND_LINES when the labels
-// have not settled (the caller then factors the lines).
-constexpr int kClusterRounds = 64;
+// A cooperative launch: its CTAs are all resident, so that its barriers end.
+template <class P>
+int launch_cooperative(void (*kern)(const P), const P &arg, long long grid, int threads, cudaStream_t st) {
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3((unsigned)std::max(1LL, grid));
+  cfg.blockDim = dim3(threads);
+  cfg.stream = st;
+  cudaLaunchAttribute at[1];
+  at[0].id = cudaLaunchAttributeCooperative;
+  at[0].val.cooperative = 1;
+  cfg.attrs = at;
+  cfg.numAttrs = 1;
+  SCUDA(cudaLaunchKernelEx(&cfg, kern, arg));
+  return 0;
+}
 
+// Clusters for the current Jacobian and their factors.  Returns 0 with
+// precond_used = TDY_PRECOND_LINES when the labels have not settled in
+// kClusterRounds rounds (the caller then factors the lines).
 template <class T>
 int cluster_setup(SolverState *s, Krylov &k, double tau, cudaStream_t st) {
-  int ierr;
+  int ierr, dev = 0, nsm = 0, per_sm = 0;
   const int n = s->n;
+  SCUDA(cudaGetDevice(&dev));
+  SCUDA(cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev));
+  SCUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, cl_setup_kernel<T>, kClusterThreads, 0));
+  const long long want = ((long long)n * kClusterRowLanes + kClusterThreads - 1) / kClusterThreads;
+  const long long grid = std::max(1LL, std::min(want, (long long)nsm * per_sm));
+  constexpr size_t nsync = GS_COUNT + kClusterRounds;
   if (!s->clab) {
-    if ((ierr = salloc(s, &s->clab, n))) return ierr;
-    if ((ierr = salloc(s, &s->cflag, 1))) return ierr;
-    if ((ierr = salloc(s, &s->cloc, n))) return ierr;
-    if ((ierr = salloc(s, &s->cmem, n))) return ierr;
-    if ((ierr = salloc(s, &s->coff, n + 1))) return ierr;
-    if ((ierr = salloc(s, &s->cluoff, n + 1))) return ierr;
-    if ((ierr = salloc(s, &s->cperm, n))) return ierr;
+    Arena ar;
+    ar.work(&s->clab, n);
+    ar.work(&s->cloc, n);
+    ar.work(&s->cmem, n);
+    ar.work(&s->cperm, n);
+    ar.work(&s->ccnt, n);
+    ar.work(&s->cid, n);
+    ar.work(&s->coff, n + 1);
+    ar.work(&s->cluoff, n + 1);
+    ar.work(&s->cstrong, s->nnz);
+    ar.work(&s->ctotal, 3 * (size_t)nsm * 4);  // (at most 2048 threads per SM)
+    ar.work(&s->csync, nsync);
+    ar.work(&s->ccounts, 1);
+    if ((ierr = ar.commit(st))) return ierr;
+    s->allocs.push_back(ar.base);
   }
   if (!k.cinv) {
     T *p;
     if ((ierr = salloc(s, &p, n))) return ierr;
     k.cinv = p;
   }
-  cl_init_kernel<<<nblk(n, 256), 256, 0, st>>>(n, s->clab);
-  bool settled = false;
-  for (int round = 0; round < kClusterRounds && !settled; round++) {
-    SCUDA(cudaMemsetAsync(s->cflag, 0, sizeof(int), st));
-    cl_hook_kernel<<<nblk(n, 128), 128, 0, st>>>(n, s->rowptr, s->colidx, s->dpos, s->J, tau, s->clab, s->cflag);
-    for (int j = 0; j < 4; j++) cl_jump_kernel<<<nblk(n, 256), 256, 0, st>>>(n, s->clab, s->cflag);
-    int flag = 1;
-    SCUDA(cudaMemcpyAsync(&flag, s->cflag, sizeof(int), cudaMemcpyDeviceToHost, st));
-    SCUDA(cudaStreamSynchronize(st));
-    settled = flag == 0;
-  }
-  if (!settled) {
+  ClusterSetup<T> C;
+  C.n = n;
+  C.tau = tau;
+  C.rowptr = s->rowptr;
+  C.colidx = s->colidx;
+  C.dpos = s->dpos;
+  C.J = s->J;
+  C.strong = s->cstrong;
+  C.lab = s->clab;
+  C.cnt = s->ccnt;
+  C.id = s->cid;
+  C.loc = s->cloc;
+  C.coff = s->coff;
+  C.cmem = s->cmem;
+  C.cluoff = s->cluoff;
+  C.inv = (T *)k.cinv;
+  C.total = s->ctotal;
+  C.out = s->ccounts;
+  C.sync = s->csync;
+  SCUDA(cudaMemsetAsync(s->csync, 0, nsync * sizeof(unsigned), st));
+  if ((ierr = launch_cooperative(cl_setup_kernel<T>, C, grid, kClusterThreads, st))) return ierr;
+  ClusterCounts counts;
+  unsigned err = 0;
+  SCUDA(cudaMemcpyAsync(&counts, s->ccounts, sizeof(counts), cudaMemcpyDeviceToHost, st));
+  SCUDA(cudaMemcpyAsync(&err, s->csync + GS_ERR, sizeof(err), cudaMemcpyDeviceToHost, st));
+  SCUDA(cudaStreamSynchronize(st));
+  if (err) return set_error(TDY_ERR_GPU, "solver: a wait of the cluster set-up ran out");
+  if (!counts.settled) {
     s->precond_used = TDY_PRECOND_LINES;
     return 0;
   }
-  // compaction: clusters of 2..kClusterMax cells in order of their smallest
-  // cell, members in ascending cell order
-  std::vector<int> &lab = s->h_lab, &cnt = s->h_cnt, &id = s->h_id, &fill = s->h_fill, &loc = s->h_loc,
-                   &mem = s->h_mem, &off = s->h_off;
-  std::vector<long long> &luoff = s->h_luoff;
-  lab.resize(n);
-  SCUDA(cudaMemcpyAsync(lab.data(), s->clab, sizeof(int) * n, cudaMemcpyDeviceToHost, st));
-  SCUDA(cudaStreamSynchronize(st));
-  cnt.assign(n, 0);
-  for (int i = 0; i < n; i++) {
-    if (lab[i] < 0 || lab[i] >= n) return set_error(TDY_ERR_LIB, "solver: cluster label %d out of range", lab[i]);
-    cnt[lab[i]]++;
-  }
-  id.assign(n, -1);
-  off.assign(1, 0);
-  luoff.assign(1, 0);
-  int ncl = 0, big = 0;
-  for (int r = 0; r < n; r++)
-    if (cnt[r] >= 2 && cnt[r] <= kClusterMax) {
-      id[r] = ncl++;
-      off.push_back(off.back() + cnt[r]);
-      luoff.push_back(luoff.back() + (long long)cnt[r] * cnt[r]);
-    } else if (cnt[r] > kClusterMax) {
-      big += cnt[r];
-    }
-  s->ncl_cells = off.back();
-  s->ncl_big_cells = big;
-  fill.assign(ncl, 0);
-  loc.assign(n, -1);
-  mem.resize(off.back());
-  for (int i = 0; i < n; i++) {
-    const int c = id[lab[i]];
-    if (c < 0) continue;
-    loc[i] = fill[c]++;
-    mem[off[c] + loc[i]] = i;
-  }
-  s->ncl = ncl;
-  SCUDA(cudaMemcpyAsync(s->cloc, loc.data(), sizeof(int) * n, cudaMemcpyHostToDevice, st));
-  if (ncl > 0) {
-    SCUDA(cudaMemcpyAsync(s->cmem, mem.data(), sizeof(int) * mem.size(), cudaMemcpyHostToDevice, st));
-    SCUDA(cudaMemcpyAsync(s->coff, off.data(), sizeof(int) * off.size(), cudaMemcpyHostToDevice, st));
-    SCUDA(cudaMemcpyAsync(s->cluoff, luoff.data(), sizeof(long long) * luoff.size(), cudaMemcpyHostToDevice, st));
-    const size_t need = (size_t)luoff.back();
+  s->ncl = (int)(counts.both >> 32);
+  s->ncl_cells = (int)(unsigned)counts.both;
+  s->ncl_big_cells = (int)counts.big;
+  if (s->ncl > 0) {
+    const size_t need = (size_t)counts.lu;
     if (need > k.clu_cap) {  // stream-ordered: no device synchronisation
       if (k.clu) dmem_free(k.clu, st);
       k.clu = nullptr;
@@ -1621,14 +1791,10 @@ int cluster_setup(SolverState *s, Krylov &k, double tau, cudaStream_t st) {
       if ((ierr = dmem_alloc(&k.clu, need * sizeof(T), st))) return ierr;
       k.clu_cap = need;
     }
+    cl_factor_kernel<T><<<s->ncl, 32, kClusterMax * kClusterLd * sizeof(T), st>>>(
+        s->ncl, s->coff, s->cluoff, s->cmem, s->cloc, s->clab, s->rowptr, s->colidx, s->J, (T *)k.clu, s->cperm);
+    SCUDA(cudaGetLastError());
   }
-  cl_diag_kernel<T><<<nblk(n, 256), 256, 0, st>>>(n, s->cloc, s->dpos, s->J, (T *)k.cinv);
-  if (ncl > 0)
-    cl_factor_kernel<T><<<ncl, 32, kClusterMax * kClusterLd * sizeof(T), st>>>(
-        ncl, s->coff, s->cluoff, s->cmem, s->cloc, s->clab, s->rowptr, s->colidx, s->J, (T *)k.clu, s->cperm);
-  SCUDA(cudaGetLastError());
-  // the host vectors above stay alive until the copies complete
-  SCUDA(cudaStreamSynchronize(st));
   s->precond_used = TDY_PRECOND_CLUSTERS;
   return 0;
 }
@@ -1857,26 +2023,15 @@ int launch_block(SolverState *s, Krylov &k, const TDyNewtonOptions &o, double to
   return 0;
 }
 
-// The active instances of the tile schedule.  As many CTAs as the product has
-// rows for, up to what the GPU holds at once: a cooperative launch, whose CTAs
-// are all resident, so that its barriers end.
+// The active instances of the tile schedule: as many CTAs as the product has
+// rows for, up to what the GPU holds at once.
 template <class T, int TPR>
 int launch_grid_tpr(const GridSolve<T> &G, int nsm, cudaStream_t st) {
   auto kern = bicgstab_grid_kernel<T, TPR>;
   int per_sm = 0;
   SCUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, kGridThreads, 0));
   const long long want = ((long long)G.n * TPR + kGridThreads - 1) / kGridThreads;
-  cudaLaunchConfig_t cfg = {};
-  cfg.gridDim = dim3((unsigned)std::max(1LL, std::min(want, (long long)nsm * per_sm)));
-  cfg.blockDim = dim3(kGridThreads);
-  cfg.stream = st;
-  cudaLaunchAttribute at[1];
-  at[0].id = cudaLaunchAttributeCooperative;
-  at[0].val.cooperative = 1;
-  cfg.attrs = at;
-  cfg.numAttrs = 1;
-  SCUDA(cudaLaunchKernelEx(&cfg, kern, G));
-  return 0;
+  return launch_cooperative(kern, G, std::min(want, (long long)nsm * per_sm), kGridThreads, st);
 }
 
 template <class T>

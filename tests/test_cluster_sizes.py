@@ -43,3 +43,36 @@ def test_column_is_one_cluster(nz):
     if nz <= 64:
         assert c["linear_iterations"] == c["newton_iterations"] >= 1, c
     assert np.max(np.abs(U["clusters"] - U["lines"]) / np.abs(U["lines"])) < 1e-9
+
+
+@pytest.mark.parametrize("triangles,layers", [(60, 3), (500, 9), (2000, 20)])
+@pytest.mark.parametrize("tau", [0.02, 0.05, 0.3, 1e300])
+def test_clusters_are_the_connected_components(triangles, layers, tau):
+    """Number and cells of the clusters of the first inner solve against the
+    connected components of the strong couplings of the Jacobian there."""
+    import torch
+    from scipy.sparse import coo_matrix
+    from scipy.sparse.csgraph import connected_components
+
+    from tdycore_gb300.workloads import infiltration_prisms
+
+    T.options_clear()
+    t, U, top, src, _ = infiltration_prisms(triangles, layers)
+    t.setup()
+    t.set_source_sink_values(src, cells=top)
+    n = t.ncells
+    d = torch.tensor(U, dtype=torch.float64, device="cuda")
+    st, _, _ = t.backward_euler_step_device(d, 600.0, max_it=1, precond="clusters", cluster_threshold=tau)
+    t.set_dtime(600.0)
+    t.presolve(U)
+    J = np.abs(t.snes_jacobian(U))
+    row, col = np.repeat(np.arange(n), np.diff(t.rowptr)), t.colidx
+    diag = np.zeros(n)
+    diag[row[row == col]] = J[row == col]
+    strong = (row != col) & (J > 0) & (J >= tau * np.sqrt(diag[row] * diag[col]))
+    label = connected_components(coo_matrix((strong[strong], (row[strong], col[strong])), shape=(n, n)), directed=False)[1]
+    size = np.bincount(label)
+    used = (size >= 2) & (size <= 64)
+    assert st["precond_used"] == T.PRECOND_CLUSTERS
+    assert (st["clusters"], st["cluster_cells"], st["cluster_cells_diagonal"]) == (
+        used.sum(), size[used].sum(), size[size > 64].sum())
