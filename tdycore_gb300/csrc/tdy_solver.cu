@@ -50,7 +50,7 @@ namespace {
 inline unsigned nblk(long long n, int bs) { return (unsigned)((n + bs - 1) / bs); }
 
 // per-instance scalars, [slot][nseg]
-enum { S_RHO = 0, S_ALPHA, S_OMEGA, S_BETA, S_BNORM2, S_XNORM2, S_HALF, S_NSCAL };
+enum { S_RHO = 0, S_ALPHA, S_OMEGA, S_BETA, S_BNORM2, S_HALF, S_NSCAL };
 
 // what the host reads of a set-up of clusters
 struct ClusterCounts {
@@ -80,15 +80,19 @@ struct SolverState {
   std::vector<int> h_seg_off;
   int *rowptr = nullptr, *colidx = nullptr, *seg_off = nullptr, *cell_seg = nullptr;
   int *line_off = nullptr, *line_cells = nullptr, *pos_d = nullptr, *pos_lo = nullptr, *pos_hi = nullptr;
-  double *x = nullptr, *xb = nullptr, *F = nullptr, *J = nullptr, *fn2 = nullptr, *scal = nullptr, *lam = nullptr;
+  double *x = nullptr, *xb = nullptr, *F = nullptr, *J = nullptr, *norms = nullptr, *scal = nullptr, *lam = nullptr;
   int *trial = nullptr, *commit = nullptr;
   int *newt_active = nullptr, *lin_active = nullptr, *lin_its = nullptr;
   int nchunks = 0;
   int *chunk_off = nullptr, *seg_chunk = nullptr;  // chunks of the per-instance reductions
   double *part = nullptr;
-  // the tile schedule's sums (accumulators and chunk sums) and counters, on its first use
+  // the tile schedule's sums (accumulators and chunk sums), on its first use
   double *grid_acc = nullptr, *grid_part = nullptr;
+  // what the host reads of a linear solve, in one copy: ||y||^2 and iterations
+  // per instance, then the words of the tile schedule (GS_*; zeroed with lin_its)
+  double *y2 = nullptr;
   unsigned *grid_sync = nullptr;
+  std::vector<double> h_out;
   int *dpos = nullptr;  // position of each row's diagonal in the CSR values
   // strong-coupling clusters, rebuilt for every linear solve that uses them:
   // scratch of the set-up (cl_setup_kernel), label per cell, local index in
@@ -219,34 +223,36 @@ __global__ void cast_masked_kernel(int n, const int *cell_seg, const int *flag, 
   if (i < n && flag[cell_seg[i]]) b[i] = (float)a[i];
 }
 
-// Per-instance dot products in two deterministic passes: one block per chunk
-// of at most kChunk cells (chunks counted from each instance's first cell, so
-// an instance is reduced the same way alone and in a batch), then one thread
-// per instance adding its chunks in order.
+// Per-instance squared norms of one or two vectors in two deterministic
+// passes: one block per chunk of at most kChunk cells (chunks counted from
+// each instance's first cell, so an instance is reduced the same way alone and
+// in a batch), then one thread per instance adding its chunks in order.
 constexpr int kChunk = 4096;
 
-template <class TA, class TB>
-__global__ void __launch_bounds__(256) chunk_dot_kernel(const int *chunk_off, const TA *a, const TB *b, double *part) {
+template <class T>
+__global__ void __launch_bounds__(256) chunk_norm_kernel(const int *chunk_off, int nchunks, const T *a, const T *b,
+                                                         double *part) {
   __shared__ double sh[256];
   const int ch = blockIdx.x;
   const int i0 = chunk_off[ch], i1 = chunk_off[ch + 1];
+  const T *v = blockIdx.y ? b : a;
   double acc = 0.0;
-  for (int i = i0 + threadIdx.x; i < i1; i += blockDim.x) acc = op_dot(acc, a[i], b[i]);
+  for (int i = i0 + threadIdx.x; i < i1; i += blockDim.x) acc = op_dot(acc, v[i], v[i]);
   sh[threadIdx.x] = acc;
   __syncthreads();
   for (int w = blockDim.x / 2; w > 0; w >>= 1) {
     if ((int)threadIdx.x < w) sh[threadIdx.x] += sh[threadIdx.x + w];
     __syncthreads();
   }
-  if (threadIdx.x == 0) part[ch] = sh[0];
+  if (threadIdx.x == 0) part[(size_t)blockIdx.y * nchunks + ch] = sh[0];
 }
 
-__global__ void chunk_sum_kernel(int nseg, const int *seg_chunk, const double *part, double *out) {
+__global__ void chunk_sum_kernel(int nseg, const int *seg_chunk, int nchunks, const double *part, double *out) {
   const int s = blockIdx.x * blockDim.x + threadIdx.x;
   if (s >= nseg) return;
   double acc = 0.0;
-  for (int k = seg_chunk[s]; k < seg_chunk[s + 1]; k++) acc += part[k];
-  out[s] = acc;
+  for (int k = seg_chunk[s]; k < seg_chunk[s + 1]; k++) acc += part[(size_t)blockIdx.y * nchunks + k];
+  out[(size_t)blockIdx.y * nseg + s] = acc;
 }
 
 // y = A x over the CSR pattern with TPR threads per row
@@ -668,7 +674,7 @@ __global__ void __launch_bounds__(kBlockThreads, sizeof(T) == 4 ? 2 : 1) bicgsta
     };
 
     // (vector k0, vector k1) and, with k2 >= 0, (vector k2, vector k3): per
-    // chunk the accumulators and the 256-way tree of chunk_dot_kernel, then the
+    // chunk the accumulators and the 256-way tree of chunk_norm_kernel, then the
     // chunks in order.  With C > 1 each sum and chunk has threads (and a part of
     // the FP64 pipe) of its own, and one warp does each tree (the additions of a
     // warp take 60 cycles each); another one does `side` meanwhile.  Thread 0 of
@@ -1298,7 +1304,7 @@ __device__ __forceinline__ bool last_arrival(unsigned *count, int of, int lane) 
 
 // The accumulators 32 w + lane of chunk ch (of `cells` cells, instance g) are
 // in a.  True in the warp that holds the instance's sums, in every lane: the
-// tree of chunk_dot_kernel (levels 128, 64, 32 across the 8 values of a lane,
+// tree of chunk_norm_kernel (levels 128, 64, 32 across the 8 values of a lane,
 // the others by shuffles), then the chunks in order.
 template <int ND, class T>
 __device__ __forceinline__ bool chunk_sums(const GridSolve<T> &G, int ch, int w, int cells, int g, int lane,
@@ -1638,10 +1644,12 @@ void spmv(SolverState *s, const Krylov &k, const T *x, T *y, cudaStream_t st) {
   }
 }
 
-template <class TA, class TB>
-void seg_dot(SolverState *s, const TA *a, const TB *b, double *out, cudaStream_t st) {
-  chunk_dot_kernel<TA, TB><<<s->nchunks, 256, 0, st>>>(s->chunk_off, a, b, s->part);
-  chunk_sum_kernel<<<nblk(s->nseg, 128), 128, 0, st>>>(s->nseg, s->seg_chunk, s->part, out);
+// out = ||a||^2 per instance (, then ||b||^2)
+template <class T>
+void seg_norms(SolverState *s, const T *a, const T *b, double *out, cudaStream_t st) {
+  const unsigned nv = b ? 2 : 1;
+  chunk_norm_kernel<T><<<dim3(s->nchunks, nv), 256, 0, st>>>(s->chunk_off, s->nchunks, a, b, s->part);
+  chunk_sum_kernel<<<dim3(nblk(s->nseg, 128), nv), 128, 0, st>>>(s->nseg, s->seg_chunk, s->nchunks, s->part, out);
 }
 
 // (one allocation for every vector; ordered on the solve's stream, which uses
@@ -1738,10 +1746,10 @@ int cluster_setup(SolverState *s, Krylov &k, double tau, cudaStream_t st) {
     ar.work(&s->cluoff, n + 1);
     ar.work(&s->cstrong, s->nnz);
     ar.work(&s->ctotal, 3 * (size_t)nsm * 4);  // (at most 2048 threads per SM)
-    ar.work(&s->csync, nsync);
-    ar.work(&s->ccounts, 1);
+    ar.work(&s->ccounts, 1 + (nsync * sizeof(unsigned) + sizeof(ClusterCounts) - 1) / sizeof(ClusterCounts));  // then csync
     if ((ierr = ar.commit(st))) return ierr;
     s->allocs.push_back(ar.base);
+    s->csync = reinterpret_cast<unsigned *>(s->ccounts + 1);
   }
   if (!k.cinv) {
     T *p;
@@ -1769,12 +1777,14 @@ int cluster_setup(SolverState *s, Krylov &k, double tau, cudaStream_t st) {
   C.sync = s->csync;
   SCUDA(cudaMemsetAsync(s->csync, 0, nsync * sizeof(unsigned), st));
   if ((ierr = launch_cooperative(cl_setup_kernel<T>, C, grid, kClusterThreads, st))) return ierr;
-  ClusterCounts counts;
-  unsigned err = 0;
-  SCUDA(cudaMemcpyAsync(&counts, s->ccounts, sizeof(counts), cudaMemcpyDeviceToHost, st));
-  SCUDA(cudaMemcpyAsync(&err, s->csync + GS_ERR, sizeof(err), cudaMemcpyDeviceToHost, st));
+  struct {
+    ClusterCounts counts;
+    unsigned sync[GS_COUNT];
+  } out;
+  SCUDA(cudaMemcpyAsync(&out, s->ccounts, sizeof(ClusterCounts) + sizeof(unsigned) * GS_COUNT, cudaMemcpyDeviceToHost, st));
   SCUDA(cudaStreamSynchronize(st));
-  if (err) return set_error(TDY_ERR_GPU, "solver: a wait of the cluster set-up ran out");
+  if (out.sync[GS_ERR]) return set_error(TDY_ERR_GPU, "solver: a wait of the cluster set-up ran out");
+  const ClusterCounts &counts = out.counts;
   if (!counts.settled) {
     s->precond_used = TDY_PRECOND_LINES;
     return 0;
@@ -2034,21 +2044,21 @@ int launch_grid_tpr(const GridSolve<T> &G, int nsm, cudaStream_t st) {
   return launch_cooperative(kern, G, std::min(want, (long long)nsm * per_sm), kGridThreads, st);
 }
 
+// words of the tile schedule behind lin_its
+inline size_t grid_words(const SolverState *s) { return GS_COUNT + (size_t)s->nchunks + s->nseg; }
+
 template <class T>
 int launch_grid(SolverState *s, Krylov &k, const TDyNewtonOptions &o, double tol2, cudaStream_t st) {
   int ierr, dev = 0, nsm = 0;
   SCUDA(cudaGetDevice(&dev));
   SCUDA(cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev));
-  const size_t nsync = GS_COUNT + (size_t)s->nchunks + s->nseg;
-  if (!s->grid_sync) {
+  if (!s->grid_acc) {
     Arena ar;
     ar.work(&s->grid_acc, (size_t)s->nchunks * kGridSums * 256);
     ar.work(&s->grid_part, (size_t)s->nchunks * kGridSums);
-    ar.work(&s->grid_sync, nsync);
     if ((ierr = ar.commit(st))) return ierr;
     s->allocs.push_back(ar.base);
   }
-  SCUDA(cudaMemsetAsync(s->grid_sync, 0, nsync * sizeof(unsigned), st));
   GridSolve<T> G;
   G.n = s->n;
   G.ns = s->nseg;
@@ -2110,16 +2120,21 @@ int solve_scheduled(SolverState *s, Krylov &k, const TDyNewtonOptions &o, double
   int ierr;
   const int ns = s->nseg;
   if ((ierr = set_block_split(s, thr, st))) return ierr;
-  SCUDA(cudaMemsetAsync(s->lin_its, 0, sizeof(int) * ns, st));
+  SCUDA(cudaMemsetAsync(s->lin_its, 0, sizeof(int) * (ns + grid_words(s)), st));
   if (s->n_block > 0 && (ierr = launch_block<T>(s, k, o, tol2, thr, newt_act, st))) return ierr;
-  unsigned err = 0;
-  if (s->n_tile > 0) {
-    if ((ierr = launch_grid<T>(s, k, o, tol2, st))) return ierr;
-    SCUDA(cudaMemcpyAsync(&err, s->grid_sync + GS_ERR, sizeof(err), cudaMemcpyDeviceToHost, st));
-  }
-  its.resize(ns);
-  SCUDA(cudaMemcpyAsync(its.data(), s->lin_its, sizeof(int) * ns, cudaMemcpyDeviceToHost, st));
+  if (s->n_tile > 0 && (ierr = launch_grid<T>(s, k, o, tol2, st))) return ierr;
+  SCUDA(cudaEventRecord(s->tev[4], st));
+  seg_norms<T>(s, (const T *)k.y, nullptr, s->y2, st);
+  SCUDA(cudaGetLastError());
+  const size_t bytes = sizeof(double) * ns + sizeof(int) * ns + sizeof(unsigned) * GS_COUNT;
+  s->h_out.resize((bytes + 7) / 8);
+  SCUDA(cudaMemcpyAsync(s->h_out.data(), s->y2, bytes, cudaMemcpyDeviceToHost, st));
   SCUDA(cudaStreamSynchronize(st));
+  const char *tail = reinterpret_cast<const char *>(s->h_out.data() + ns);
+  its.resize(ns);
+  std::memcpy(its.data(), tail, sizeof(int) * ns);
+  unsigned err;
+  std::memcpy(&err, tail + sizeof(int) * ns + sizeof(unsigned) * GS_ERR, sizeof(err));
   if (err) return set_error(TDY_ERR_GPU, "solver: a wait of the tile schedule ran out");
   return 0;
 }
@@ -2243,7 +2258,6 @@ int linear_solve(SolverState *s, Krylov &k, const TDyNewtonOptions &o, const std
   std::vector<int> its(ns);
   if (tune && (ierr = tune_schedule<T>(s, k, o, tol2, act, st, &thr))) return ierr;
   if ((ierr = solve_scheduled<T>(s, k, o, tol2, thr, act, st, its))) return ierr;
-  SCUDA(cudaEventRecord(s->tev[4], st));
   for (int v : its) *lin_total += v;
   inst_lin_its = its;
   return 0;
@@ -2326,7 +2340,7 @@ int solver_init(_p_TDy *t) {
   ar.up(&s->seg_off, seg_off);
   ar.up(&s->chunk_off, chunk_off);
   ar.up(&s->seg_chunk, seg_chunk);
-  ar.work(&s->part, s->nchunks);
+  ar.work(&s->part, 2 * (size_t)s->nchunks);
   ar.up(&s->cell_seg, cell_seg);
   ar.up(&s->line_off, line_off);
   ar.up(&s->line_cells, line_cells);
@@ -2336,22 +2350,24 @@ int solver_init(_p_TDy *t) {
   ar.up(&s->pos_hi, phi);
   ar.work(&s->x, s->n);
   ar.work(&s->xb, s->n);
-  ar.work(&s->lam, s->nseg);
-  ar.work(&s->trial, s->nseg);
+  ar.work(&s->lam, s->nseg + (s->nseg + 1) / 2);  // then trial, copied with it
   ar.work(&s->commit, s->nseg);
   ar.work(&s->F, s->n);
   ar.work(&s->J, s->nnz);
-  ar.work(&s->fn2, s->nseg);
+  ar.work(&s->norms, 2 * s->nseg);
   ar.work(&s->scal, (size_t)S_NSCAL * s->nseg);
   ar.work(&s->newt_active, s->nseg);
   ar.work(&s->lin_active, s->nseg);
-  ar.work(&s->lin_its, s->nseg);
+  ar.work(&s->y2, s->nseg + (s->nseg + grid_words(s) + 1) / 2);  // then lin_its and grid_sync
   ar.up(&s->inst_line_off, inst_line_off);
   ar.work(&s->block_inst, s->nseg);
   ar.work(&s->block_mask, s->nseg);
   ar.work(&s->ticket, kBlockClasses);
   if ((ierr = ar.commit(s->st))) return ierr;
   s->allocs.push_back(ar.base);
+  s->trial = reinterpret_cast<int *>(s->lam + s->nseg);
+  s->lin_its = reinterpret_cast<int *>(s->y2 + s->nseg);
+  s->grid_sync = reinterpret_cast<unsigned *>(s->lin_its + s->nseg);
   // the allocations and uploads complete before any other stream uses them
   // (and before the host vectors above go out of scope)
   SCUDA(cudaStreamSynchronize(s->st));
@@ -2393,8 +2409,11 @@ int device_be_solve(_p_TDy *t, double dt, double *dU, const TDyNewtonOptions &o,
   if ((ierr = device_presolve(t, dU, st, true))) return ierr;
   SCUDA(cudaMemcpyAsync(s->x, dU, sizeof(double) * n, cudaMemcpyDeviceToDevice, st));
   SCUDA(cudaMemcpyAsync(s->xb, dU, sizeof(double) * n, cudaMemcpyDeviceToDevice, st));
-  std::vector<double> f0(ns, 0.0), fn(ns, 0.0), g2(ns, 0.0), lam(ns, 1.0);
-  std::vector<int> act(ns, 1), its(ns, 0), trial(ns, 0), commit(ns, 0), step_conv(ns, 0), failed(ns, 0);
+  std::vector<double> f0(ns, 0.0), fn(ns, 0.0), g2(2 * ns, 0.0);  // (g2: of F, then of x)
+  std::vector<char> lam_trial((sizeof(double) + sizeof(int)) * ns);  // packed as on the device
+  double *const lam = reinterpret_cast<double *>(lam_trial.data());
+  int *const trial = reinterpret_cast<int *>(lam + ns);
+  std::vector<int> act(ns, 1), its(ns, 0), commit(ns, 0), step_conv(ns, 0), failed(ns, 0);
   // instances retired by the caller are not advanced (TDySetActiveInstances)
   const bool masked = (int)t->inst_active.size() == ns;
   std::vector<int> live;
@@ -2410,7 +2429,7 @@ int device_be_solve(_p_TDy *t, double dt, double *dU, const TDyNewtonOptions &o,
   double t_eval = 0.0, t_prec = 0.0, t_kry = 0.0;  // ms on the stream
   int inner_redo = 0;  // FP32 inner solves redone in FP64 (instances x Newton iterations)
   // F and J at x (= xb for every instance after each evaluation below), and
-  // the squared per-instance residual norms into g2
+  // the squared per-instance norms of F and x into g2
   // `sub` (host list of instances, or null for all): only those instances'
   // states changed since the last evaluation, the others keep F and J
   auto evaluate = [&](const std::vector<int> *sub = nullptr) -> int {
@@ -2423,9 +2442,9 @@ int device_be_solve(_p_TDy *t, double dt, double *dU, const TDyNewtonOptions &o,
       e = device_eval(t, FORM_SNES, 0.0, s->x, nullptr, 0.0, s->F, s->J, st, true);
     if (e) return e;
     SCUDA(cudaEventRecord(s->tev[1], st));
-    seg_dot<double, double>(s, s->F, s->F, s->fn2, st);
+    seg_norms<double>(s, s->F, s->x, s->norms, st);
     SCUDA(cudaGetLastError());
-    SCUDA(cudaMemcpyAsync(g2.data(), s->fn2, sizeof(double) * ns, cudaMemcpyDeviceToHost, st));
+    SCUDA(cudaMemcpyAsync(g2.data(), s->norms, sizeof(double) * 2 * ns, cudaMemcpyDeviceToHost, st));
     SCUDA(cudaStreamSynchronize(st));
     float ms = 0.f;
     SCUDA(cudaEventElapsedTime(&ms, s->tev[0], s->tev[1]));
@@ -2433,7 +2452,10 @@ int device_be_solve(_p_TDy *t, double dt, double *dU, const TDyNewtonOptions &o,
     return 0;
   };
   if ((ierr = evaluate(masked ? &live : nullptr))) return ierr;
-  for (int g = 0; g < ns; g++) f0[g] = fn[g] = std::sqrt(g2[g]);
+  for (int g = 0; g < ns; g++) {
+    f0[g] = fn[g] = std::sqrt(g2[g]);
+    x2[g] = g2[ns + g];
+  }
   const double alpha = 1e-4;  // sufficient-decrease constant of PETSc's backtracking line search
   constexpr double kMaxStep = 1e8;  // PETSc's default SNESLineSearch maxstep
   const int max_backtracks = 12;
@@ -2485,6 +2507,9 @@ int device_be_solve(_p_TDy *t, double dt, double *dU, const TDyNewtonOptions &o,
         cast_masked_kernel<<<nblk(n, 256), 256, 0, st>>>(n, s->cell_seg, s->newt_active, (const double *)s->k64.y,
                                                          (float *)s->k32.y);
         SCUDA(cudaMemcpyAsync(s->newt_active, act.data(), sizeof(int) * ns, cudaMemcpyHostToDevice, st));
+        seg_norms<float>(s, (const float *)s->k32.y, nullptr, s->y2, st);
+        SCUDA(cudaGetLastError());
+        SCUDA(cudaMemcpyAsync(s->h_out.data(), s->y2, sizeof(double) * ns, cudaMemcpyDeviceToHost, st));
         SCUDA(cudaStreamSynchronize(st));  // redo and act (host vectors) stay valid until here
         for (int g = 0; g < ns; g++)
           if (redo[g]) {
@@ -2499,20 +2524,11 @@ int device_be_solve(_p_TDy *t, double dt, double *dU, const TDyNewtonOptions &o,
       y = s->k64.y;
     }
     if (ierr) return ierr;
-    // ||y|| and ||x|| before the step: PETSc's backtracking line search caps
-    // the step at maxstep and ends with convergence by the step test when the
-    // full step fails and ||y|| < stol ||x||
-    {
-      if (fp32)
-        seg_dot<float, float>(s, (const float *)y, (const float *)y, s->fn2, st);
-      else
-        seg_dot<double, double>(s, (const double *)y, (const double *)y, s->fn2, st);
-      seg_dot<double, double>(s, s->xb, s->xb, s->scal + (size_t)S_XNORM2 * ns, st);
-      SCUDA(cudaGetLastError());
-      SCUDA(cudaMemcpyAsync(y2.data(), s->fn2, sizeof(double) * ns, cudaMemcpyDeviceToHost, st));
-      SCUDA(cudaMemcpyAsync(x2.data(), s->scal + (size_t)S_XNORM2 * ns, sizeof(double) * ns, cudaMemcpyDeviceToHost, st));
-      SCUDA(cudaStreamSynchronize(st));
-    }
+    // ||y|| and ||x|| before the step (y2 and x2, from the solve and the last
+    // accepted evaluation): PETSc's backtracking line search caps the step at
+    // maxstep and ends with convergence by the step test when the full step
+    // fails and ||y|| < stol ||x||
+    for (int g = 0; g < ns; g++) y2[g] = s->h_out[g];
     // backtracking per instance: accept when ||F(x - lam y)||^2 <= (1 - 2 alpha lam) ||F(x)||^2
     // (initial slope -||F||^2 of the Newton direction), else a quadratic fit of
     // lam clamped to [0.1 lam, 0.5 lam] (PETSc SNESLineSearchApply_BT)
@@ -2524,8 +2540,7 @@ int device_be_solve(_p_TDy *t, double dt, double *dU, const TDyNewtonOptions &o,
       lam[g] = yn > kMaxStep ? kMaxStep / yn : 1.0;
     }
     for (int ls = 0; ls <= max_backtracks; ls++) {
-      SCUDA(cudaMemcpyAsync(s->trial, trial.data(), sizeof(int) * ns, cudaMemcpyHostToDevice, st));
-      SCUDA(cudaMemcpyAsync(s->lam, lam.data(), sizeof(double) * ns, cudaMemcpyHostToDevice, st));
+      SCUDA(cudaMemcpyAsync(s->lam, lam, (sizeof(double) + sizeof(int)) * ns, cudaMemcpyHostToDevice, st));
       if (fp32)
         trial_kernel<float><<<nblk(n, 256), 256, 0, st>>>(n, s->cell_seg, s->trial, s->lam, (const float *)y, s->xb,
                                                           s->x);
@@ -2552,6 +2567,7 @@ int device_be_solve(_p_TDy *t, double dt, double *dU, const TDyNewtonOptions &o,
           commit[g] = 1;
           trial[g] = 0;
           fn[g] = std::sqrt(gg);
+          x2[g] = g2[ns + g];
         } else if (ls == max_backtracks) {
           // no finite residual along the step, or an unconverged inner solve
           // whose smallest step more than doubles ||F||: keep the last
@@ -2582,22 +2598,12 @@ int device_be_solve(_p_TDy *t, double dt, double *dU, const TDyNewtonOptions &o,
     // y the full Newton step (PETSc's backtracking line search reports the
     // norm of the step before its lambda scaling), so a step cut short by the
     // line search does not count as convergence.
-    if (o.stol > 0.0) {
-      if (fp32)
-        seg_dot<float, float>(s, (const float *)y, (const float *)y, s->fn2, st);
-      else
-        seg_dot<double, double>(s, (const double *)y, (const double *)y, s->fn2, st);
-      seg_dot<double, double>(s, s->xb, s->xb, s->scal + (size_t)S_XNORM2 * ns, st);
-      SCUDA(cudaGetLastError());
-      SCUDA(cudaMemcpyAsync(y2.data(), s->fn2, sizeof(double) * ns, cudaMemcpyDeviceToHost, st));
-      SCUDA(cudaMemcpyAsync(x2.data(), s->scal + (size_t)S_XNORM2 * ns, sizeof(double) * ns, cudaMemcpyDeviceToHost, st));
-      SCUDA(cudaStreamSynchronize(st));
+    if (o.stol > 0.0)
       for (int g = 0; g < ns; g++)
         if (act[g] && std::sqrt(y2[g]) < o.stol * std::sqrt(x2[g])) {
           act[g] = 0;
           step_conv[g] = 1;
         }
-    }
   }
   SCUDA(cudaMemcpyAsync(dU, s->xb, sizeof(double) * n, cudaMemcpyDeviceToDevice, st));
   SCUDA(cudaStreamSynchronize(st));
