@@ -1171,6 +1171,7 @@ __device__ __forceinline__ void generic_vertex_group(const DevArgs &a, int block
 // so they overlap and the chain of their rows is off the launch's tail.
 template <int RHO, bool FFJ>
 __global__ void __launch_bounds__(128) vertex_kernel(DevArgs a, int gen_blocks) {
+  stage_begin();
   if ((int)blockIdx.x >= gen_blocks) {
     const int vc = a.vc0 + ((int)blockIdx.x - gen_blocks) * blockDim.x + threadIdx.x;
     if (vc < a.vc1 && !inst_skipped(a, a.cellc[vc])) canon_vertex_at<RHO, FFJ>(a, vc, threadIdx.x);
@@ -1184,6 +1185,7 @@ __global__ void __launch_bounds__(128) vertex_kernel(DevArgs a, int gen_blocks) 
 constexpr int kPairThreads = 128;
 template <int RHO>
 __global__ void __launch_bounds__(kPairThreads, 7) vertex_pair_kernel(DevArgs a, int gen_blocks) {
+  stage_begin();
   if ((int)blockIdx.x >= gen_blocks) {
     const int slot = threadIdx.x >> 1, h = threadIdx.x & 1;
     const int vc = a.vc0 + ((int)blockIdx.x - gen_blocks) * (kPairThreads / 2) + slot;
@@ -1195,6 +1197,7 @@ __global__ void __launch_bounds__(kPairThreads, 7) vertex_pair_kernel(DevArgs a,
 
 template <bool FFJ>
 __global__ void __launch_bounds__(128) generic_vertex_kernel(DevArgs a) {
+  stage_begin();
   generic_vertex_group<FFJ>(a, blockIdx.x);
 }
 
@@ -1292,6 +1295,7 @@ constexpr int kCellThreads = 128;
 constexpr int kCellWords = 8;  // words held per lane: rows of up to 64 entries
 
 __global__ void __launch_bounds__(kCellThreads) generic_cell_kernel(DevArgs a) {
+  stage_begin();
   extern __shared__ double rowbuf[];  // per cell: the row, then the vertices' rows
   constexpr int NC = kCellThreads / kCellLanes, L = kCellLanes;
   const int tid = threadIdx.x, grp = tid / L, lane = tid % L, block = blockIdx.x;
@@ -1392,6 +1396,7 @@ __global__ void __launch_bounds__(kCellThreads) generic_cell_kernel(DevArgs a) {
 // shared memory, 0.22 ms with 80 registers and 24 warps, 0.31 ms with the
 // other cells in the same launch (69 registers).
 __global__ void __launch_bounds__(64, 8) cell_kernel(DevArgs a) {
+  stage_begin();
   struct_cell_at(a, blockIdx.x * blockDim.x + threadIdx.x, a.nS);
 }
 
@@ -1973,6 +1978,7 @@ static int launch_eval(const DevArgs &a, cudaStream_t st, cudaEvent_t *events) {
   Emit e(st);
   if (events) CUDA_TRY(cudaEventRecord(events[0], st));
   launch_state(a, e);
+  e.overlap = true;  // (behind an event record the stages follow as before)
   if (events) CUDA_TRY(cudaEventRecord(events[1], st));
   launch_vertices(a, e);
   if (events) CUDA_TRY(cudaEventRecord(events[2], st));
