@@ -1880,7 +1880,8 @@ constexpr int kBlockClasses = 2 * 4 * 3 + 2;
 template <class T, int C, int KEEP>
 int launch_block_class(const BlockSolve<T> &B, size_t smem, int nsm, cudaStream_t st) {
   auto kern = bicgstab_block_kernel<T, C, KEEP>;
-  if (smem > 48 * 1024) SCUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kBlockSmemMax));
+  // (the 48 KB that need no attribute hold the static shared memory as well)
+  if (smem > 47 * 1024) SCUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kBlockSmemMax));
   int per_sm = 0;
   SCUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, kBlockThreads, smem));
   const int grid = C * std::max(1, std::min(B.ninst, nsm * std::max(per_sm, 1) / C));
@@ -1929,6 +1930,7 @@ int launch_block(SolverState *s, Krylov &k, const TDyNewtonOptions &o, double to
     std::vector<int> inst;
     size_t smem = 0, slots = 0;
   } cls[kBlockClasses];
+  constexpr size_t slot_bytes = sizeof(T) + sizeof(uint16_t);  // of a matrix entry
   for (int g : s->h_order) {
     if (!act[g] || !on_block(s, thr, g)) continue;
     int c = block_ctas(cells(g), total, nsm, sizeof(T)), lg = c == 8 ? 3 : c == 4 ? 2 : c == 2 ? 1 : 0;
@@ -1937,15 +1939,28 @@ int launch_block(SolverState *s, Krylov &k, const TDyNewtonOptions &o, double to
     // the matrix in shared memory, in batches of many CTAs where it leaves two
     // per SM (28 instances up to 5,264 cells: 2.0 ms against 2.5 ms with the
     // half limit; 192 instances: 4.6 against 3.8 ms)
-    size_t smem = smem_of(KEEP_MATRIX, 1 << lg, g);
-    if (smem <= (ctas <= 2 * nsm ? kBlockSmemMax : kBlockSmemMax / 2))
-      keep = KEEP_MATRIX;
-    else
-      smem = smem_of(KEEP_ALL, 1 << lg, g);
-    if (smem <= kBlockSmemMax) {
+    size_t smem = smem_of(KEEP_MATRIX, 1 << lg, g), slots = slots_of(1 << lg, g);
+    auto class_of = [&] {
       int step = 0;
       while (smem > kBlockSmemSteps[step]) step++;
-      i = ((3 - lg) * 2 + keep) * 3 + 2 - step;  // larger instances first
+      return ((3 - lg) * 2 + keep) * 3 + 2 - step;  // larger instances first
+    };
+    if (smem <= (ctas <= 2 * nsm ? kBlockSmemMax : kBlockSmemMax / 2)) {
+      // (the matrix lies behind everything else: its slots are the class's,
+      // and with them the whole class has to fit)
+      keep = KEEP_MATRIX;
+      i = class_of();
+      const size_t all = std::max(cls[i].smem, smem - slot_bytes * slots) + slot_bytes * std::max(cls[i].slots, slots);
+      if (all > kBlockSmemMax) i = -1;
+    }
+    if (i < 0) {
+      keep = KEEP_ALL;
+      slots = 0;
+      smem = smem_of(KEEP_ALL, 1 << lg, g);
+    }
+    if (i >= 0) {
+    } else if (smem <= kBlockSmemMax) {
+      i = class_of();
     } else if ((smem = smem_of(KEEP_Z, 8, g)) <= kBlockSmemMax) {
       i = kBlockClasses - 2;
     } else {
@@ -1953,12 +1968,10 @@ int launch_block(SolverState *s, Krylov &k, const TDyNewtonOptions &o, double to
       i = kBlockClasses - 1;
     }
     cls[i].inst.push_back(g);
-    // (the matrix lies behind everything else: its slots are the class's)
-    const size_t slots = keep == KEEP_MATRIX ? slots_of(1 << lg, g) : 0;
     cls[i].slots = std::max(cls[i].slots, slots);
-    cls[i].smem = std::max(cls[i].smem, smem - (sizeof(T) + sizeof(uint16_t)) * slots);
+    cls[i].smem = std::max(cls[i].smem, smem - slot_bytes * slots);
   }
-  for (Class &c : cls) c.smem += (sizeof(T) + sizeof(uint16_t)) * c.slots;
+  for (Class &c : cls) c.smem += slot_bytes * c.slots;
   s->h_block_list.clear();
   int first[kBlockClasses], used = 0;
   for (int i = 0; i < kBlockClasses; i++) {
