@@ -906,7 +906,7 @@ def run_gpu(args, rank, world, local_rank):
                          "algorithmic_bytes_formula": "8 * (sum_v R_v C_v + sum_v R_v + Nc): Trans, gravity "
                                                       "term per row, cell pressures",
                          "avg_launch_ms": vk_ms,
-                         "binding_roof": "FP64 pipe (see fp64.pipe_active_ncu)"},
+                         "binding_roof": "issue slots and FP64 pipe (see fp64.pipe_active_ncu)"},
             "roofline_evaluation": {"algorithmic_bytes": balg, "GBps": balg / (ms_per_step * 1e-3) / 1e9,
                                     "frac_hbm": balg / (ms_per_step * 1e-3) / 1e9 / hbm_peak,
                                     "bytes_per_cell": balg / nc},

@@ -1918,8 +1918,6 @@ int device_presolve_host(_p_TDy *t, const double *Uprev) {
   return 0;
 }
 
-// The four launches of one evaluation; events[] (5 entries, or null) bracket
-// them for the per-kernel timers.
 static void launch_state_range(const DevArgs &a, int e0, int e1, Emit &e) {
   if (e1 <= e0) return;
   const int nchunks = (int)nblocks(e1 - e0, 32);

@@ -14,7 +14,7 @@ have arrived and wait (up to ``cohort`` of them, consecutive in arrival
 order and of one size class) become one batched handle, each request an
 instance, driven by one worker thread (the C-ABI calls release the
 interpreter lock).  A cohort's Newton iterations evaluate and solve only its
-instances still iterating (one CTA per instance), and a request that fails
+instances still iterating, and a request that fails
 a step is retired from its cohort.  An instance gets the same bits alone and
 in any batch (every schedule gives the same bits, reductions are chunked per
 instance), so a request's result is the same alone and in any mix.
