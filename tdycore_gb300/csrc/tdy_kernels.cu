@@ -338,13 +338,14 @@ struct Curves {
 // cycles (one cell per lane); the state stage of 204 k unsaturated cells took
 // 0.225 ms and takes 0.035 ms so.
 // The cell's parameters: par = m, alpha, n; p = the Mualem parameters.  False
-// (nothing set) outside the range of the integer powers.
+// (nothing set) outside the range of the integer powers, whose exponents are
+// positive: m above 1 makes n negative.
 __device__ __forceinline__ bool vg_mualem(const double *par, const double *p, double Sr, double Pc, bool want_kr,
                                           bool want_d, bool want_d2, Curves *c) {
   const double m = par[0], alpha = par[1], n = par[2];
   const double x = __dmul_rn(Pc, alpha);
   const int be = (int)((unsigned)__double2hiint(x) >> 20) - 1023;  // (a set sign bit puts it out of range)
-  if (!(be > -300 && be < 300 && m >= 0.00390625 && n <= 32.0 && (abs(be) + 1) * (int)(n + 1.0) < 500)) return false;
+  if (!(be > -300 && be < 300 && m >= 0.00390625 && n >= 1.0 && n <= 32.0 && (abs(be) + 1) * (int)(n + 1.0) < 500)) return false;
   const fx lx = log2_fx(x), tn = fx_scale(n, lx);
   const double xn = exp2_fx(tn), w = __dadd_rn(1.0, xn);
   const fx lw = log2_fx(w), mw = fx_scale(m, lw);
