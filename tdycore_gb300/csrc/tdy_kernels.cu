@@ -823,8 +823,9 @@ __device__ __forceinline__ void canon_vertex_at(const DevArgs &a, int vc, int ti
 // state of one thread (the upwind cell data sit in shared memory), which
 // doubles the warps that hide the FP64 latency.
 constexpr int pair_shared_rows(int rho) { return 36 + 16 + (rho == 0 ? 0 : 8) + (rho == 2 ? 8 : 0); }
+// (warp, for the constant density: the lanes of the warp that call it)
 template <int RHO>
-__device__ __forceinline__ void canon_vertex_pair(const DevArgs &a, int vc, int slot, int h, int ns) {
+__device__ __forceinline__ void canon_vertex_pair(const DevArgs &a, int vc, int slot, int h, int ns, unsigned warp) {
   constexpr bool CONST_RHO = RHO != RHO_EXP;
   // [36][ns]: w, E_up, E_dn per row; [8][ns] kr/mu and d(kr/mu)/dP per
   // octant; rho/2 and d(rho/2)/dP per octant where the density varies
@@ -914,8 +915,9 @@ __device__ __forceinline__ void canon_vertex_pair(const DevArgs &a, int vc, int 
     }
   }
   if (!a.needJ) return;
-  // whether any row of this warp's vertices has an E term
-  const bool with_e = RHO != RHO_CONST || __any_sync(__activemask(), any_e != 0);
+  // whether any row of this warp's vertices has an E term (the two lanes of a
+  // pair have to agree: each reads the E terms of the other's rows)
+  const bool with_e = RHO != RHO_CONST || __any_sync(warp, any_e != 0);
   if (RHO == RHO_CONST && with_e) {
 #pragma unroll 1
     for (int t = 0; t < 6; t++) {
@@ -1190,7 +1192,9 @@ __global__ void __launch_bounds__(kPairThreads, 7) vertex_pair_kernel(DevArgs a,
   if ((int)blockIdx.x >= gen_blocks) {
     const int slot = threadIdx.x >> 1, h = threadIdx.x & 1;
     const int vc = a.vc0 + ((int)blockIdx.x - gen_blocks) * (kPairThreads / 2) + slot;
-    if (vc < a.vc1 && !inst_skipped(a, a.cellc[vc])) canon_vertex_pair<RHO>(a, vc, slot, h, kPairThreads / 2);
+    const bool on = vc < a.vc1 && !inst_skipped(a, a.cellc[vc]);
+    const unsigned warp = RHO == RHO_CONST ? __ballot_sync(0xffffffffu, on) : 0;
+    if (on) canon_vertex_pair<RHO>(a, vc, slot, h, kPairThreads / 2, warp);
   } else {
     generic_vertex_group<true>(a, blockIdx.x);
   }
