@@ -2407,16 +2407,10 @@ static int add_linear_times(SolverState *s, double *prec, double *kry) {
   return 0;
 }
 
-int device_be_solve(_p_TDy *t, double dt, double *dU, const TDyNewtonOptions &o, TDyNewtonStats *stats,
-                    int *inst_its, double *inst_rel, void *stream) {
+static int be_solve(_p_TDy *t, double dt, double *dU, const TDyNewtonOptions &o, TDyNewtonStats *stats,
+                    int *inst_its, double *inst_rel, cudaStream_t st) {
   int ierr;
-  if ((ierr = solver_init(t))) {
-    device_solver_destroy(t);
-    return ierr;
-  }
   SolverState *s = t->solver;
-  // a capturable stream: the caller's, else the handle's own
-  cudaStream_t st = (cudaStream_t)(stream ? stream : device_default_stream(t));
   const int n = s->n, ns = s->nseg;
   t->dtime = dt;
   if ((ierr = device_presolve(t, dU, st, true))) return ierr;
@@ -2659,6 +2653,26 @@ int device_be_solve(_p_TDy *t, double dt, double *dU, const TDyNewtonOptions &o,
     stats->block_max_cells = s->precond_used == TDY_PRECOND_LINES ? s->mask_for : -1;
   }
   return 0;
+}
+
+int device_be_solve(_p_TDy *t, double dt, double *dU, const TDyNewtonOptions &o, TDyNewtonStats *stats,
+                    int *inst_its, double *inst_rel, void *stream) {
+  int ierr;
+  if ((ierr = solver_init(t))) {
+    device_solver_destroy(t);
+    return ierr;
+  }
+  // the caller's stream, else the handle's own
+  cudaStream_t st = (cudaStream_t)(stream ? stream : device_default_stream(t));
+  ierr = be_solve(t, dt, dU, o, stats, inst_its, inst_rel, st);
+  if (ierr) {
+    // some of the solve may still run, on the side streams without a join: its
+    // memory and its streams are free for other uses once this returns
+    for (cudaStream_t side : t->solver->side)
+      if (side) cudaStreamSynchronize(side);
+    cudaStreamSynchronize(st);
+  }
+  return ierr;
 }
 
 }  // namespace tdy

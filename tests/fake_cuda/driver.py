@@ -1,0 +1,74 @@
+"""The library linked against fake_cudart.cpp (argument 1), in a process of its
+own: what its device Newton does when a runtime call is refused."""
+import ctypes
+import sys
+from pathlib import Path
+
+import numpy as np
+
+sys.path.insert(0, str(Path(__file__).resolve().parents[2]))
+_cdll = ctypes.CDLL
+ctypes.CDLL = lambda name, *a, **k: _cdll(sys.argv[1] if "libtdycore" in str(name) else name, *a, **k)
+import tdycore_gb300 as T  # noqa: E402
+from tdycore_gb300.workloads import layered_z, structured_surface  # noqa: E402
+
+fake = _cdll(sys.argv[1])
+for name in ("fake_calls", "fake_launches", "fake_violations", "fake_in_flight"):
+    getattr(fake, name).restype = ctypes.c_longlong
+fake.fake_arm.argtypes = [ctypes.c_longlong]
+
+
+def handle():
+    """Instances of three launch classes of the block schedule."""
+    t = T.create_richards_mpfao()
+    blocks, x0 = [], 0.0
+    for n, nz in ((1, 4), (4, 20), (8, 8)):
+        xy, quads = structured_surface(n, n, float(n), float(n))
+        xy[:, 0] += x0
+        x0 += n + 1.0
+        blocks.append((xy, quads, layered_z(xy.shape[0], nz, 0.3 * nz)))
+    t.set_extruded_meshes(blocks)
+    t.set_from_options()
+    t.set_constant_isotropic_permeability(1e-12)
+    t.set_boundary_pressure_type_function(lambda x, y, z: np.full(np.shape(x), T.NEUMANN_BC))
+    t.setup()
+    return t
+
+
+def new_stream():
+    st = ctypes.c_void_p()
+    assert fake.cudaStreamCreateWithFlags(ctypes.byref(st), 1) == 0
+    return st.value
+
+
+def step(t, U, k=0, **kw):
+    """One step whose k-th call is refused (0: none); whether it succeeded."""
+    fake.fake_arm(k)
+    try:
+        t.backward_euler_step_device(U.ctypes.data, 10.0, max_it=1, **kw)
+        ok = True
+    except T.TDyError:
+        ok = False
+    return ok
+
+
+def refusals(stream):
+    """Every call of a step refused in turn: the step fails, leaves nothing in
+    flight, and the handle's memory is freed after its last use."""
+    st = new_stream() if stream == "caller" else None
+    for k in range(1, 10000):
+        t = handle()
+        U = np.full(t.ncells, 1e5)
+        ok = step(t, U, k, schedule="block", stream=st)
+        calls, flying = fake.fake_calls(), fake.fake_in_flight()
+        fake.fake_arm(0)
+        t.destroy()
+        assert flying == 0 and fake.fake_violations() == 0 and fake.fake_in_flight() == 0, k
+        if calls < k:
+            assert ok and k > 100, k
+            return
+    raise AssertionError("the step never ended")
+
+
+if __name__ == "__main__":
+    globals()[sys.argv[2]](*sys.argv[3:])
