@@ -2003,13 +2003,12 @@ int launch_block(SolverState *s, Krylov &k, const TDyNewtonOptions &o, double to
   B.tol2 = tol2;
   B.max_it = o.linear_max_it;
   if (used > 1) {
-    if (!s->fork) {
-      s->device = dev;
-      if ((ierr = device_pool_event(&s->fork))) return ierr;
-      for (int i = 0; i < 3; i++) {
-        if ((ierr = device_pool_stream(&s->side[i]))) return ierr;
-        if ((ierr = device_pool_event(&s->joined[i]))) return ierr;
-      }
+    // (each by itself: an earlier solve may have got some of them only)
+    s->device = dev;
+    if (!s->fork && (ierr = device_pool_event(&s->fork))) return ierr;
+    for (int i = 0; i < 3; i++) {
+      if (!s->side[i] && (ierr = device_pool_stream(&s->side[i]))) return ierr;
+      if (!s->joined[i] && (ierr = device_pool_event(&s->joined[i]))) return ierr;
     }
     SCUDA(cudaEventRecord(s->fork, st));
     for (int i = 0; i < std::min(used - 1, 3); i++) SCUDA(cudaStreamWaitEvent(s->side[i], s->fork, 0));

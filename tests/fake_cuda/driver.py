@@ -13,7 +13,7 @@ import tdycore_gb300 as T  # noqa: E402
 from tdycore_gb300.workloads import layered_z, structured_surface  # noqa: E402
 
 fake = _cdll(sys.argv[1])
-for name in ("fake_calls", "fake_launches", "fake_violations", "fake_in_flight"):
+for name in ("fake_calls", "fake_launches", "fake_violations", "fake_in_flight", "fake_null_stream"):
     getattr(fake, name).restype = ctypes.c_longlong
 fake.fake_arm.argtypes = [ctypes.c_longlong]
 
@@ -66,6 +66,24 @@ def refusals(stream):
         assert flying == 0 and fake.fake_violations() == 0 and fake.fake_in_flight() == 0, k
         if calls < k:
             assert ok and k > 100, k
+            return
+    raise AssertionError("the step never ended")
+
+
+def again():
+    """A refused step, then the same step on the same handle: it succeeds, and
+    nothing goes to the null stream.  (The handles live to the end, so that
+    each takes new streams and events.)"""
+    handles = []
+    for k in range(1, 10000):
+        t = handle()
+        handles.append(t)
+        U = np.full(t.ncells, 1e5)
+        step(t, U, k, schedule="block")
+        calls = fake.fake_calls()
+        assert step(t, U, schedule="block") and fake.fake_null_stream() == 0, k
+        if calls < k:
+            assert k > 100, k
             return
     raise AssertionError("the step never ended")
 

@@ -5,7 +5,7 @@
 // copies and fills are done at once, kernels do nothing.  The k-th call after
 // fake_arm(k) that a runtime can refuse (allocations, copies, launches, events,
 // waits) returns an error.  Streams, events and waits are followed by vector
-// clocks: memory freed on a stream that is not ordered after the work of the
+// clocks (fake_null_stream(): operations on the null stream): memory freed on a stream that is not ordered after the work of the
 // others is counted in fake_violations(), and fake_in_flight() counts the
 // streams whose work the host has not waited for.
 #include <cuda_runtime.h>
@@ -54,6 +54,7 @@ void fake_arm(long long k) { g_calls = 0, g_fail_at = k, g_launches = 0, g_last 
 long long fake_calls() { return g_calls; }
 long long fake_launches() { return g_launches; }
 long long fake_violations() { return g_violations; }
+long long fake_null_stream() { return g_after[nullptr][nullptr]; }
 long long fake_in_flight() {
   long long n = 0;
   for (auto &s : g_after)

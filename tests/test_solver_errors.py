@@ -29,3 +29,7 @@ def run(library, *args):
 @pytest.mark.parametrize("stream", ["own", "caller"])
 def test_refused_calls(fake_library, stream):
     run(fake_library, "refusals", stream)
+
+
+def test_step_after_a_refused_one(fake_library):
+    run(fake_library, "again")
