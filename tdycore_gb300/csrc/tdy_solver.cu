@@ -1810,7 +1810,8 @@ int cluster_setup(SolverState *s, Krylov &k, double tau, cudaStream_t st) {
 }
 
 // The sliced matrix layout of the block schedule, on its first use: offsets
-// from the rows' lengths, column indices by sell_fill_kernel.
+// from the rows' lengths, column indices by sell_fill_kernel.  (sell_col is set
+// when all of it is in place.)
 int sell_setup(SolverState *s, cudaStream_t st) {
   if (s->sell_col) return 0;
   int ierr;
@@ -1819,19 +1820,22 @@ int sell_setup(SolverState *s, cudaStream_t st) {
     for (int k = s->h_slice_off[g]; k < s->h_slice_off[g + 1]; k++)
       end[k] = std::min(s->h_slice_row[k] + 32, s->h_seg_off[g + 1]);
   Arena ar;
+  uint16_t *col = nullptr;
   ar.up(&s->slice_off, s->h_slice_off);
   ar.up(&s->slice_row, s->h_slice_row);
   ar.up(&s->slice_end, end);
   ar.up(&s->sell_off, s->h_sell_off);
-  ar.work(&s->sell_col, (size_t)s->h_sell_off.back());
-  if ((ierr = ar.commit(st))) return ierr;
-  s->allocs.push_back(ar.base);
+  ar.work(&col, (size_t)s->h_sell_off.back());
+  ierr = ar.commit(st);
+  if (ar.base) s->allocs.push_back(ar.base);
+  if (ierr) return ierr;
   if (s->nslices > 0)
     sell_fill_kernel<uint16_t, int><<<nblk(s->nslices, kSliceWarps), 32 * kSliceWarps, 0, st>>>(
         s->nslices, s->slice_row, s->slice_end, s->sell_off, s->cell_seg, nullptr, s->seg_off, s->rowptr, s->colidx,
-        s->sell_col);
+        col);
   SCUDA(cudaGetLastError());
   SCUDA(cudaStreamSynchronize(st));  // the host vectors are read
+  s->sell_col = col;
   return 0;
 }
 

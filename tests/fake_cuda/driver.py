@@ -71,8 +71,8 @@ def refusals(stream):
 
 
 def again():
-    """A refused step, then the same step on the same handle: it succeeds, and
-    nothing goes to the null stream.  (The handles live to the end, so that
+    """A refused step, then the same step on the same handle: it succeeds, makes
+    the copy or launch that was refused, and nothing goes to the null stream.  (The handles live to the end, so that
     each takes new streams and events.)"""
     handles = []
     for k in range(1, 10000):
@@ -81,7 +81,7 @@ def again():
         U = np.full(t.ncells, 1e5)
         step(t, U, k, schedule="block")
         calls = fake.fake_calls()
-        assert step(t, U, schedule="block") and fake.fake_null_stream() == 0, k
+        assert step(t, U, schedule="block") and fake.fake_null_stream() == 0 and not fake.fake_missed(), k
         if calls < k:
             assert k > 100, k
             return

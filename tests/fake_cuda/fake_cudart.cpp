@@ -7,13 +7,16 @@
 // waits) returns an error.  Streams, events and waits are followed by vector
 // clocks (fake_null_stream(): operations on the null stream): memory freed on a stream that is not ordered after the work of the
 // others is counted in fake_violations(), and fake_in_flight() counts the
-// streams whose work the host has not waited for.
+// streams whose work the host has not waited for.  fake_missed(): a copy or
+// launch was refused in the call sequence before the last fake_arm and no copy
+// of that size, or launch of that kernel, was made since.
 #include <cuda_runtime.h>
 
 #include <algorithm>
 #include <cstdlib>
 #include <cstring>
 #include <map>
+#include <set>
 #include <string>
 
 namespace {
@@ -30,13 +33,19 @@ long long g_calls, g_fail_at, g_launches, g_next = 1;
 long long g_violations;
 cudaError_t g_last = cudaSuccess;
 
-cudaError_t refuse() {
+size_t g_refused, g_missing;  // a kernel's address or a copy's size
+std::set<size_t> g_done;
+
+cudaError_t refuse(size_t what = 0) {
   if (++g_calls != g_fail_at) return cudaSuccess;
+  g_refused = what;
   return g_last = cudaErrorUnknown;
 }
-cudaError_t work(const void *st) {
-  cudaError_t e = refuse();
-  if (e == cudaSuccess) g_after[st][st]++;
+cudaError_t work(const void *st, size_t what = 0) {
+  cudaError_t e = refuse(what);
+  if (e != cudaSuccess) return e;
+  g_after[st][st]++;
+  g_done.insert(what);
   return e;
 }
 void *fresh() { return reinterpret_cast<void *>(0x1000 + 16 * g_next++); }
@@ -50,7 +59,12 @@ struct Config {
 
 extern "C" {
 
-void fake_arm(long long k) { g_calls = 0, g_fail_at = k, g_launches = 0, g_last = cudaSuccess; }
+void fake_arm(long long k) {
+  g_calls = 0, g_fail_at = k, g_launches = 0, g_last = cudaSuccess;
+  g_missing = g_refused, g_refused = 0;
+  g_done.clear();
+}
+int fake_missed() { return g_missing && !g_done.count(g_missing); }
 long long fake_calls() { return g_calls; }
 long long fake_launches() { return g_launches; }
 long long fake_violations() { return g_violations; }
@@ -93,7 +107,7 @@ cudaError_t cudaFreeAsync(void *, cudaStream_t st) {
   return cudaSuccess;
 }
 cudaError_t cudaMemcpyAsync(void *d, const void *s, size_t n, enum cudaMemcpyKind, cudaStream_t st) {
-  const cudaError_t e = work(st);
+  const cudaError_t e = work(st, n);
   if (e == cudaSuccess) std::memcpy(d, s, n);
   return e;
 }
@@ -139,9 +153,9 @@ cudaError_t cudaFuncSetAttribute(const void *, enum cudaFuncAttribute, int) { re
 cudaError_t cudaOccupancyMaxActiveBlocksPerMultiprocessorWithFlags(int *n, const void *, int, size_t, unsigned) {
   return *n = 2, cudaSuccess;
 }
-cudaError_t cudaLaunchKernelExC(const cudaLaunchConfig_t *c, const void *, void **) {
+cudaError_t cudaLaunchKernelExC(const cudaLaunchConfig_t *c, const void *f, void **) {
   g_launches++;
-  return work(c->stream);
+  return work(c->stream, (size_t)f);
 }
 unsigned __cudaPushCallConfiguration(dim3 grid, dim3 block, size_t smem, struct CUstream_st *st) {
   g_config = {grid, block, smem, st};
@@ -152,9 +166,9 @@ cudaError_t __cudaPopCallConfiguration(dim3 *grid, dim3 *block, size_t *smem, vo
   return cudaSuccess;
 }
 cudaError_t __cudaGetKernel(cudaKernel_t *k, const void *f) { return *k = (cudaKernel_t)f, cudaSuccess; }
-cudaError_t __cudaLaunchKernel(cudaKernel_t, dim3, dim3, void **, size_t, cudaStream_t st) {
+cudaError_t __cudaLaunchKernel(cudaKernel_t f, dim3, dim3, void **, size_t, cudaStream_t st) {
   g_launches++;
-  return work(st);
+  return work(st, (size_t)f);
 }
 void **__cudaRegisterFatBinary(void *) {
   static void *h;
