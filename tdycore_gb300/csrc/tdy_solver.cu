@@ -71,6 +71,9 @@ struct Krylov {
   void *clu = nullptr;                                 // clusters: LU factors (T), grown on demand
   size_t clu_cap = 0;                                  // elements of clu
   int tpr = 0;  // spmv threads per row (autotuned)
+  // instances of at most this many cells take the block schedule (-2: not
+  // timed yet; the precisions differ in what fits shared memory)
+  long long block_max_cells = -2;
 };
 
 }  // namespace
@@ -111,8 +114,7 @@ struct SolverState {
   int precond_used = 0;
   Krylov k32, k64;
   // schedules of the line-preconditioned inner solve (block: a cluster per
-  // instance; tile: one grid for all cells): instances with at most
-  // block_max_cells cells take the block schedule (-2: not chosen yet)
+  // instance; tile: one grid for all cells)
   int *inst_line_off = nullptr, *block_inst = nullptr, *block_mask = nullptr, *ticket = nullptr;
   std::vector<int> h_inst_line_off, h_order;  // h_order: instances by size, largest first
   // the block schedule's matrix layout (built on its first use): slices of 32
@@ -130,7 +132,7 @@ struct SolverState {
   cudaStream_t side[3] = {nullptr, nullptr, nullptr};  // the classes run side by side
   cudaEvent_t fork = nullptr, joined[3] = {nullptr, nullptr, nullptr};
   int device = 0;
-  long long block_max_cells = -2, mask_for = -3;
+  long long mask_for = -3;  // the split (block_max_cells) of block_mask
   int n_block = 0, n_tile = 0;
   std::vector<double> tune_ms;  // measured candidates of the last tuning (ms per linear solve)
   // phase timers on the solve's stream: evaluation, Jacobian cast and
@@ -2177,15 +2179,15 @@ long long sched_key(const SolverState *s) {
 
 // The split already chosen for this handle or its size class; false if none.
 template <class T>
-bool tuned_schedule(SolverState *s, long long *thr) {
-  if (s->block_max_cells == -2) {
+bool tuned_schedule(const SolverState *s, Krylov &k, long long *thr) {
+  if (k.block_max_cells == -2) {
     const long long key = sched_key<T>(s);
     std::lock_guard<std::mutex> lk(g_sched_mutex);
     for (auto &e : g_sched)
-      if (e.first == key) s->block_max_cells = e.second;
+      if (e.first == key) k.block_max_cells = e.second;
   }
-  *thr = s->block_max_cells;
-  return s->block_max_cells != -2;
+  *thr = k.block_max_cells;
+  return k.block_max_cells != -2;
 }
 
 template <class T>
@@ -2219,7 +2221,7 @@ int tune_schedule(SolverState *s, Krylov &k, const TDyNewtonOptions &o, double t
     std::lock_guard<std::mutex> lk(g_sched_mutex);
     g_sched.emplace_back(key, best_thr);
   }
-  s->block_max_cells = *thr = best_thr;
+  k.block_max_cells = *thr = best_thr;
   return 0;
 }
 
@@ -2237,7 +2239,10 @@ int linear_solve(SolverState *s, Krylov &k, const TDyNewtonOptions &o, const std
     if (o.schedule == TDY_SCHEDULE_BLOCK)
       thr = LLONG_MAX;
     else if (o.schedule != TDY_SCHEDULE_TILE)
-      tune = !tuned_schedule<T>(s, &thr);
+      tune = !tuned_schedule<T>(s, k, &thr);
+    // (FP64 solves within an FP32 step are of the few instances that need
+    // them: too few to time the class on, so they follow the FP32 split)
+    if (tune && sizeof(T) == 8 && o.linear_fp32) tune = !tuned_schedule<float>(s, s->k32, &thr);
   }
   bool tile = tune, block = tune && s->nslices > 0;
   if (!tune)

@@ -88,5 +88,22 @@ def again():
     raise AssertionError("the step never ended")
 
 
+def tuning(first):
+    """The schedule is timed once for each precision of a size class, whichever
+    comes first.  (The timed solves take 16 launches more than a step's own.)"""
+    def extra(t, fp32):
+        n = []
+        for _ in range(2):
+            assert step(t, U, fp32=fp32, spmv_threads=4)
+            n.append(fake.fake_launches())
+        return n[0] - n[1]
+
+    t, order = handle(), (first == "fp32", first != "fp32")
+    U = np.full(t.ncells, 1e5)
+    assert [extra(t, fp32) > 8 for fp32 in order] == [True, True]
+    t = handle()  # another of the class
+    assert [extra(t, fp32) > 8 for fp32 in order] == [False, False]
+
+
 if __name__ == "__main__":
     globals()[sys.argv[2]](*sys.argv[3:])

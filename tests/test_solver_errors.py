@@ -1,6 +1,7 @@
-"""Error paths of the device Newton's host code, on a CUDA runtime without a
-GPU (fake_cuda/): a call that the runtime refuses leaves nothing running on
-memory and streams that go back to their pools."""
+"""The device Newton's host code on a CUDA runtime without a GPU (fake_cuda/):
+a call that the runtime refuses leaves nothing running on memory and streams
+that go back to their pools, and nothing half made for the next step; what is
+timed once is timed once."""
 import subprocess
 import sys
 from pathlib import Path
@@ -33,3 +34,8 @@ def test_refused_calls(fake_library, stream):
 
 def test_step_after_a_refused_one(fake_library):
     run(fake_library, "again")
+
+
+@pytest.mark.parametrize("first", ["fp32", "fp64"])
+def test_schedule_is_timed_for_each_precision(fake_library, first):
+    run(fake_library, "tuning", first)
