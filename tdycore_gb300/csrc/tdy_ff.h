@@ -27,39 +27,11 @@ struct ff {
 // biased exponent field of a double (0 for zero and subnormal numbers)
 __device__ __forceinline__ int d_bexp(double x) { return (int)(((unsigned)__double2hiint(x) >> 20) & 0x7ffu); }
 
-// x * 2^s as hi + lo: hi is x truncated to 24 significant bits, lo the
-// remainder truncated to 24 bits (|error| < 2^-47 |x|).  Results below the
-// float normal range flush to signed zero; above it, hi saturates.
-__device__ __forceinline__ ff ff_split(double x, int s) {
-  const unsigned hw = (unsigned)__double2hiint(x), lw = (unsigned)__double2loint(x);
-  const unsigned sign = hw & 0x80000000u;
-  const int ef = (int)((hw >> 20) & 0x7ffu);
-  const int fe = ef + s - 896;  // float biased exponent of hi
-  ff r;
-  if (ef == 0 || fe <= 0) {
-    r.h = __uint_as_float(sign);
-    r.l = 0.0f;
-    return r;
-  }
-  if (fe >= 255) {
-    r.h = __uint_as_float(sign | 0x7f7fffffu);
-    r.l = 0.0f;
-    return r;
-  }
-  r.h = __uint_as_float(sign | ((unsigned)fe << 23) | ((hw & 0xfffffu) << 3) | (lw >> 29));
-  const unsigned rem = lw & 0x1fffffffu;  // the 29 significand bits below hi
-  const int lz = __clz(rem);              // 32 when rem == 0
-  const int lfe = fe - 21 - lz;           // float biased exponent of lo
-  const unsigned m = (rem << (lz & 31)) >> 8;
-  r.l = (rem == 0u || lfe <= 0) ? __uint_as_float(sign) : __uint_as_float(sign | ((unsigned)lfe << 23) | (m & 0x7fffffu));
-  return r;
-}
-
-// x * 2^s as hi + lo for the Jacobian products, given bx = d_bexp(x) and
-// the scale s, with fewer operations than ff_split: hi is x truncated to 24
-// bits, lo the next 23 significand bits (unnormalised), so |error| < 2^-46
-// |x|.  Callers choose s so that |x| 2^s < 4; parts that fall below the float
-// normal range come out as subnormal or zero floats of magnitude < 2^-126.
+// x * 2^s as hi + lo for the Jacobian products, given bx = d_bexp(x) and the
+// scale s: hi is x truncated to 24 bits, lo the next 23 significand bits
+// (unnormalised), so |error| < 2^-46 |x|.  Callers choose s so that |x| 2^s <
+// 4; parts that fall below the float normal range come out as subnormal or
+// zero floats of magnitude < 2^-126.
 __device__ __forceinline__ ff ff_split_scaled(double x, int bx, int s) {
   const unsigned hw = (unsigned)__double2hiint(x), lw = (unsigned)__double2loint(x);
   const unsigned sign = hw & 0x80000000u;

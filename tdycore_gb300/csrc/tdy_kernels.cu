@@ -467,7 +467,7 @@ __device__ __forceinline__ void state_entity(const DevArgs &a, int i) {
     double rho, drho, d2rho;
     density(a.rho_type, P, &rho, &drho, &d2rho);
     a.P[i] = P;
-    if (a.rho_type != WATER_DENSITY_CONSTANT) {  // (constant: only the other vertices gather rho/2)
+    if (a.rho_type != WATER_DENSITY_CONSTANT) {  // (constant: no vertex gathers it)
       a.hr[i] = 0.5 * rho;
       a.hdr[i] = 0.5 * drho;
     }
@@ -512,8 +512,10 @@ __device__ __forceinline__ void state_entity(const DevArgs &a, int i) {
       lam = cv.kr / a.bnd_vis[b];
     }
     a.P[i] = p;
-    a.hr[i] = 0.5 * a.bnd_rho[b];
-    a.hdr[i] = 0.0;
+    if (a.rho_type != WATER_DENSITY_CONSTANT) {
+      a.hr[i] = 0.5 * a.bnd_rho[b];
+      a.hdr[i] = 0.0;
+    }
     a.lam[i] = a.rho_type == WATER_DENSITY_CONSTANT ? __dmul_rn(kRhoConst, lam) : lam;
     a.dlam[i] = 0.0;
     a.seep[i] = (a.bnd_type[b] == SEEPAGE_BC && p <= a.Pref) ? 1 : 0;
@@ -526,14 +528,6 @@ __global__ void __launch_bounds__(256) state_kernel(DevArgs a, int e0, int e1, i
   if (gw >= nchunks) return;
   const int i = e0 + (int)(((long long)gw * chunk_mul) % nchunks) * 32 + (int)(threadIdx.x & 31);
   if (i < e1) state_entity(a, i);
-}
-
-// rho/2 and its derivative of every entity for the constant density
-__global__ void __launch_bounds__(256) const_density_kernel(int n, double *hr, double *hdr) {
-  const int i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= n) return;
-  hr[i] = 0.5 * kRhoConst;
-  hdr[i] = 0.0;
 }
 
 // Accumulation at the previous solution (TDyMPFAOSNESPreSolve,
@@ -653,8 +647,9 @@ __host__ __device__ constexpr int canon_first_row(int o) {
 // with its derivative).
 enum { RHO_CONST = 0, RHO_NODERIV = 1, RHO_EXP = 2 };
 
-// canonical vertex vc; tid: its slot of the block's shared rows
-template <int RHO, bool FFJ>
+// canonical vertex vc with FP64 Jacobian products; tid: its slot of the
+// block's shared rows
+template <int RHO>
 __device__ __forceinline__ void canon_vertex_at(const DevArgs &a, int vc, int tid) {
   constexpr bool CONST_RHO = RHO != RHO_EXP;
   extern __shared__ double sh[];  // [36][blockDim]: w, E_up, E_dn per row
@@ -723,92 +718,31 @@ __device__ __forceinline__ void canon_vertex_at(const DevArgs &a, int vc, int ti
   if (!a.needJ) return;
   // J_v[c][b] = sum over the three rows k of octant c of
   //   -+ w_r T_rb  (minus when c is the row's up cell)  -+ E terms
-  if (FFJ) {
-    // Octants in a runtime loop (keeps the code small enough for the
-    // instruction cache); entries are indexed relative to the octant,
-    // j = b ^ c, so the row of axis k touches entries 0 (c itself) and 1 << k
-    // at compile-time register indices.
-#pragma unroll 1
-    for (int c = 0; c < 8; c++) {
-      // Each entry is accumulated at its own power-of-two scale, chosen from
-      // the exponent fields of its terms so that its largest term is O(1):
-      // entries of rows upwinded from nearly dry cells (kr ~ 1e-30 and
-      // below) keep full relative accuracy next to O(1) entries.
-      double wk[3], es[3], en[3], Tk[3][8];
-      int bw[3], mb[8];
 #pragma unroll
-      for (int j = 0; j < 8; j++) mb[j] = 0;
+  for (int c = 0; c < 8; c++) {
+    double out[8];
 #pragma unroll
-      for (int k = 0; k < 3; k++) {
-        const int r = canon_row(c, k);
-        const bool up = canon_is_up(c, k);
-        wk[k] = sh[r * bs + tid];
-        bw[k] = d_bexp(wk[k]);
-        const double eu = sh[(12 + r) * bs + tid], ed = sh[(24 + r) * bs + tid];
-        es[k] = up ? eu : ed;  // E term of c itself
-        en[k] = up ? ed : eu;  // E term of the neighbour c ^ (1 << k)
-        const double *T = a.Tc + (long long)(r * 8) * P + vc;
+    for (int b = 0; b < 8; b++) out[b] = 0.0;
 #pragma unroll
-        for (int j = 0; j < 8; j++) {
-          Tk[k][j] = T[(j ^ c) * P];
-          // biased exponent of |w T| (a zero factor gives a negligible value)
-          mb[j] = max(mb[j], bw[k] + d_bexp(Tk[k][j]) - 1023);
-        }
-        mb[0] = max(mb[0], d_bexp(es[k]));
-        mb[1 << k] = max(mb[1 << k], d_bexp(en[k]));
-      }
-      ff acc[8];
+    for (int k = 0; k < 3; k++) {
+      const int r = canon_row(c, k);
+      const bool up = canon_is_up(c, k);
+      const double wr = sh[r * bs + tid];
+      const double sw = up ? -wr : wr;
+      const double *T = a.Tc + (long long)(r * 8) * P + vc;
 #pragma unroll
-      for (int j = 0; j < 8; j++) acc[j] = ff{0.0f, 0.0f};
-#pragma unroll
-      for (int k = 0; k < 3; k++) {
-        const bool up = canon_is_up(c, k);
-        // w normalised to [1, 2); T carries the rest of the entry's scale
-        ff wf = ff_split_scaled(wk[k], bw[k], 1023 - bw[k]);
-        ff ef = ff_split_scaled(es[k], d_bexp(es[k]), 1023 - mb[0]);
-        ff nf = ff_split_scaled(en[k], d_bexp(en[k]), 1023 - mb[1 << k]);
-        if (up) {
-          wf = ff_neg(wf);
-          ef = ff_neg(ef);
-          nf = ff_neg(nf);
-        }
-#pragma unroll
-        for (int j = 0; j < 8; j++)
-          ff_acc(acc[j], ff_mul(wf, ff_split_scaled(Tk[k][j], d_bexp(Tk[k][j]), bw[k] - mb[j])));
-        ff_acc(acc[0], ef);
-        ff_acc(acc[1 << k], nf);
-      }
-      double *dst = S + ((long long)c * P + vc) * 8;
-#pragma unroll
-      for (int j = 0; j < 8; j++) dst[j ^ c] = ff_to_d(acc[j], mb[j] - 1023);
+      for (int b = 0; b < 8; b++) out[b] = __fma_rn(sw, T[b * P], out[b]);
+      const double eu = sh[(12 + r) * bs + tid], ed = sh[(24 + r) * bs + tid];
+      const int u = canon_up(r), d = canon_dn(r);
+      out[u] = __dadd_rn(out[u], up ? -eu : eu);
+      out[d] = __dadd_rn(out[d], up ? -ed : ed);
     }
-  } else {
-#pragma unroll
-    for (int c = 0; c < 8; c++) {
-      double out[8];
-#pragma unroll
-      for (int b = 0; b < 8; b++) out[b] = 0.0;
-#pragma unroll
-      for (int k = 0; k < 3; k++) {
-        const int r = canon_row(c, k);
-        const bool up = canon_is_up(c, k);
-        const double wr = sh[r * bs + tid];
-        const double sw = up ? -wr : wr;
-        const double *T = a.Tc + (long long)(r * 8) * P + vc;
-#pragma unroll
-        for (int b = 0; b < 8; b++) out[b] = __fma_rn(sw, T[b * P], out[b]);
-        const double eu = sh[(12 + r) * bs + tid], ed = sh[(24 + r) * bs + tid];
-        const int u = canon_up(r), d = canon_dn(r);
-        out[u] = __dadd_rn(out[u], up ? -eu : eu);
-        out[d] = __dadd_rn(out[d], up ? -ed : ed);
-      }
-      // J_v[c][0..7] is 64 contiguous bytes at [c][vc][b]
-      double2 *dst = reinterpret_cast<double2 *>(S + ((long long)c * P + vc) * 8);
-      dst[0] = make_double2(out[0], out[1]);
-      dst[1] = make_double2(out[2], out[3]);
-      dst[2] = make_double2(out[4], out[5]);
-      dst[3] = make_double2(out[6], out[7]);
-    }
+    // J_v[c][0..7] is 64 contiguous bytes at [c][vc][b]
+    double2 *dst = reinterpret_cast<double2 *>(S + ((long long)c * P + vc) * 8);
+    dst[0] = make_double2(out[0], out[1]);
+    dst[1] = make_double2(out[2], out[3]);
+    dst[2] = make_double2(out[4], out[5]);
+    dst[3] = make_double2(out[6], out[7]);
   }
 }
 
@@ -818,10 +752,16 @@ __device__ __forceinline__ void canon_vertex_at(const DevArgs &a, int vc, int ti
 // and y rows of octants 4h..4h+3 and half of their z rows (the other half
 // comes from the partner by a shuffle); it writes R_v of octants 4h..4h+3 and
 // entries 4h..4h+3 (relative to the octant, column j ^ c) of every octant's
-// J_v.  Every value is formed by the operations of canon_vertex_at<RHO, true>
-// in the same order, so both give the same bits.  A pair holds half the live
-// state of one thread (the upwind cell data sit in shared memory), which
-// doubles the warps that hide the FP64 latency.
+// J_v.  Rows, fluxes and R_v are formed by the operations of canon_vertex_at in
+// the same order (the same bits).  A pair holds half the live state of one
+// thread (the upwind cell data sit in shared memory), which doubles the warps
+// that hide the FP64 latency.  J_v's octants go in a runtime loop (small enough
+// for the instruction cache), entries indexed relative to the octant, j = b ^ c,
+// so that the row of axis k touches entries 0 (c itself) and 1 << k at
+// compile-time register indices.  Each entry is accumulated at its own
+// power-of-two scale, chosen from the exponent fields of its terms so that its
+// largest term is O(1): entries of rows upwinded from nearly dry cells (kr ~
+// 1e-30 and below) keep full relative accuracy next to O(1) entries.
 constexpr int pair_shared_rows(int rho) { return 36 + 16 + (rho == 0 ? 0 : 8) + (rho == 2 ? 8 : 0); }
 // (warp, for the constant density: the lanes of the warp that call it)
 template <int RHO>
@@ -1172,14 +1112,14 @@ __device__ __forceinline__ void generic_vertex_group(const DevArgs &a, int block
 
 // The other vertices take the first blocks of the canonical vertices' launch,
 // so they overlap and the chain of their rows is off the launch's tail.
-template <int RHO, bool FFJ>
+template <int RHO>
 __global__ void __launch_bounds__(128) vertex_kernel(DevArgs a, int gen_blocks) {
   stage_begin();
   if ((int)blockIdx.x >= gen_blocks) {
     const int vc = a.vc0 + ((int)blockIdx.x - gen_blocks) * blockDim.x + threadIdx.x;
-    if (vc < a.vc1 && !inst_skipped(a, a.cellc[vc])) canon_vertex_at<RHO, FFJ>(a, vc, threadIdx.x);
+    if (vc < a.vc1 && !inst_skipped(a, a.cellc[vc])) canon_vertex_at<RHO>(a, vc, threadIdx.x);
   } else {
-    generic_vertex_group<FFJ>(a, blockIdx.x);
+    generic_vertex_group<false>(a, blockIdx.x);
   }
 }
 
@@ -1792,8 +1732,8 @@ int device_setup(_p_TDy *t) {
   ar.up(&a.sc_cells, s.sc_cells);
   ar.up(&a.sc_vc, s.sc_vc);
   ar.work(&a.P, next);
-  ar.work(&a.hr, next);
-  ar.work(&a.hdr, next);
+  ar.work(&a.hr, a.rho_type == WATER_DENSITY_CONSTANT ? 0 : next);
+  ar.work(&a.hdr, a.rho_type == WATER_DENSITY_CONSTANT ? 0 : next);
   ar.work(&a.lam, next);
   ar.work(&a.dlam, next);
   ar.work(&a.seep, next);
@@ -1821,12 +1761,8 @@ int device_setup(_p_TDy *t) {
   if ((ierr = ar.commit(d->stream))) return ierr;
   d->allocs.push_back(ar.base);
   CUDA_TRY(cudaMemsetAsync(accum_prev, 0, sizeof(double) * m.nc, d->stream));
-  // what no evaluation changes: no cell seeps; constant density
+  // what no evaluation changes: no cell seeps
   CUDA_TRY(cudaMemsetAsync(a.seep, 0, next, d->stream));
-  if (a.rho_type == WATER_DENSITY_CONSTANT) {
-    const_density_kernel<<<(unsigned)((next + 255) / 256), 256, 0, d->stream>>>(next, a.hr, a.hdr);
-    CUDA_TRY(cudaGetLastError());
-  }
   a.accum_prev = accum_prev;
   if (t->opt.setup_on_device &&
       (ierr = device_canon_trans(t, a.cellc, a.facec, const_cast<double *>(a.Tc), d->stream)))
@@ -1958,9 +1894,9 @@ static void launch_vertices(const DevArgs &a, Emit &e) {
   }
   const int cb = (int)nblocks(a.vc1 - a.vc0, 128);
   const size_t smem = cb ? 36 * 128 * sizeof(double) : 0;
-  auto k = rho == RHO_CONST ? vertex_kernel<RHO_CONST, false>
-           : rho == RHO_NODERIV ? vertex_kernel<RHO_NODERIV, false>
-                                : vertex_kernel<RHO_EXP, false>;
+  auto k = rho == RHO_CONST ? vertex_kernel<RHO_CONST>
+           : rho == RHO_NODERIV ? vertex_kernel<RHO_NODERIV>
+                                : vertex_kernel<RHO_EXP>;
   e(k, cb + gb, 128, std::max(smem, gen_smem), a, gb);
 }
 
