@@ -14,8 +14,10 @@
 //   log2 x = e - log2 c + log2(1 + r),  r = f c - 1 exact, |r| < 2^-7.6, c a
 //   10-bit approximation of 1/f from the leading 7 fraction bits of x = f 2^e;
 //   2^t = 2^k 2^(i/128) e^s,  s = (the rest of t) ln 2 < 2^-7.5.
-// The logarithm's absolute error is below 2^-61.4.  Errors of x^y against
-// 200-bit arithmetic, x in 2^-10..2^10 and beside 1: see fx_scale.
+// Measured against 200-bit arithmetic: the logarithm's absolute error is below
+// 2^-61.4 (x in 2^-300..2^300 and beside 1); x^y as exp2_fx(fx_scale(y,
+// log2_fx(x))) is within 0.51 ulp for y up to 4, 0.60 up to 32 and 0.68 up to
+// 64 (x in 2^-10..2^10 and beside 1).
 #pragma once
 
 #include <cuda_runtime.h>
@@ -128,7 +130,7 @@ __device__ __forceinline__ fx log2_fx(double x) {
   return fx{(int)((b >> 52) & 0x7ff) - 1023, t.l + fx_mulhi(p, 0x5c551d94ae0bf85eLL)};
 }
 
-// y a, for y with an exponent in [-8, 6] and |a| < 512
+// y a, for positive y with an exponent in [-8, 6] and |a| < 512
 __device__ __forceinline__ fx fx_scale(double y, fx a) {
   const long long b = __double_as_longlong(y);
   const int s = 52 - ((int)((b >> 52) & 0x7ff) - 1023);  // y = m 2^-s, 46 <= s <= 60
