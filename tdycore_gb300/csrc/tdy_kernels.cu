@@ -1624,13 +1624,19 @@ static int pack_generic(const _p_TDy *t, std::vector<GenVertex> &gen, std::vecto
   // doubles and an int
   const bool vary = a->rho_type != WATER_DENSITY_CONSTANT;
   a->gen_doubles = (vary ? 5 : 3) * max_col + 4 * max_row + (4 * max_row + max_col + 7) / 8;
-  // 4 lanes where a vertex's Trans is small (hexahedra's boundary: 4 rows, 4
-  // columns; 532 k of them 0.34 ms, 0.43 with 8 lanes, 0.76 with 32), a warp
-  // where it is large (prisms: 18 x 12; 108 k of them 0.31 ms, 0.36 with 16
-  // lanes, 0.50 with 8): it is read for the rows and again for J_v, and more
-  // vertices in flight push it out of L1.  A launch of their own where they
-  // are the many (48 registers: 0.31 ms against 0.39 ms in the first blocks of
-  // the canonical ones), not where a launch costs more (10 x 10 x 10 cells).
+  // 4 lanes where a vertex's Trans is small (hexahedra's boundary: 13 to 27
+  // elements), a warp where it is large (prisms: 107 to 205): it is read for
+  // the rows and again for J_v, and more vertices in flight push it out of L1.
+  // F and J in us with 4, 8, 32 lanes: 8 columns 39, 40, 52; 128 columns 173,
+  // 194, 306; 512 columns 582, 653, 1125; 60 x 110 x 40 cells 224, 229, 258; 31 x
+  // 57 x 23 cells 66, 62, 73; 500 prisms 61, 61, 29; 20 k 127, 127, 69; 204 k
+  // 612, 611, 518.  Nothing measured lies between 27 and 107.
+  // A launch of their own where they are many and the most (fewer registers),
+  // not where a launch costs more.  F and J in us in the canonical launch and
+  // in one of their own, with the lanes above: 8 columns (6.1 k other
+  // vertices) 39, 47; 32 columns (30 k) 63, 62; 128 columns (128 k) 173, 179;
+  // 512 columns (532 k) 582, 557; prisms with 12 k 69, 66; 23 k 126, 124; 108 k
+  // 518, 436; 60 x 110 x 40 cells (27 k, and 251 k canonical ones) 224, 236.
   a->gen_lanes = trans <= 64LL * a->ngen ? 4 : 32;
   a->gen_apart = a->ngen > s.nC && a->ngen > 20000;
   while (a->gen_lanes < 32 && (size_t)(128 / a->gen_lanes) * a->gen_doubles * sizeof(double) > 40 * 1024) a->gen_lanes *= 2;
