@@ -235,18 +235,19 @@ typedef struct {
   int fp32_max_it;     /* with linear_fp32: Newton iterations with the FP32 inner solve, FP64 after
                           (an instance still iterating then stalls on FP32 directions; default 8,
                           negative: FP32 throughout) */
-  int spmv_threads;    /* threads per row of the inner solve's sparse products: 0 (default) timed
-                          on the process's first solve; 1, 2, 4 or 8.  Every choice gives the same
-                          bits (each row is summed in 8 phases added by a fixed tree) */
+  int spmv_threads;    /* threads per row of the tile schedule's sparse products: 0 (default) timed
+                          on the handle's first such solve in each precision; 1, 2, 4 or 8.  Every
+                          choice gives the same bits (each row is summed in 8 phases added by a
+                          fixed tree) */
 } TDyNewtonOptions;
 /* Inner-solve schedules.  TILE: one cooperative grid runs the BiCGStab loop over
- * all cells of the batch, instances masked as they converge.  BLOCK: one to eight CTAs per instance (a cluster) run the
- * instance's whole BiCGStab loop (clusters take instances from a counter,
- * largest first); an instance of more than 65536 cells stays on the tile
- * schedule.  AUTO: an autotuner times the tile, block and split schedules (instances up to
- * 4096, 16384 or 65536 cells on the block schedule, the rest on the tile
- * schedule) on the first solve of a size class and keeps the fastest for the
- * process.  The cluster preconditioner runs on the tile schedule. */
+ * all cells of the batch, instances masked as they converge.  BLOCK: one to
+ * eight CTAs per instance (a cluster) run the instance's whole BiCGStab loop
+ * (clusters take instances from a counter, largest first); an instance of more
+ * than 65536 cells stays on the tile schedule.  AUTO: an autotuner times the
+ * tile, block and split schedules (instances up to 4096, 16384 or 65536 cells on
+ * the block schedule, the rest on the tile schedule) on the first solve of a
+ * size class in each precision and keeps the fastest for the process.  The cluster preconditioner runs on the tile schedule. */
 #define TDY_SCHEDULE_AUTO 0
 #define TDY_SCHEDULE_TILE 1
 #define TDY_SCHEDULE_BLOCK 2
